@@ -242,6 +242,24 @@ inline cudaError_t launch_kernel_priority(int priority, void (*kernel)(P...), di
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
 }
 
+// Two values handled together.  FP32 pairs run as one packed instruction (fma.rn.f32x2 and its kin,
+// sm_100 and later): each half is the rounded FP32 operation, at half the issue slots, which is
+// what bounds the per-edge loops.  FP64 pairs are two plain operations.
+template <typename T> struct Pair { T x, y; };
+template <typename T>
+__device__ __forceinline__ Pair<T> fma2(Pair<T> a, Pair<T> b, Pair<T> c) {
+  if constexpr (sizeof(T) == 4) {
+    Pair<T> d;
+    asm("{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
+        " fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+  } else {
+    return {fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)};
+  }
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

@@ -15,10 +15,19 @@
 //
 // GPU mapping: one warp owns one centre atom at a time.  Lanes take edges (32 per batch); each
 // lane evaluates Y_lm and the radial functions of its edge in registers and stages u_mu =
-// x0 x3 R_mu and Y_h in shared memory; lanes then switch to owning (k, lm) moment items and
-// reduce over the staged edges in a fixed order: a plain sum over each batch of <= 32 edges, then a
-// Kahan-compensated add of the batch partial into the atom's moment (FP32 bulk) -- no atomics,
-// deterministic.  The rank contraction and the product graph, forward and reverse, run as the
+// x0 x3 R_mu and Y_h in shared memory, one column per quantity; lanes then switch to owning (k, lm)
+// moment items and reduce over the staged edges in a fixed order: plain sums over each batch of
+// <= 32 edges (even and odd edges apart, then together), then a Kahan-compensated add of the batch
+// partial into the atom's moment (FP32 bulk) -- no atomics, deterministic.
+//
+// What bounds it: instruction issue and the latency of dependent steps at 12 to 16 resident warps
+// per SM (DRAM 1-12% busy), so the per-edge loops are written for few instructions: staged
+// columns read four edges at a time with one Y read per channel group, packed FP32 pairs over
+// edges (moments), basis index (radial sums) and harmonics (adjoints), gate-signal rows moved as
+// whole sectors.  Against one row per edge with scalar reads of both factors: gate forward 133.7 ->
+// 72.2 M warp instructions and 266 -> 183 us, outer 259 -> 195 M and 533 -> 435 us, gate reverse
+// 149 -> 124 M and 259 -> 241 us (Effect L4/K8/R2/O3, 8,000 atoms); Static L3/K4/O2, 32,768 atoms:
+// step 782 -> 680 us.  The rank contraction and the product graph, forward and reverse, run as the
 // pass's lane-balanced graph program (GraphProg) over shared-memory node arrays.  The adjoint
 // pass recomputes Y and R per edge instead of storing them and writes g_e per edge; forces are
 // gathered per atom through the reverse-edge permutation by a separate kernel.
@@ -86,26 +95,48 @@ __host__ __device__ inline int pass_table_size(int C, int F, int B, int nblk) {
   return F * B + 2 * nblk * C * C + 3 * C * F;
 }
 __host__ __device__ constexpr int round4(int n) { return (n + 3) & ~3; }
-// Staged edge row of the forward reduction: u_mu at [0, F), Y_h at [stage_yoff, + H), padded so
-// that rows start on 16-byte boundaries and the row stride in 16-byte units is odd (128-bit row
-// stores of a warp then hit distinct bank groups).
-__host__ __device__ constexpr int stage_yoff(int F) { return round4(F); }
-__host__ __device__ constexpr int stage_stride(int F, int H) {
-  return ((round4(stage_yoff(F) + H) / 4) % 2) ? round4(stage_yoff(F) + H) : round4(stage_yoff(F) + H) + 4;
+// Staged edge columns of the forward reduction: column c holds one quantity of the batch's 32 edges
+// (u_mu at columns [0, F), Y_h at [F, F + H)), so that a lane writes its edge's values without bank
+// conflicts and the reduction reads four edges of a column with one 128-bit access.  The column
+// stride is a multiple of 16 bytes and odd in 16-byte units: the 128-bit reads of neighbouring
+// columns hit distinct bank groups.
+template <typename Real>
+__host__ __device__ constexpr int stage_stride() { return sizeof(Real) == 4 ? 36 : 34; }
+// Moment items of a lane: harmonic lm (all of l's (2 l + 1) functions are neighbouring lanes) and
+// radial channels k = kg + s G, s < slots; G channel groups of H lanes fit in a warp.  A lane's Y
+// value serves every channel it owns, and its u columns of one step are G (L + 1) columns apart.
+template <int L>
+struct MomentItems {
+  static constexpr int Lp = L + 1, H = Lp * Lp;
+  static constexpr int G = H <= kWarp ? kWarp / H : 1;
+  static constexpr int KS = (kMaxK + G - 1) / G;
+  static constexpr int kTail = H > kWarp ? H - kWarp : 0;  // harmonics past the warp width: one (k, lm) item a lane
+  static_assert(kTail == 0 || kWarp / (kTail ? kTail : 1) >= kMaxK, "tail items");
+};
+// Slots a pass runs: half of KS when the model's channels fit there (two compiled trip counts).
+__host__ __device__ constexpr int moment_slots(int L, int K) {
+  const int H = (L + 1) * (L + 1), G = H <= kWarp ? kWarp / H : 1, KS = (kMaxK + G - 1) / G, nk = (K + G - 1) / G;
+  return KS >= 2 && nk <= KS / 2 ? KS / 2 : KS;
+}
+// Staged columns: F + H, and at least those the unused slots of the last channel group reach.
+__host__ __device__ constexpr int stage_cols(int L, int K) {
+  const int H = (L + 1) * (L + 1), G = H <= kWarp ? kWarp / H : 1;
+  const int need = K * (L + 1) + H, reach = moment_slots(L, K) * G * (L + 1);
+  return need > reach ? need : reach;
 }
 // E/F/virial pass tables: radial coefficients [F][B], warp (slope, shift) [2 nblk][C^2], and per
 // species pair (t_i, t_j) the products x0(t_i) x1(t_j) and x0(t_i) wadd(t_j) [C^2][F] each.
 __host__ __device__ inline int efs_table_size(int C, int F, int B, int nblk) {
   return round4(F * B + 2 * nblk * C * C + 2 * C * C * F);
 }
-// Per-warp scratch: the staged edge rows, the node values v [M + 1] (v[M] = 1, the graph
-// program's constant node), the node adjoints [M + 1] (in the staging rows when they fit: those
-// are free once the forward reduction is done), abar [K][H], hbar [F] and the graph program's
-// partial slots [parts].
-__host__ __device__ constexpr bool adj_in_stage(int F, int H, int M) { return M + 1 <= kWarp * stage_stride(F, H); }
+// Per-warp scratch: the staged edge columns, overlaid by the node values v [M + 1] (v[M] = 1, the
+// graph program's constant node) and the node adjoints [M + 1] (they live between the forward
+// reduction and the per-edge adjoint, when the columns are free); the moment adjoints abar
+// [K][round4(H)], hbar [F] and the graph program's partial slots [parts].
 template <typename Real>
-__host__ __device__ inline int pass_warp_size(int F, int H, int M, int K, int parts) {
-  return round4(kWarp * stage_stride(F, H) + (M + 1) + (adj_in_stage(F, H, M) ? 0 : M + 1) + K * H + F + parts + 4);
+__host__ __device__ inline int pass_warp_size(int L, int M, int K, int parts) {
+  const int H = (L + 1) * (L + 1), stage = stage_cols(L, K) * stage_stride<Real>(), nodes = 2 * (M + 1);
+  return round4(round4(stage > nodes ? stage : nodes) + K * round4(H) + K * (L + 1) + parts + 4);
 }
 // Whether the Effect outer pass can stage the neighbours' gate-signal rows h_j with bulk async
 // copies: a row must be a whole number of 16-byte units (the copy's size and alignment rule).
@@ -121,8 +152,8 @@ __host__ __device__ inline bool pass_h_bulk(int mode, int flag, int F) {
 // Per-warp scratch with the h_j staging area appended: 32 rows of F (one per lane, 16-byte
 // aligned) and the warp's mbarrier (4 values, 16 bytes or more).
 template <typename Real>
-__host__ __device__ inline int pass_warp_stride(int F, int H, int M, int K, int parts, bool h_bulk) {
-  return pass_warp_size<Real>(F, H, M, K, parts) + (h_bulk ? kWarp * F + 4 : 0);
+__host__ __device__ inline int pass_warp_stride(int L, int M, int K, int parts, bool h_bulk) {
+  return pass_warp_size<Real>(L, M, K, parts) + (h_bulk ? kWarp * K * (L + 1) + 4 : 0);
 }
 
 // Kahan-compensated accumulation for the FP32 bulk form (explicitly rounded steps, never fused
@@ -194,30 +225,110 @@ __device__ __forceinline__ EdgeIn<Real> load_edge(const typename Vec4<Real>::typ
   return x;
 }
 
-// n values between a global row and a shared-memory row, 128-bit accesses when n is a multiple
-// of 16 bytes' worth (both rows are then 16-byte aligned: row starts are multiples of n values).
+// Rows of a per-atom or per-edge array [.][F] against the staged columns of a batch's nb edges: row
+// index r of lane q's edge <-> column entries stage[mu * stride + q].  Eight edges by four 16-byte
+// units per access: each row's 64 consecutive bytes are whole sectors, where one row per lane
+// would touch 32 lines per access and write half sectors.  Rows that are not whole 16-byte units
+// go value by value, one row per lane.
 template <typename Real>
-__device__ __forceinline__ void copy_row(Real* dst, const Real* src, int n) {
-  constexpr int V = 16 / sizeof(Real);
-  if (n % V == 0) {
-    using W = typename std::conditional<sizeof(Real) == 4, float4, double2>::type;
-    for (int q = 0; q < n / V; ++q) reinterpret_cast<W*>(dst)[q] = reinterpret_cast<const W*>(src)[q];
+struct RowUnit { using type = typename std::conditional<sizeof(Real) == 4, float4, double2>::type; };
+template <typename Real>
+__device__ __forceinline__ void rows_to_cols(Real* stage, const Real* rows, int F, int r, int nb, int lane) {
+  constexpr int V = 16 / sizeof(Real), S = stage_stride<Real>();
+  using W = typename RowUnit<Real>::type;
+  if (F % V == 0) {
+    const int nc = F / V, q8 = lane & 7;
+    const W* src[4];
+#pragma unroll
+    for (int qb = 0; qb < 4; ++qb)
+      src[qb] = reinterpret_cast<const W*>(rows + static_cast<size_t>(__shfl_sync(0xffffffffu, r, 8 * qb + q8)) * F);
+    for (int c = lane >> 3; c < nc; c += 4) {
+      W w[4];
+#pragma unroll
+      for (int qb = 0; qb < 4; ++qb)
+        if (8 * qb + q8 < nb) w[qb] = src[qb][c];
+#pragma unroll
+      for (int qb = 0; qb < 4; ++qb)
+        if (8 * qb + q8 < nb) {
+          Real* d = stage + V * c * S + 8 * qb + q8;
+          d[0] = w[qb].x;
+          d[S] = w[qb].y;
+          if constexpr (V == 4) { d[2 * S] = w[qb].z; d[3 * S] = w[qb].w; }
+        }
+    }
+  } else if (lane < nb) {
+    for (int mu = 0; mu < F; ++mu) stage[mu * S + lane] = rows[static_cast<size_t>(r) * F + mu];
+  }
+  __syncwarp();
+}
+template <typename Real>
+__device__ __forceinline__ void cols_to_rows(Real* rows, const Real* stage, int F, int r, int nb, int lane) {
+  constexpr int V = 16 / sizeof(Real), S = stage_stride<Real>();
+  using W = typename RowUnit<Real>::type;
+  __syncwarp();
+  if (F % V == 0) {
+    const int nc = F / V, q8 = lane & 7;
+    W* dst[4];
+#pragma unroll
+    for (int qb = 0; qb < 4; ++qb)
+      dst[qb] = reinterpret_cast<W*>(rows + static_cast<size_t>(__shfl_sync(0xffffffffu, r, 8 * qb + q8)) * F);
+    for (int c = lane >> 3; c < nc; c += 4) {
+#pragma unroll
+      for (int qb = 0; qb < 4; ++qb)
+        if (8 * qb + q8 < nb) {
+          const Real* d = stage + V * c * S + 8 * qb + q8;
+          W w;
+          w.x = d[0];
+          w.y = d[S];
+          if constexpr (V == 4) { w.z = d[2 * S]; w.w = d[3 * S]; }
+          dst[qb][c] = w;
+        }
+    }
+  } else if (lane < nb) {
+    for (int mu = 0; mu < F; ++mu) rows[static_cast<size_t>(r) * F + mu] = stage[mu * S + lane];
+  }
+  __syncwarp();
+}
+
+// Four consecutive values of a 16-byte aligned shared-memory column as two pairs.
+template <typename Real>
+__device__ __forceinline__ void load_quad(const Real* p, Pair<Real>& a, Pair<Real>& b) {
+  if constexpr (sizeof(Real) == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    a = {v.x, v.y};
+    b = {v.z, v.w};
   } else {
-    for (int q = 0; q < n; ++q) dst[q] = src[q];
+    const double2 v = reinterpret_cast<const double2*>(p)[0], w = reinterpret_cast<const double2*>(p)[1];
+    a = {v.x, v.y};
+    b = {w.x, w.y};
   }
 }
 
-// N (a multiple of 4) values to a 16-byte aligned shared-memory row, 128-bit stores for FP32.
-template <typename Real, int N>
-__device__ __forceinline__ void store_row(Real* dst, const Real (&x)[N]) {
-  static_assert(N % 4 == 0, "row length");
-  if constexpr (sizeof(Real) == 4) {
+// Edge->moment sums of one staged batch: part[s] = sum_q u[q][k_s, l] Y[q][lm] over the batch's
+// edges (rounded up to four: the entries past nb are zero), even and odd edges in the two halves.
+// Per four edges a lane reads Y once and one u column per channel, 128 bits each, and issues two
+// packed multiply-adds per channel.
+template <int NS, int STEP, int TAIL, typename Real, int N>
+__device__ __forceinline__ void moment_batch(const Real* u, const Real* y, const Real* ut, const Real* yt, int nb,
+                                             Pair<Real> (&part)[N]) {
 #pragma unroll
-    for (int q = 0; q < N / 4; ++q)
-      reinterpret_cast<float4*>(dst)[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-  } else {
+  for (int s = 0; s < N; ++s) part[s] = {Real(0), Real(0)};
+#pragma unroll 2
+  for (int q = 0; q < nb; q += 4) {
+    Pair<Real> y0, y1, u0, u1;
+    load_quad(y + q, y0, y1);
 #pragma unroll
-    for (int q = 0; q < N / 2; ++q) reinterpret_cast<double2*>(dst)[q] = make_double2(x[2 * q], x[2 * q + 1]);
+    for (int s = 0; s < NS; ++s) {
+      load_quad(u + s * STEP + q, u0, u1);
+      part[s] = fma2(u0, y0, part[s]);
+      part[s] = fma2(u1, y1, part[s]);
+    }
+    if constexpr (TAIL) {
+      load_quad(yt + q, y0, y1);
+      load_quad(ut + q, u0, u1);
+      part[N - 1] = fma2(u0, y0, part[N - 1]);
+      part[N - 1] = fma2(u1, y1, part[N - 1]);
+    }
   }
 }
 
@@ -269,6 +380,104 @@ __device__ __forceinline__ void radial_loop(const DevModel<Real>& dm, const Real
   }
 }
 
+// Envelopes of an edge's l = 0 and l > 0 functions, times the model's scaling.
+template <typename Real>
+struct Envelopes { Real f0, fd0, f1, fd1; };
+template <typename Real>
+__device__ __forceinline__ Envelopes<Real> edge_envelopes(const DevModel<Real>& dm, Real r) {
+  Envelopes<Real> e;
+  envelope<Real>(r, dm.rmax, dm.poly, dm.cutoff_p, e.f0, e.fd0);
+  if (dm.split) envelope<Real>(r, dm.rang, dm.poly, dm.cutoff_p, e.f1, e.fd1);
+  else { e.f1 = e.f0; e.fd1 = e.fd0; }
+  e.f0 *= dm.scaling; e.fd0 *= dm.scaling; e.f1 *= dm.scaling; e.fd1 *= dm.scaling;
+  return e;
+}
+
+// Chebyshev values T_b(xi) and derivatives D_b = dT_b / dxi (DERIV) of one warp as pairs over b.
+template <typename Real, int NP, bool DERIV>
+__device__ __forceinline__ void cheb_pairs(Real xi, int B, Pair<Real> (&T)[NP], Pair<Real> (&D)[NP]) {
+  Real t2 = Real(1), t1 = xi, d2 = Real(0), d1 = Real(1);
+  const Real x2 = xi + xi;
+  T[0] = {t2, t1};
+  D[0] = {d2, d1};
+#pragma unroll
+  for (int b = 2; b < 2 * NP; ++b) {
+    Real t = Real(0), d = Real(0);
+    if (b < B) {
+      t = x2 * t1 - t2;
+      if (DERIV) d = Real(2) * t1 + (x2 * d1 - d2);
+      t2 = t1; t1 = t;
+      d2 = d1; d1 = d;
+    }
+    if (b & 1) { T[b / 2].y = t; D[b / 2].y = d; }
+    else { T[b / 2].x = t; D[b / 2].x = d; }
+  }
+}
+
+// sum_b c_b T_b and sum_b c_b D_b of one radial function: the even and odd terms are the halves of
+// the packed sums.
+template <typename Real, int BF, int NP, bool DERIV>
+__device__ __forceinline__ void cheb_dot(const Real* c, int B, const Pair<Real> (&T)[NP], const Pair<Real> (&D)[NP],
+                                         Real& a, Real& ad) {
+  Real cc[2 * NP];
+  load_coeff_row<Real, BF, 2 * NP>(c, B, cc);
+  Pair<Real> sa{Real(0), Real(0)}, sd{Real(0), Real(0)};
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    if (2 * p < B) {
+      sa = fma2(Pair<Real>{cc[2 * p], cc[2 * p + 1]}, T[p], sa);
+      if (DERIV) sd = fma2(Pair<Real>{cc[2 * p], cc[2 * p + 1]}, D[p], sd);
+    }
+  }
+  a = sa.x + sa.y;
+  ad = sd.x + sd.y;
+}
+
+// The radial functions R_mu (and dR_mu/dr) of channel k for every l.  Beyond a cutoff the envelope
+// and its slope are exactly zero, so the l > 0 functions of a two-cutoff model vanish by themselves
+// outside the angular cutoff.  The warp is shared by the l of a channel unless the model's scaling
+// map gives each l its own (then a rolled loop: one copy of the warp's code).
+template <int L, typename Real, bool DERIV, int BF>
+__device__ __forceinline__ void radial_channel(const DevModel<Real>& dm, const Real* s_coeff, const Real* s_scal,
+                                               int pair, Real r, const Envelopes<Real>& env, int k, Real (&R)[L + 1],
+                                               Real (&Rd)[L + 1]) {
+  constexpr int Lp = L + 1, NP = ((BF ? BF : kMaxB) + 1) / 2;
+  const int B = BF ? BF : dm.B, C2 = dm.C * dm.C;
+  Pair<Real> T[NP], D[NP];
+  auto warp = [&](int sb) {
+    const Real slope = s_scal[2 * sb * C2 + pair], shift = s_scal[(2 * sb + 1) * C2 + pair];
+    const Real xi = tanh(slope * (r - shift) * Real(0.5));
+    cheb_pairs<Real, NP, DERIV>(xi, B, T, D);
+    return (Real(1) - xi * xi) * slope * Real(0.5);  // dxi / dr
+  };
+  if (dm.scaling_mode == 2 || dm.scaling_mode == 0) {
+    const Real xr = warp(scaling_block(dm.scaling_mode, k, 0, Lp));
+    const Real fx0 = env.f0 * xr, fx1 = env.f1 * xr;
+#pragma unroll
+    for (int l = 0; l < Lp; ++l) {
+      Real a, ad;
+      cheb_dot<Real, BF, NP, DERIV>(s_coeff + (k * Lp + l) * B, B, T, D, a, ad);
+      R[l] = (l == 0 ? env.f0 : env.f1) * a;
+      if (DERIV) Rd[l] = (l == 0 ? env.fd0 : env.fd1) * a + (l == 0 ? fx0 : fx1) * ad;
+    }
+  } else {
+#pragma unroll 1
+    for (int l = 0; l < Lp; ++l) {
+      const Real xr = warp(scaling_block(dm.scaling_mode, k, l, Lp));
+      Real a, ad;
+      cheb_dot<Real, BF, NP, DERIV>(s_coeff + (k * Lp + l) * B, B, T, D, a, ad);
+      const Real f = l == 0 ? env.f0 : env.f1, fd = l == 0 ? env.fd0 : env.fd1;
+      const Real v = f * a, vd = fd * a + f * xr * ad;
+#pragma unroll
+      for (int q = 0; q < Lp; ++q)
+        if (q == l) {
+          R[q] = v;
+          if (DERIV) Rd[q] = vd;
+        }
+    }
+  }
+}
+
 // Steps [s0, s1) of a pass's graph program (GraphProg, device_common.cuh) on the warp's node
 // arrays: forward steps add into v, reverse steps into adj (DIR 1 / 2: the range holds forward /
 // reverse steps only).  Each lane runs its term stream (one
@@ -313,8 +522,8 @@ __device__ __forceinline__ void run_prog(const GraphProg<Real>& g, int s0, int s
 // form the products D[mu][lm] = sum_q u[q][mu] Y[q][lm] (q < 32 edges), computed as m16n8k8 TF32
 // mma.sync tiles with each operand split into a TF32 head and a TF32 tail (3xTF32: head*head +
 // head*tail + tail*head, about FP32 accuracy); the entries with l(mu) = l(lm) are the moment
-// partials, written to part[k][lm].  Rows past the batch are zero; tile columns past F / H read
-// other staged values and are discarded.
+// partials, written to part[k][lm].  Edges past the batch are zero; tile columns past F / H repeat the
+// last one and are discarded.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned tf32_head(float x) {
   unsigned h;
@@ -328,8 +537,8 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const unsigned (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 template <int L>
-__device__ __forceinline__ void moments_mma_batch(const float* stage, int sw, int yoff, int F, float* part, int lane) {
-  constexpr int Lp = L + 1, H = Lp * Lp;
+__device__ __forceinline__ void moments_mma_batch(const float* stage, int F, float* part, int lane) {
+  constexpr int Lp = L + 1, H = Lp * Lp, S = stage_stride<float>();
   const int g = lane >> 2, t = lane & 3;
   const int mtiles = (F + 15) / 16;
   constexpr int ntiles = (H + 7) / 8;
@@ -339,10 +548,11 @@ __device__ __forceinline__ void moments_mma_batch(const float* stage, int sw, in
       float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int ks = 0; ks < kWarp / 8; ++ks) {
-        const float* r0 = stage + (8 * ks + t) * sw;
-        const float* r4 = r0 + 4 * sw;
-        const float av[4] = {r0[16 * mt + g], r0[16 * mt + g + 8], r4[16 * mt + g], r4[16 * mt + g + 8]};
-        const float bv[2] = {r0[yoff + 8 * nt + g], r4[yoff + 8 * nt + g]};
+        const float* a0 = stage + min(16 * mt + g, F - 1) * S + 8 * ks + t;
+        const float* a1 = stage + min(16 * mt + g + 8, F - 1) * S + 8 * ks + t;
+        const float* b0 = stage + (F + min(8 * nt + g, H - 1)) * S + 8 * ks + t;
+        const float av[4] = {a0[0], a1[0], a0[4], a1[4]};
+        const float bv[2] = {b0[0], b0[4]};
         unsigned ah[4], al[4], bh[2], bl[2];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -416,8 +626,10 @@ __host__ __device__ constexpr int default_min_blocks(int L, bool fp32, int mode)
 
 template <int L, typename Real, int MODE, bool KAHAN, int BF, int MINB>
 __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(PassArgs<Real> a) {
-  constexpr int Lp = L + 1, H = Lp * Lp;
-  constexpr int kMaxItems = (kMaxK * H + kWarp - 1) / kWarp;
+  constexpr int Lp = L + 1, H = Lp * Lp, H4 = round4(H), NPH = (H + 1) / 2;
+  constexpr int S = stage_stride<Real>();
+  using MI = MomentItems<L>;
+  constexpr int NS = MI::KS + (MI::kTail ? 1 : 0);  // moment item slots of a lane
   using V4 = typename Vec4<Real>::type;
   const DevModel<Real>& dm = a.dm;
   const bool gate_pass = MODE == kModeGateForward || MODE == kModeGateReverse || MODE == kModeGateFwdEdges ||
@@ -439,15 +651,13 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
   Real* s_scal = s_coeff + F * B;
   Real* s_pw = s_scal + 2 * dm.nblk * C * C;        // [C^2][F] x0(t_i) x1(t_j)
   Real* s_pa = s_pw + C * C * F;                    // [C^2][F] x0(t_i) wadd(t_j)
-  const int wsize = pass_warp_size<Real>(F, H, M, K, dm.prog_parts);
-  Real* wbase = sm + efs_table_size(C, F, B, dm.nblk) + pass_warp_stride<Real>(F, H, M, K, dm.prog_parts, hb_on) * warp;
-  const int sw = stage_stride(F, H), yoff = stage_yoff(F);
-  Real* stage = wbase;                              // [32][sw]: u at [0, F), Y at [yoff, yoff + H)
-  Real* v = stage + kWarp * sw;                     // [M + 1], v[M] = 1
-  const bool adj_staged = adj_in_stage(F, H, M);
-  Real* adj = adj_staged ? stage : v + M + 1;       // [M + 1]
-  Real* abar = v + (M + 1) + (adj_staged ? 0 : M + 1);  // [K][H]
-  Real* hbar = abar + K * H;                        // [F]
+  const int wsize = pass_warp_size<Real>(L, M, K, dm.prog_parts);
+  Real* wbase = sm + efs_table_size(C, F, B, dm.nblk) + pass_warp_stride<Real>(L, M, K, dm.prog_parts, hb_on) * warp;
+  Real* stage = wbase;                              // columns [F + H][S]: u_mu, then Y_h
+  Real* v = wbase;                                  // [M + 1], v[M] = 1 (over the free columns)
+  Real* adj = v + M + 1;                            // [M + 1]
+  Real* abar = wbase + round4(max(stage_cols(L, K) * S, 2 * (M + 1)));  // [K][H4]
+  Real* hbar = abar + K * H4;                       // [F]
   Real* parts = hbar + F;                           // [prog_parts]
   Real* hbuf = wbase + wsize;                       // [32][F] h_j rows of one batch (hb_on)
   unsigned long long* hb_bar = reinterpret_cast<unsigned long long*>(hbuf + kWarp * F);
@@ -499,24 +709,28 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
     return ok;
   };
 
-  // Lane-owned moment items for the forward reduction: item t = lane + 32 s <-> (k, lm); the
-  // first nit of the kMaxItems register slots are in use.
-  const int nit = (K * H + kWarp - 1) / kWarp;
-  int it_u[kMaxItems], it_y[kMaxItems];
+  // the lane's moment items (MomentItems): slot q < KS is (k = kg + q G, lm), the tail slot of L = 5
+  // is (kt, lmt); item_of gives the slot's index k H + lm, -1 when it is none of the model's
+  const bool item_on = lane < MI::G * H;
+  const int lm = H <= kWarp ? (item_on ? lane % H : 0) : lane, kg = H <= kWarp && item_on ? lane / H : 0;
+  auto l_of = [](int h) {
+    int l = 0;
 #pragma unroll
-  for (int s = 0; s < kMaxItems; ++s) {
-    const int t = lane + kWarp * s;
-    if (t < K * H) {
-      const int kk = t / H, lm = t - kk * H;
-      int l = 0;
-      while ((l + 1) * (l + 1) <= lm) ++l;
-      it_u[s] = kk * Lp + l;
-      it_y[s] = yoff + lm;
-    } else {
-      it_u[s] = -1;
-      it_y[s] = 0;
-    }
-  }
+    for (int q = 1; q < Lp; ++q) l += h >= q * q;
+    return l;
+  };
+  const Real* col_u = stage + (kg * Lp + l_of(lm)) * S;
+  const Real* col_y = stage + (F + lm) * S;
+  constexpr int TW = MI::kTail ? MI::kTail : 1;
+  const int lmt = kWarp + lane % TW, kt = lane / TW;
+  const Real* col_ut = stage + (min(kt, K - 1) * Lp + L) * S;
+  const Real* col_yt = stage + (F + lmt) * S;
+  auto item_of = [&](int q) {
+    if (MI::kTail && q == MI::KS) return kt < K ? kt * H + lmt : -1;
+    const int k = kg + q * MI::G;
+    return (H > kWarp || item_on) && k < K ? k * H + lm : -1;
+  };
+  const bool half_slots = MI::KS >= 2 && moment_slots(L, K) < MI::KS;
 
   // centres of this warp: grid-strided, one contiguous run (neighbouring centres share their
   // neighbours' rows in L1), or taken one at a time from a device counter
@@ -558,107 +772,95 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
       cur = load_edge<Real>(a.d4, a.nbr, a.types, e0 + (nbat - 1) * kWarp + lane, C);
     if (kRevOnly) {
       // ---------------- split pass, per-edge part: adjoint moments from the graph kernel ----------
-      for (int t = lane; t < K * H; t += kWarp) abar[t] = a.amom[static_cast<size_t>(atom) * (K * H) + t];
+      for (int t = lane; t < K * H; t += kWarp) abar[t / H * H4 + t % H] = a.amom[static_cast<size_t>(atom) * (K * H) + t];
       __syncwarp();
     } else if (MODE != kModeGateReverse) {
       // ---------------- forward moments ----------------
-      Real acc[kMaxItems], cmp[kMaxItems];
+      Real acc[NS], cmp[NS];
 #pragma unroll
-      for (int s = 0; s < kMaxItems; ++s) { acc[s] = Real(0); cmp[s] = Real(0); }
+      for (int q = 0; q < NS; ++q) { acc[q] = Real(0); cmp[q] = Real(0); }
       // the next batch's edge inputs are loaded while the current batch is evaluated
       if (e0 + lane < e1) cur = load_edge<Real>(a.d4, a.nbr, a.types, e0 + lane, C);
       if (hb_on && nbat > 0) hb_issue(e0 + lane < e1, cur.j, min(kWarp, e1 - e0));
       for (int base = e0; base < e1; base += kWarp) {
-        const int e = base + lane;
+        const int e = base + lane, nb = min(kWarp, e1 - base);
         const bool more = base + kWarp < e1;
         EdgeIn<Real> nxt = cur;
         if (more && e + kWarp < e1) nxt = load_edge<Real>(a.d4, a.nbr, a.types, e + kWarp, C);
         if (hb_on && !hb_arrived()) return;
-        Real* row = stage + lane * sw;
+        // Effect: the neighbours' gate signals h_j, from the bulk-copied batch rows or brought into
+        // the u columns (each value read once before its u_mu overwrites it)
+        if (effect_outer && !hb_on) rows_to_cols<Real>(stage, a.hsig, F, cur.j, nb, lane);
+        Real* col = stage + lane;
         if (e < e1) {
           const V4 dv = cur.d;
-          const int j = cur.j;
-          const int tj = cur.tj;
           const Real r = dv.w, ir = Real(1) / r;
-          Real Y[round4(H)];
-          sph_values<L, Real>(dv.x * ir, dv.y * ir, dv.z * ir, Y);
-          const bool ang = !(r >= dm.rang);
+          {
+            Real Y[H];
+            sph_values<L, Real>(dv.x * ir, dv.y * ir, dv.z * ir, Y);
+            // (with two cutoffs the l > 0 functions beyond the angular one meet u = 0)
 #pragma unroll
-          for (int h = 0; h < round4(H); ++h) Y[h] = (h < H && (h == 0 || ang)) ? Y[h] : Real(0);
-          store_row<Real, round4(H)>(row + yoff, Y);
-          const int pair = ti * C + tj;
+            for (int h = 0; h < H; ++h) col[(F + h) * S] = Y[h];
+          }
+          const int pair = ti * C + cur.tj;
           const Real* pw = s_pw + pair * F;
           const Real* pa = s_pa + pair * F;
-          // Effect: the neighbour's gate signal h_j, from the bulk-copied batch rows or staged in
-          // the row's u slots (each read once before its u_mu overwrites it)
-          const Real* hj = hb_on ? hbuf + lane * F : row;
-          if (effect_outer && !hb_on) copy_row<Real>(row, a.hsig + (size_t)j * F, F);
-          else if (!effect_outer) for (int mu = 0; mu < F; ++mu) row[mu] = Real(0);
-          radial_loop<L, Real, false, BF>(dm, s_coeff, s_scal, pair, r, [&](int k, int l, int mu, Real R, Real) {
-            Real w = pw[mu];
-            if (effect_outer) w += pa[mu] * hj[mu];
-            row[mu] = w * R;
-          });
-          if (effect_outer && !ang)
-            for (int mu = 0; mu < F; ++mu)
-              if (mu % Lp != 0) row[mu] = Real(0);
+          const Real* hj = hbuf + lane * F;
+          const Envelopes<Real> env = edge_envelopes<Real>(dm, r);
+#pragma unroll 1
+          for (int k = 0; k < K; ++k) {
+            Real R[Lp], Rd[Lp];
+            radial_channel<L, Real, false, BF>(dm, s_coeff, s_scal, pair, r, env, k, R, Rd);
+            Real* ck = col + k * Lp * S;
+#pragma unroll
+            for (int l = 0; l < Lp; ++l) {
+              Real w = pw[k * Lp + l];
+              if (effect_outer) w += pa[k * Lp + l] * (hb_on ? hj[k * Lp + l] : ck[l * S]);
+              ck[l * S] = w * R[l];
+            }
+          }
         } else {
-          for (int q = 0; q < sw; ++q) row[q] = Real(0);
+          for (int q = 0; q < F + H; ++q) col[q * S] = Real(0);
         }
         __syncwarp();
         // the next batch's h_j rows travel while this batch is reduced
         if (hb_on && more) hb_issue(e + kWarp < e1, nxt.j, min(kWarp, e1 - base - kWarp));
-        // plain sum over the batch's (<= 32) staged edges, then a compensated add of the batch
+        // plain sums over the batch's (<= 32) staged edges, then a compensated add of the batch
         // partial into the atom's running moment
-        const int nb = min(kWarp, e1 - base);
-        Real part[kMaxItems];
-#pragma unroll
-        for (int s = 0; s < kMaxItems; ++s) part[s] = Real(0);
+        Pair<Real> part[NS];
         if (sizeof(Real) == 4 && a.moment_mma) {
           // tensor-core batch sums into the abar rows (free until the reverse), then each lane
           // reads its items
-          moments_mma_batch<L>(reinterpret_cast<const float*>(stage), sw, yoff, F, reinterpret_cast<float*>(abar), lane);
+          moments_mma_batch<L>(reinterpret_cast<const float*>(stage), F, reinterpret_cast<float*>(abar), lane);
 #pragma unroll
-          for (int s = 0; s < kMaxItems; ++s) {
-            if (s >= nit) break;
-            if (it_u[s] >= 0) part[s] = abar[lane + kWarp * s];
-          }
+          for (int q = 0; q < NS; ++q) part[q] = {item_of(q) >= 0 ? abar[item_of(q)] : Real(0), Real(0)};
+        } else if (half_slots) {
+          moment_batch<MI::KS >= 2 ? MI::KS / 2 : MI::KS, MI::G * Lp * S, MI::kTail>(col_u, col_y, col_ut, col_yt, nb, part);
         } else {
-          for (int q = 0; q < nb; ++q) {
-            const Real* sr = stage + q * sw;
-#pragma unroll
-            for (int s = 0; s < kMaxItems; ++s) {
-              if (s >= nit) break;  // warp-uniform: only the model's K H items are issued
-              if (it_u[s] >= 0) part[s] += sr[it_u[s]] * sr[it_y[s]];
-            }
-          }
+          moment_batch<MI::KS, MI::G * Lp * S, MI::kTail>(col_u, col_y, col_ut, col_yt, nb, part);
         }
 #pragma unroll
-        for (int s = 0; s < kMaxItems; ++s) {
-          if (s >= nit) break;
-          kadd<Real, KAHAN>(acc[s], cmp[s], part[s]);
-        }
+        for (int q = 0; q < NS; ++q) kadd<Real, KAHAN>(acc[q], cmp[q], part[q].x + part[q].y);
         __syncwarp();
         if (more) cur = nxt;
       }
       if (kFwdOnly) {
         // split pass, forward part: the moments go to the graph kernel
 #pragma unroll
-        for (int s = 0; s < kMaxItems; ++s) {
-          if (s >= nit) break;
-          const int t = lane + kWarp * s;
-          if (t < K * H) a.mom[static_cast<size_t>(atom) * (K * H) + t] = acc[s];
+        for (int q = 0; q < NS; ++q) {
+          const int t = item_of(q);
+          if (t >= 0) a.mom[static_cast<size_t>(atom) * (K * H) + t] = acc[q];
         }
         continue;
       }
       for (int q = lane; q <= M; q += kWarp) v[q] = q < M ? Real(0) : Real(1);
       __syncwarp();
 #pragma unroll
-      for (int s = 0; s < kMaxItems; ++s) {
-        const int t = lane + kWarp * s;
-        if (t < K * H) {
+      for (int q = 0; q < NS; ++q) {
+        const int t = item_of(q);
+        if (t >= 0) {
           const int b = dm.basic_of[t];
-          if (b >= 0) v[b] = acc[s];
+          if (b >= 0) v[b] = acc[q];
         }
       }
       __syncwarp();
@@ -715,7 +917,7 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
       run_prog<Real, 2>(pt.prog, pt.prog.nfwd, pt.prog.nsteps, v, adj, parts, lane);
       for (int t = lane; t < K * H; t += kWarp) {
         const int b = dm.basic_of[t];
-        abar[t] = b >= 0 ? adj[b] : Real(0);
+        abar[t / H * H4 + t % H] = b >= 0 ? adj[b] : Real(0);
       }
       __syncwarp();
     }
@@ -725,70 +927,97 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
     // (with bulk-copied h_j rows the last forward batch's rows are still in hbuf: the first
     // adjoint batch uses them, and each batch's copies for the one after are issued mid-batch)
     for (int bt = nbat - 1; bt >= 0; --bt) {
-      const int e = e0 + bt * kWarp + lane;
+      const int e = e0 + bt * kWarp + lane, nb = min(kWarp, e1 - e0 - bt * kWarp);
       const bool valid = e < e1;
       EdgeIn<Real> nxt = cur;
       if (bt > 0) nxt = load_edge<Real>(a.d4, a.nbr, a.types, e - kWarp, C);
       if (hb_on && bt < nbat - 1 && !hb_arrived()) return;
-      if (!hb_on && !valid) { cur = nxt; continue; }
+      // Effect: h_j in the columns (or the bulk-copied batch rows); each value is read before the
+      // hbar contribution overwrites it, and the contributions go out as rows
+      if (effect_outer && !hb_on) rows_to_cols<Real>(stage, a.hsig, F, cur.j, nb, lane);
+      if (!effect_outer && !valid) { cur = nxt; continue; }
       const V4 dv = cur.d;
-      const int j = cur.j;
       const int tj = cur.tj;
       cur = nxt;
       Real r = Real(1), ir = Real(1), ux = Real(0), uy = Real(0), uz = Real(0), s = Real(0);
-      bool ang = false;
       // P[h] = sum_k w R_kl(h) abar[k][h] feeds the angular gradient; the radial-derivative term
       // sum_h Qd[h] Y[h], Qd[h] = sum_k w R'_kl(h) abar[k][h], is summed per (k, l) as
-      // w R'_kl S_kl with S_kl = sum_{h in l} abar[k][h] Y[h] (no per-h Qd registers)
-      Real P[H];
-      // Effect: the hbar contributions are written to the lane's row (free after the forward
-      // reduction) and go out as one row; h_j comes from the bulk-copied batch rows, or is staged
-      // in that row first (each read before its contribution overwrites it)
-      Real* hrow = stage + lane * sw;
+      // w R'_kl S_kl with S_kl = sum_{h in l} abar[k][h] Y[h] (no per-h Qd registers).  Both run on
+      // pairs of harmonics (2 p, 2 p + 1): of one l (one packed step), or of two neighbouring l.
+      Pair<Real> P[NPH];
       if (valid) {
         r = dv.w;
         ir = Real(1) / r;
         ux = dv.x * ir; uy = dv.y * ir; uz = dv.z * ir;
-        ang = !(r >= dm.rang);
-        Real Y[H];
+        Real Y[2 * NPH];
+        Y[2 * NPH - 1] = Real(0);
         sph_values<L, Real>(ux, uy, uz, Y);
 #pragma unroll
-        for (int h = 0; h < H; ++h) { P[h] = Real(0); if (h > 0 && !ang) Y[h] = Real(0); }
-        const Real* hj = hb_on ? hbuf + lane * F : hrow;
-        if (effect_outer && !hb_on) copy_row<Real>(hrow, a.hsig + (size_t)j * F, F);
+        for (int p = 0; p < NPH; ++p) P[p] = {Real(0), Real(0)};
         const int pair = ti * C + tj;
         const Real* pw = s_pw + pair * F;
         const Real* pa = s_pa + pair * F;
-        radial_loop<L, Real, true, BF>(dm, s_coeff, s_scal, pair, r, [&](int k, int l, int mu, Real R, Real Rd) {
-          Real w = pw[mu], wa = Real(0);
-          if (effect_outer) { wa = pa[mu]; w += wa * hj[mu]; }
-          const Real wR = w * R;
-          const Real* ab = abar + k * H;
-          Real S = Real(0);
+        const Real* hj = hbuf + lane * F;
+        Real* col = stage + lane;
+        const Envelopes<Real> env = edge_envelopes<Real>(dm, r);
+#pragma unroll 1
+        for (int k = 0; k < K; ++k) {
+          Real R[Lp], Rd[Lp];
+          radial_channel<L, Real, true, BF>(dm, s_coeff, s_scal, pair, r, env, k, R, Rd);
+          Real* ck = col + k * Lp * S;
+          Real wR[Lp];
+          Pair<Real> Sl[Lp];
 #pragma unroll
-          for (int h = l * l; h < (l + 1) * (l + 1); ++h) {
-            const Real av = ab[h];
-            P[h] += wR * av;
-            S += av * Y[h];
+          for (int l = 0; l < Lp; ++l) {
+            Real w = pw[k * Lp + l];
+            if (effect_outer) {
+              const Real wa = pa[k * Lp + l];
+              w += wa * (hb_on ? hj[k * Lp + l] : ck[l * S]);
+              ck[l * S] = wa * R[l];
+            }
+            wR[l] = w * R[l];
+            Rd[l] *= w;
+            Sl[l] = {Real(0), Real(0)};
           }
-          s += w * Rd * S;
-          if (effect_outer) hrow[mu] = wa * R * S;
-        });
+          const Real* ab = abar + k * H4;
+#pragma unroll
+          for (int h0 = 0; h0 < H; h0 += 4) {
+            Pair<Real> A[2];
+            load_quad(ab + h0, A[0], A[1]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int h = h0 + 2 * u;
+              if (h < H) {
+                const int la = l_of(h), lb = h + 1 < H ? l_of(h + 1) : la;
+                P[h / 2] = fma2(Pair<Real>{wR[la], wR[lb]}, A[u], P[h / 2]);
+                if (h + 1 < H && la == lb) {
+                  Sl[la] = fma2(A[u], Pair<Real>{Y[h], Y[h + 1]}, Sl[la]);
+                } else {
+                  Sl[la].x += A[u].x * Y[h];
+                  if (h + 1 < H) Sl[lb].y += A[u].y * Y[h + 1];
+                }
+              }
+            }
+          }
+#pragma unroll
+          for (int l = 0; l < Lp; ++l) {
+            const Real sum = Sl[l].x + Sl[l].y;
+            s += Rd[l] * sum;
+            if (effect_outer) ck[l * S] *= sum;
+          }
+        }
       }
       // the next (earlier, full) batch's h_j rows travel while this one finishes
       if (hb_on && bt > 0) {
         __syncwarp();
         hb_issue(true, cur.j, kWarp);
       }
-      if (!valid) continue;
       if (effect_outer) {
-        if (!ang)
-          for (int mu = 0; mu < F; ++mu)
-            if (mu % Lp != 0) hrow[mu] = Real(0);
-        copy_row<Real>(a.hcontrib + (size_t)a.rev[e] * F, hrow, F);
+        cols_to_rows<Real>(a.hcontrib, stage, F, valid ? a.rev[e] : 0, nb, lane);
+        if (!valid) continue;
       }
       Real gx = Real(0), gy = Real(0), gz = Real(0);
-      if (ang) sph_grad_dot<L, Real>(ux, uy, uz, P, gx, gy, gz);
+      sph_grad_dot<L, Real>(ux, uy, uz, reinterpret_cast<const Real*>(P), gx, gy, gz);
       const Real ug = ux * gx + uy * gy + uz * gz;
       const Real Gx = ux * s + (gx - ux * ug) * ir;
       const Real Gy = uy * s + (gy - uy * ug) * ir;

@@ -18,12 +18,11 @@ int launch_one(const PassArgs<Real>& a, int sm_count, cudaStream_t stream, bool 
   constexpr bool kKahan = sizeof(Real) == 4;
   auto kern = atom_pass_kernel<L, Real, MODE, kKahan, BF, MINB>;
   const auto& dm = a.dm;
-  const int H = (L + 1) * (L + 1);
   const bool h_bulk = MODE == kModeOuterBulk && h_rows_bulk_ok<Real>(dm.F);
   // warps per block: at most the compiled launch bound
   const int wpb = a.block_warps > 0 && a.block_warps < kPassWarps ? a.block_warps : kPassWarps;
   const size_t smem = sizeof(Real) * (efs_table_size(dm.C, dm.F, dm.B, dm.nblk) +
-                                      wpb * pass_warp_stride<Real>(dm.F, H, dm.M, dm.K, dm.prog_parts, h_bulk));
+                                      wpb * pass_warp_stride<Real>(L, dm.M, dm.K, dm.prog_parts, h_bulk));
   static size_t configured = 0;
   if (smem > configured) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
