@@ -76,6 +76,31 @@ struct GraphProg {
   const ProgRec<Real>* rows = nullptr;  // [row][32]
 };
 
+// The same program for the block-per-32-centres kernel (graph_block.cuh; FP32 engines): node values
+// and adjoints in numbered slots, each step's target lists dealt to the block's warps.
+constexpr int kGraphWarps = 16;       // warps of a block
+constexpr int kGraphAtoms = 32;       // centres of a block
+constexpr int kGraphMaxSlots = 4095;  // 12-bit slots in the packed records
+// A unit is two terms.  Words x and z hold a term's slots, a at bits 7-18 and b at bits 20-31 (a slot
+// times 128 is its byte offset), y and w the coefficients' bits; x's low 7 and z's low 5 bits are
+// the target slot, and flags in z close a chunk (its sum joins the list's), the list (its sum is
+// added to the target slot) and the step (the block's barrier).
+constexpr unsigned kUnitChunkEnd = 1u << 5, kUnitListEnd = 1u << 6, kUnitStepEnd = 1u << 19;
+struct BlockProg {
+  int nslots = 0;                         // 0: the pass has no such program (too many nodes)
+  int one = 0;                            // slot of the constant 1
+  int nzero_v = 0, nzero_adj = 0, nkeep = 0;
+  const int4* units = nullptr;            // term pairs (graph_block.cuh)
+  const int* begin = nullptr;             // [warps][3] the warp's stream: forward, reverse, end
+  const int* basic_slot = nullptr;        // [K H] value slot of moment t, -1 when absent
+  const int* basic_adj = nullptr;         // [K H] its adjoint slot
+  const int* zero_v = nullptr;            // value slots that start at zero
+  const int* zero_adj = nullptr;          // adjoint slots that start at zero (seeded nodes excepted)
+  const int* seed_v = nullptr;            // [S] (outer) / [Q] (gate): slots of the scalars
+  const int* seed_adj = nullptr;
+  const int* keep = nullptr;              // [nkeep] value slots the reverse reads
+};
+
 // Per-pass tables: the outer (energy) pass and the Effect gate pass share this layout.
 template <typename Real>
 struct PassTables {
@@ -109,6 +134,7 @@ struct PassTables {
   const int* rprod_other;
   const Real* rprod_c;
   GraphProg<Real> prog;   // the same contraction and graph as a lane-balanced program (E/F/virial passes)
+  BlockProg block;        // and as a block program (FP32 split passes)
 };
 
 // Parameter-vector offsets (the trainer's Coeff() order) and the gradient-only tables of one pass.
@@ -141,6 +167,7 @@ struct DevModel {
   const double* shift;      // C
   const int* scalar_map;    // S
   const Real* gate_wmat;    // F x Q gate projection h = W g
+  const Real* gate_wmat_t;  // Q x F, its transpose (lanes over mu read neighbouring weights)
   const int* gate_nodes;    // Q
   GradLayout grad;          // parameter-gradient layout
   int prog_parts;           // partial slots of the larger of the two passes' graph programs

@@ -41,7 +41,7 @@ namespace sus2g {
 enum PassMode : int {
   kModeStatic = 0, kModeGateForward = 1, kModeOuter = 2, kModeGateReverse = 3,
   // the Static pass split at the per-atom boundary into three kernels: the edge->moment forward
-  // (moments to a.mom), the per-atom graph (atom_graph_kernel: readout, adjoint moments to
+  // (moments to a.mom), the per-atom graph (graph_block_kernel: readout, adjoint moments to
   // a.amom) and the per-edge adjoint (from a.amom)
   kModeStaticFwd = 4, kModeStaticRev = 5,
   // the Effect outer pass compiled with the neighbours' gate-signal rows h_j brought into shared
@@ -51,8 +51,8 @@ enum PassMode : int {
   // adjoint writing the hbar contributions)
   kModeOuterFwd = 7, kModeOuterRev = 8,
   // the Effect gate passes split the same way: the gate forward pass's edge->moment part (the
-  // per-atom gate graph and gate-signal projection then run in atom_graph_kernel), and the gate
-  // reverse pass's per-edge adjoint (after atom_graph_kernel gathered the gate-signal adjoint and
+  // per-atom gate graph and gate-signal projection then run in graph_block_kernel), and the gate
+  // reverse pass's per-edge adjoint (after graph_block_kernel gathered the gate-signal adjoint and
   // ran the gate graph's reverse)
   kModeGateFwdEdges = 9, kModeGateRevEdges = 10
 };
@@ -72,6 +72,8 @@ struct PassArgs {
   Real* hcontrib;          // [E][F] per-edge hbar contributions, stored at the reverse edge
   Real* gmom;              // [natoms][M] gate moment values (gate forward -> gate reverse)
   const double* hbar_atom; // [natoms][F] gate-signal adjoint already summed per atom (caller edges), or null
+  Real* gkeep;             // [natoms / 32][nkeep][32] gate values the reverse reads (split gate passes)
+  Real* hbar;              // [natoms][F] the same, as hbar_atom, by hbar_sum_kernel (split gate reverse pass)
   double* site_energy;     // [natoms]
   double* virial;          // [natoms][6] (xx, yy, zz, xy, xz, yz), minus d (x) g
   double* desc;            // [natoms][S] scalar moments (descriptors), or null
@@ -877,7 +879,7 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
         for (int mu = lane; mu < F; mu += kWarp) {
           Real h = Real(0);
           for (int q = 0; q < dm.Q; ++q)
-            h += dm.gate_wmat[mu * dm.Q + q] * (staged ? hbar[q] : v[dm.gate_nodes[q]]);
+            h += dm.gate_wmat_t[q * F + mu] * (staged ? hbar[q] : v[dm.gate_nodes[q]]);
           a.hsig[(size_t)atom * F + mu] = h;
         }
         __syncwarp();
@@ -1064,97 +1066,6 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
     __syncwarp();
   }
   finish_dynamic();
-}
-
-// ---------------------------------------------------------------------------------------------
-// The per-atom part of a split pass, warp per centre: for the energy pass (Static or Effect
-// outer), moments a.mom -> the graph program forward -> readout (site energy, descriptors) -> the
-// program's reverse -> adjoint moments a.amom; for the Effect gate passes, the gate graph forward
-// with the gate-signal projection, or the gate-signal adjoint gather and the gate graph reverse.
-// Independent of L; several warps of centres in flight per SM hide the program's load latency
-// that the fused pass serialises between its edge phases.
-// ---------------------------------------------------------------------------------------------
-constexpr int kGraphWarps = 4;
-__host__ __device__ inline int graph_warp_size(int M, int parts, int F, int Q) {
-  return round4(2 * (M + 1) + parts + (F > Q ? F : Q) + 4);
-}
-
-// GM: 0 the energy pass (Static or Effect outer tables: readout, adjoint moments to a.amom);
-// 1 the gate forward pass (gate tables: gate values to a.gmom, gate signals to a.hsig);
-// 2 the gate reverse pass (the gate-signal adjoint gathered per atom, projected onto the gate
-// nodes, the gate graph's reverse, adjoint moments to a.amom).
-
-template <typename Real, int GM>
-__global__ void __launch_bounds__(kGraphWarps * kWarp) atom_graph_kernel(PassArgs<Real> a) {
-  const DevModel<Real>& dm = a.dm;
-  const PassTables<Real>& pt = GM == 0 ? dm.outer : dm.gate;
-  const int M = dm.M, KH = dm.K * dm.H, C = dm.C, F = dm.F;
-  const int warps = blockDim.x / kWarp, warp = threadIdx.x / kWarp, lane = warp_lane();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Real* v = reinterpret_cast<Real*>(smem_raw) + graph_warp_size(M, dm.prog_parts, F, dm.Q) * warp;
-  Real* adj = v + M + 1;
-  Real* parts = adj + M + 1;
-  Real* hbar = parts + dm.prog_parts;  // [F] (GM 2) or the gate scalars [Q] (GM 1)
-  pdl_launch_dependents();
-  pdl_wait();
-  for (int atom = blockIdx.x * warps + warp; atom < a.natoms; atom += gridDim.x * warps) {
-    const int ti = C == 1 ? 0 : species_of(a.types, atom, C);
-    if constexpr (GM == 2) {
-      // the gate-signal adjoint of the atom: summed over its edges' contributions (stored at the
-      // reverse edges by the outer pass), or already summed per atom (caller edges)
-      const int e0 = a.row[atom], e1 = a.row_end[atom];
-      if (!a.hbar_atom && F <= 2 * kWarp) {
-        // both of a lane's columns side by side: the gather is the latency this kernel waits on
-        column_sums_2<Real>(a.hcontrib + (size_t)e0 * F, F, e1 - e0, hbar, lane);
-      } else {
-        for (int mu = lane; mu < F; mu += kWarp)
-          hbar[mu] = a.hbar_atom ? Real(a.hbar_atom[(size_t)atom * F + mu])
-                                 : column_sum<Real>(a.hcontrib + (size_t)e0 * F + mu, F, e1 - e0);
-      }
-      for (int q = lane; q <= M; q += kWarp) {
-        v[q] = q < M ? a.gmom[(size_t)atom * M + q] : Real(1);
-        adj[q] = Real(0);
-      }
-      __syncwarp();
-      for (int q = lane; q < dm.Q; q += kWarp) {
-        Real s = Real(0);
-        for (int mu = 0; mu < F; ++mu) s += hbar[mu] * dm.gate_wmat[mu * dm.Q + q];
-        adj[dm.gate_nodes[q]] += s;
-      }
-      __syncwarp();
-    } else {
-      for (int q = lane; q <= M; q += kWarp) v[q] = q < M ? Real(0) : Real(1);
-      __syncwarp();
-      for (int t = lane; t < KH; t += kWarp) {
-        const int b = dm.basic_of[t];
-        if (b >= 0) v[b] = a.mom[static_cast<size_t>(atom) * KH + t];
-      }
-      __syncwarp();
-      run_prog<Real, 1>(pt.prog, 0, pt.prog.nfwd, v, adj, parts, lane);
-    }
-    if constexpr (GM == 1) {
-      for (int q = lane; q < M; q += kWarp) a.gmom[(size_t)atom * M + q] = v[q];
-      // the gate scalars gathered once, so that each signal's sum reads its weights and the
-      // scalars without a node-index load in between
-      Real* gs = hbar;
-      for (int q = lane; q < dm.Q; q += kWarp) gs[q] = v[dm.gate_nodes[q]];
-      __syncwarp();
-      for (int mu = lane; mu < F; mu += kWarp) {
-        Real h = Real(0);
-        for (int q = 0; q < dm.Q; ++q) h += dm.gate_wmat[mu * dm.Q + q] * gs[q];
-        a.hsig[(size_t)atom * F + mu] = h;
-      }
-      __syncwarp();
-      continue;
-    }
-    if constexpr (GM == 0) readout_seeds<Real>(a, atom, ti, v, adj, lane);
-    run_prog<Real, 2>(pt.prog, pt.prog.nfwd, pt.prog.nsteps, v, adj, parts, lane);
-    for (int t = lane; t < KH; t += kWarp) {
-      const int b = dm.basic_of[t];
-      a.amom[static_cast<size_t>(atom) * KH + t] = b >= 0 ? adj[b] : Real(0);
-    }
-    __syncwarp();
-  }
 }
 
 }  // namespace sus2g

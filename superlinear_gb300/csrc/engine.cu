@@ -819,6 +819,16 @@ struct HostProg {
   bool gate = false;
 };
 
+// The block program (BlockProg, graph_block.cuh) of a pass: its slots, and the lists of build_prog's
+// steps -- term by term and chunk by chunk in that program's order -- dealt to a block's warps.
+struct HostBlockProg {
+  struct Term { int a, b, widx; double c; };
+  struct Unit { Term t[2]; int target; bool chunk_end, list_end, step_end; };
+  std::vector<Unit> units;
+  std::vector<int> begin, basic_slot, basic_adj, zero_v, zero_adj, seed_v, seed_adj, keep;
+  int nslots = 0, one = 0;
+};
+
 namespace {
 
 struct Packer {
@@ -1062,6 +1072,194 @@ HostProg build_prog(const Model& m, bool gate) {
   return hp;
 }
 
+HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::vector<int>& basic_of) {
+  HostBlockProg bp;
+  const int nsteps = static_cast<int>(hp.steps.size());
+  const std::vector<int>& seeds = hp.gate ? m.gate_nodes : m.scalar_map;
+  const int one = m.M;
+  // each step's target lists from the lane streams: chunk = terms up to a flush, list = its chunks
+  struct List { int target; std::vector<std::vector<HostProg::Rec>> chunks; };
+  std::vector<std::vector<List>> steps(nsteps);
+  std::vector<char> in_v(m.M, 0), in_adj(m.M, 0), rev_b(m.M, 0);
+  for (int st = 0; st < nsteps; ++st) {
+    const auto& info = hp.steps[st];
+    const bool rev = (info[3] & 1) != 0;
+    std::map<int, std::vector<HostProg::Rec>> parts;
+    auto mark = [&](int target) { (rev ? in_adj : in_v)[target] = 1; };
+    for (int lane = 0; lane < kWarp; ++lane) {
+      std::vector<HostProg::Rec> chunk;
+      for (int i = 0; i < info[1]; ++i) {
+        const HostProg::Rec& r = hp.rows[static_cast<size_t>(info[0] + i) * kWarp + lane];
+        chunk.push_back(r);
+        if (r.flush == kProgNoFlush) continue;
+        for (const auto& t : chunk) {
+          const int x = static_cast<int>(t.ab & 0xffffu), y = static_cast<int>(t.ab >> 16);
+          if (x != one) (rev ? in_adj : in_v)[x] = 1;
+          if (y != one) { in_v[y] = 1; if (rev) rev_b[y] = 1; }
+        }
+        if (r.flush >= 0) {
+          mark(r.flush);
+          steps[st].push_back({r.flush, {chunk}});
+        } else {
+          parts[-r.flush - 2] = chunk;
+        }
+        chunk.clear();  // (what follows a lane's last flush is padding)
+      }
+    }
+    for (int q = info[2]; q < (info[3] >> 1); ++q) {
+      const auto& c = hp.comb[q];
+      List l{c[0], {}};
+      for (int p = c[1]; p < c[2]; ++p) l.chunks.push_back(parts[p]);
+      mark(c[0]);
+      steps[st].push_back(std::move(l));
+    }
+  }
+  // slots: moments in (k, h) order, the other values, the constant, then adjoints; an adjoint takes
+  // its node's value slot when the reverse never reads the value
+  std::vector<int> vslot(m.M, -1), aslot(m.M, -1);
+  int n = 0;
+  std::vector<char> is_basic(m.M, 0), is_seed(m.M, 0);
+  for (int b : basic_of)
+    if (b >= 0) { is_basic[b] = 1; in_adj[b] = 1; if (vslot[b] < 0) vslot[b] = n++; }
+  for (int q : seeds) { is_seed[q] = 1; in_v[q] = in_adj[q] = 1; }
+  for (int q = 0; q < m.M; ++q)
+    if (in_v[q] && vslot[q] < 0) {
+      vslot[q] = n++;
+      bp.zero_v.push_back(vslot[q]);
+    }
+  bp.one = n++;
+  for (int q = 0; q < m.M; ++q)
+    if (in_adj[q]) {
+      aslot[q] = vslot[q] >= 0 && !rev_b[q] ? vslot[q] : n++;
+      if (!is_seed[q]) bp.zero_adj.push_back(aslot[q]);
+    }
+  if (n > kGraphMaxSlots) return HostBlockProg{};
+  bp.nslots = n;
+  for (int b : basic_of) {
+    bp.basic_slot.push_back(b >= 0 ? vslot[b] : -1);
+    bp.basic_adj.push_back(b >= 0 ? aslot[b] : -1);
+  }
+  for (int q : seeds) { bp.seed_v.push_back(vslot[q]); bp.seed_adj.push_back(aslot[q]); }
+  for (int q = 0; q < m.M; ++q)
+    if (rev_b[q]) bp.keep.push_back(vslot[q]);
+  // streams: lists longest first onto the least-loaded warp
+  const HostBlockProg::Term pad{bp.one, bp.one, -1, 0.0};
+  std::vector<std::vector<HostBlockProg::Unit>> stream(kGraphWarps);
+  std::vector<int> fwd_end(kGraphWarps, 0);
+  auto fours = [&](std::vector<HostBlockProg::Unit>& v) {
+    while (v.size() % 4) v.push_back({{pad, pad}, 0, false, false, false});
+  };
+  for (int st = 0; st < nsteps; ++st) {
+    const bool rev = (hp.steps[st][3] & 1) != 0;
+    std::vector<size_t> cost, order;
+    for (const List& l : steps[st]) {
+      size_t c = 1;
+      for (const auto& ch : l.chunks) c += (ch.size() + 1) / 2;
+      order.push_back(cost.size());
+      cost.push_back(c);
+    }
+    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return cost[x] > cost[y]; });
+    std::vector<size_t> load(kGraphWarps, 0);
+    for (size_t q : order) {
+      const int w = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
+      load[w] += cost[q];
+      const List& l = steps[st][q];
+      for (size_t c = 0; c < l.chunks.size(); ++c) {
+        const auto& ch = l.chunks[c];
+        for (size_t i = 0; i < ch.size(); i += 2) {
+          HostBlockProg::Unit u{{pad, pad}, 0, false, false, false};
+          for (size_t k = 0; k < 2 && i + k < ch.size(); ++k) {
+            const int x = static_cast<int>(ch[i + k].ab & 0xffffu), y = static_cast<int>(ch[i + k].ab >> 16);
+            u.t[k] = {x == one ? bp.one : (rev ? aslot : vslot)[x], y == one ? bp.one : vslot[y], ch[i + k].widx, ch[i + k].cfix};
+          }
+          if (i + 2 >= ch.size()) {
+            u.chunk_end = true;
+            u.list_end = c + 1 == l.chunks.size();
+            u.target = (rev ? aslot : vslot)[l.target];
+          }
+          stream[w].push_back(u);
+        }
+      }
+    }
+    // the step's last unit carries the barrier (a unit of its own for a warp without lists)
+    for (int w = 0; w < kGraphWarps; ++w) {
+      if (load[w] == 0) stream[w].push_back({{pad, pad}, 0, false, false, false});
+      stream[w].back().step_end = true;
+      if (st + 1 == hp.nfwd) {
+        fours(stream[w]);
+        fwd_end[w] = static_cast<int>(stream[w].size());
+      }
+    }
+  }
+  for (int w = 0; w < kGraphWarps; ++w) {
+    fours(stream[w]);
+    const int first = static_cast<int>(bp.units.size());
+    bp.begin.push_back(first);
+    bp.begin.push_back(first + fwd_end[w]);
+    bp.units.insert(bp.units.end(), stream[w].begin(), stream[w].end());
+    bp.begin.push_back(static_cast<int>(bp.units.size()));
+  }
+  bp.units.insert(bp.units.end(), 4, {{pad, pad}, 0, false, false, false});  // (an empty last stream's first read)
+  return bp;
+}
+
+// Serialises the block programs into one 16-byte aligned device image and binds them.
+void upload_block_progs(const Model& m, const HostBlockProg* const (&progs)[2], DevBuf& buf, cudaStream_t s,
+                        BlockProg (&out)[2]) {
+  std::vector<unsigned char> img;
+  auto put = [&](const void* p, size_t n) {
+    const size_t o = (img.size() + 15) & ~size_t(15);
+    img.resize(o + std::max<size_t>(n, 16));
+    if (n) std::memcpy(img.data() + o, p, n);
+    return o;
+  };
+  size_t off[2][9];
+  for (int k = 0; k < 2; ++k) {
+    const HostBlockProg& bp = *progs[k];
+    const std::vector<double>& w = k ? m.gate_w : m.outer_w;
+    std::vector<int4> units(bp.units.size());
+    for (size_t q = 0; q < units.size(); ++q) {
+      const auto& u = bp.units[q];
+      unsigned x[2];
+      float c[2];
+      for (int i = 0; i < 2; ++i) {
+        x[i] = (static_cast<unsigned>(u.t[i].a) << 7) | (static_cast<unsigned>(u.t[i].b) << 20);
+        c[i] = static_cast<float>(u.t[i].widx >= 0 ? w[u.t[i].widx] : u.t[i].c);
+      }
+      x[0] |= static_cast<unsigned>(u.target) & 127u;
+      x[1] |= static_cast<unsigned>(u.target) >> 7;
+      if (u.chunk_end) x[1] |= kUnitChunkEnd;
+      if (u.list_end) x[1] |= kUnitListEnd;
+      if (u.step_end) x[1] |= kUnitStepEnd;
+      int y[2];
+      std::memcpy(y, c, sizeof(y));
+      units[q] = make_int4(static_cast<int>(x[0]), y[0], static_cast<int>(x[1]), y[1]);
+    }
+    off[k][0] = put(units.data(), sizeof(int4) * units.size());
+    const std::vector<int>* lists[] = {&bp.begin, &bp.basic_slot, &bp.basic_adj, &bp.zero_v, &bp.zero_adj, &bp.seed_v, &bp.seed_adj,
+                                       &bp.keep};
+    for (int i = 0; i < 8; ++i) off[k][1 + i] = put(lists[i]->data(), sizeof(int) * lists[i]->size());
+  }
+  buf.ensure(img.size());
+  SUS2G_CUDA(cudaMemcpyAsync(buf.ptr, img.data(), img.size(), cudaMemcpyHostToDevice, s));
+  SUS2G_CUDA(cudaStreamSynchronize(s));
+  const unsigned char* base = static_cast<const unsigned char*>(buf.ptr);
+  for (int k = 0; k < 2; ++k) {
+    const HostBlockProg& bp = *progs[k];
+    auto ints = [&](int i) { return reinterpret_cast<const int*>(base + off[k][i]); };
+    BlockProg g;
+    g.nslots = bp.nslots; g.one = bp.one;
+    g.nzero_v = static_cast<int>(bp.zero_v.size());
+    g.nzero_adj = static_cast<int>(bp.zero_adj.size());
+    g.nkeep = static_cast<int>(bp.keep.size());
+    g.units = reinterpret_cast<const int4*>(base + off[k][0]);
+    g.begin = ints(1); g.basic_slot = ints(2); g.basic_adj = ints(3); g.zero_v = ints(4); g.zero_adj = ints(5);
+    g.seed_v = ints(6); g.seed_adj = ints(7);
+    g.keep = ints(8);
+    out[k] = g;
+  }
+}
+
 // Serialises the programs of the passes into one 16-byte aligned device image and binds them.
 template <typename Real>
 void upload_progs(const Model& m, const std::vector<const HostProg*>& progs, DevBuf& buf, cudaStream_t s,
@@ -1204,6 +1402,10 @@ void Engine::upload_tables() {
       for (int q = 0; q < m.Q; ++q) wmat[static_cast<size_t>(mu) * m.Q + q] = m.gate_weight(mu, q);
   }
   const int o_wmat = pk.add_real(wmat);
+  std::vector<double> wmat_t(wmat.size());
+  for (int mu = 0; mu < m.F && m.gated; ++mu)
+    for (int q = 0; q < m.Q; ++q) wmat_t[static_cast<size_t>(q) * m.F + mu] = wmat[static_cast<size_t>(mu) * m.Q + q];
+  const int o_wmat_t = pk.add_real(wmat_t);
   const int o_nodes = pk.add_int(nodes);
   // parameter-gradient layout: block offsets in the trainer's order and rank-weight row lists
   std::map<std::string, int> off;
@@ -1287,12 +1489,24 @@ void Engine::upload_tables() {
     dm->outer.prog = bound[0];
     dm->gate.prog = m.gated ? bound[1] : bound[0];
     dm->prog_parts = std::max(bound[0].max_parts, m.gated ? bound[1].max_parts : 0);
+    if (sizeof(Real) == 4 && m.B == 8) {  // the engines that can run the split passes
+      if (!block_prog_[0]) {
+        block_prog_[0].reset(new HostBlockProg(build_block_prog(m, *prog_[0], basic_of)));
+        block_prog_[1].reset(new HostBlockProg(m.gated ? build_block_prog(m, *prog_[1], basic_of) : HostBlockProg{}));
+      }
+      BlockProg blocks[2];
+      const HostBlockProg* const hosts[2] = {block_prog_[0].get(), block_prog_[1].get()};
+      upload_block_progs(m, hosts, tab_block_, us, blocks);
+      dm->outer.block = blocks[0];
+      dm->gate.block = blocks[1];
+    }
   }
   dm->linear = R + o_lin;
   dm->species = tab_dbl_.as<double>();
   dm->shift = tab_dbl_.as<double>() + m.C;
   dm->scalar_map = I + o_map;
   dm->gate_wmat = R + o_wmat;
+  dm->gate_wmat_t = R + o_wmat_t;
   dm->gate_nodes = I + o_nodes;
   gl.outer.w_begin = I + ow_b; gl.outer.w_src = I + ow_s; gl.outer.w_dst = I + ow_d;
   gl.gate.w_begin = I + gw_b; gl.gate.w_src = I + gw_s; gl.gate.w_dst = I + gw_d;
@@ -1820,7 +2034,8 @@ void Engine::run_efs(double* d_energy, double* d_forces, double* d_virial, doubl
       if (ghosts)
         SUS2G_CUDA(cudaMemsetAsync(hsig_.ptr, 0, sizeof(Real) * static_cast<size_t>(std::max(1, N)) * m.F, s));
       mark_begin(2);
-      if (use_gate_split<Real>(0)) launches_ += launch_gate_split<Real>(0, a, (pdl_ & kPdlFirstPass) != 0);
+      gate_ran_split_ = use_gate_split<Real>();
+      if (gate_ran_split_) launches_ += launch_gate_split<Real>(0, a, (pdl_ & kPdlFirstPass) != 0);
       else launches_ += launch_pass<Real>(kModeGateForward, a, (pdl_ & kPdlFirstPass) != 0);
       mark_end();
     }
@@ -1849,7 +2064,7 @@ void Engine::run_efs(double* d_energy, double* d_forces, double* d_virial, doubl
     if (m.gated) {
       if (user_edges_) a.hbar_atom = hbar_atom_.as<double>();
       mark_begin(3);
-      if (use_gate_split<Real>(1)) launches_ += launch_gate_split<Real>(1, a, (pdl_ & kPdlBetweenPasses) != 0);
+      if (gate_ran_split_) launches_ += launch_gate_split<Real>(1, a, (pdl_ & kPdlBetweenPasses) != 0);
       else launches_ += launch_pass<Real>(kModeGateReverse, a, (pdl_ & kPdlBetweenPasses) != 0);
       mark_end();
     }
@@ -2129,54 +2344,86 @@ void Engine::efs(double* d_energy, double* d_forces, double* d_virial, double* d
 // tile shape.
 template <typename Real>
 bool Engine::use_static_split() const {
-  return static_split_ && sizeof(Real) == 4 && model_.B == 8;
+  return sizeof(Real) == 4 && model_.B == 8 && (static_split_ < 0 ? auto_split() : static_split_ > 0) && split_fits(false);
+}
+bool Engine::split_fits(bool gate) const {
+  if (precision_ != kFP32) return false;
+  const auto* dm = static_cast<const DevModel<float>*>(dev_model_);
+  return graph_block_fits(gate ? dm->gate.block : dm->outer.block, model_.F, model_.S);
 }
 template <typename Real>
 int Engine::launch_static_split(PassArgs<Real> a, bool pdl) {
-  const size_t n = static_cast<size_t>(std::max(1, ncentres_)) * model_.K * model_.H;
-  mom_.ensure(sizeof(Real) * n);
-  amom_.ensure(sizeof(Real) * n);
-  a.mom = mom_.as<Real>();
-  a.amom = amom_.as<Real>();
-  const int mode = model_.gated ? kModeOuter : kModeStatic;
-  a.grid_mode = pass_grid_[mode];
-  a.atom_order = pass_order_[mode];
-  a.block_warps = pass_wpb_[mode];
-  int k = launch_shape<Real>(model_.gated ? kModeOuterFwd : kModeStaticFwd, a, split_blocks_, pdl);
-  k += launch_atom_graph<Real>(a, sm_count_, stream_);
-  k += launch_shape<Real>(model_.gated ? kModeOuterRev : kModeStaticRev, a, split_blocks_, false);
-  return k;
+  if constexpr (sizeof(Real) == 4) {
+    const size_t n = static_cast<size_t>(std::max(1, ncentres_)) * model_.K * model_.H;
+    mom_.ensure(sizeof(Real) * n);
+    amom_.ensure(sizeof(Real) * n);
+    a.mom = mom_.as<Real>();
+    a.amom = amom_.as<Real>();
+    const int mode = model_.gated ? kModeOuter : kModeStatic;
+    a.grid_mode = pass_grid_[mode];
+    a.atom_order = pass_order_[mode];
+    a.block_warps = pass_wpb_[mode];
+    int k = launch_shape<Real>(model_.gated ? kModeOuterFwd : kModeStaticFwd, a, split_blocks_, pdl);
+    k += launch_atom_graph(a, sm_count_, stream_, 0);
+    k += launch_shape<Real>(model_.gated ? kModeOuterRev : kModeStaticRev, a, split_blocks_, false);
+    return k;
+  } else {
+    throw Error(1, "the split passes run on FP32 engines");
+  }
 }
 
 // The Effect gate passes split at the per-atom boundary (FP32 engines, basis size 8): which 0 =
 // the gate forward pass (edge->moment kernel, then the per-atom gate graph and gate-signal
-// projection), 1 = the gate reverse pass (per-atom gather / projection / gate graph reverse,
-// then the per-edge adjoint); the per-edge kernels take the fused pass's grid and centre order
-// and their own register budget.
+// projection), 1 = the gate reverse pass (per-atom sums of the gate-signal adjoints, their
+// projection and the gate graph reverse, then the per-edge adjoint); the per-edge kernels take the
+// fused pass's grid and centre order and their own register budget.
 template <typename Real>
-bool Engine::use_gate_split(int which) const {
-  return gate_split_[which] && sizeof(Real) == 4 && model_.B == 8 && model_.gated;
+bool Engine::use_gate_split() const {
+  return sizeof(Real) == 4 && model_.B == 8 && model_.gated && (gate_split_ < 0 ? auto_split() : gate_split_ > 0) &&
+         split_fits(true);
+}
+// Without a choice by the caller or the autotuner the passes run split from this many centres on.  A
+// fused pass whose centres all have a resident warp (12 to 16 per SM) hides the per-atom work
+// behind other warps' edges and saves two launches; past that every further round pays for it.
+// Step times fused / split, us: Static L2 4,096 centres 101 / 106, 10,648 193 / 187; Static L3 4,096
+// 120 / 119, 10,648 242 / 232, 110,592 1990 / 1806; Effect L3 2,016 148 / 159, 4,096 228 / 211,
+// 110,592 4240 / 3427; Effect L4 1,000 234 / 263, 2,016 341 / 307, 110,592 10406 / 8490; Effect L5
+// 1,000 229 / 257, 2,016 418 / 344, 32,768 3622 / 2780.
+bool Engine::auto_split() const {
+  return ncentres_ >= sm_count_ * (model_.L >= 4 ? 12 : model_.gated ? 24 : 40);
 }
 template <typename Real>
 int Engine::launch_gate_split(int which, PassArgs<Real> a, bool pdl) {
-  const size_t n = static_cast<size_t>(std::max(1, ncentres_)) * model_.K * model_.H;
-  const int mode = which == 0 ? kModeGateForward : kModeGateReverse;
-  a.grid_mode = pass_grid_[mode];
-  a.atom_order = pass_order_[mode];
-  a.block_warps = pass_wpb_[mode];
-  int k = 0;
-  if (which == 0) {
-    mom_.ensure(sizeof(Real) * n);
-    a.mom = mom_.as<Real>();
-    k += launch_shape<Real>(kModeGateFwdEdges, a, gate_split_blocks_[0], pdl);
-    k += launch_atom_graph<Real>(a, sm_count_, stream_, 1);
+  if constexpr (sizeof(Real) == 4) {
+    const size_t n = static_cast<size_t>(std::max(1, ncentres_)) * model_.K * model_.H;
+    const int mode = which == 0 ? kModeGateForward : kModeGateReverse;
+    a.grid_mode = pass_grid_[mode];
+    a.atom_order = pass_order_[mode];
+    a.block_warps = pass_wpb_[mode];
+    int k = 0;
+    gkeep_.ensure(sizeof(Real) * static_cast<size_t>((std::max(1, ncentres_) + kGraphAtoms - 1) / kGraphAtoms) * kGraphAtoms *
+                  std::max(1, a.dm.gate.block.nkeep));
+    a.gkeep = gkeep_.as<Real>();
+    if (which == 0) {
+      mom_.ensure(sizeof(Real) * n);
+      a.mom = mom_.as<Real>();
+      k += launch_shape<Real>(kModeGateFwdEdges, a, gate_split_blocks_[0], pdl);
+      k += launch_atom_graph(a, sm_count_, stream_, 1);
+    } else {
+      amom_.ensure(sizeof(Real) * n);
+      a.amom = amom_.as<Real>();
+      if (!a.hbar_atom) {
+        hbar_.ensure(sizeof(Real) * static_cast<size_t>(std::max(1, ncentres_)) * model_.F);
+        a.hbar = hbar_.as<Real>();
+        k += launch_hbar_sum(a, stream_);
+      }
+      k += launch_atom_graph(a, sm_count_, stream_, 2);
+      k += launch_shape<Real>(kModeGateRevEdges, a, gate_split_blocks_[1], false);
+    }
+    return k;
   } else {
-    amom_.ensure(sizeof(Real) * n);
-    a.amom = amom_.as<Real>();
-    k += launch_atom_graph<Real>(a, sm_count_, stream_, 2);
-    k += launch_shape<Real>(kModeGateRevEdges, a, gate_split_blocks_[1], false);
+    throw Error(1, "the split passes run on FP32 engines");
   }
-  return k;
 }
 
 // One per-atom pass in the tile shape chosen for its mode (the defaults until autotune runs).
@@ -2226,6 +2473,17 @@ void Engine::autotune_passes(int reps, int* blocks_out, double* ms_out) {
   const int nmodes = m.gated ? 3 : 1;
   for (int q = 0; q < 4; ++q) { blocks_out[q] = 0; ms_out[2 * q] = ms_out[2 * q + 1] = 0.0; }
   cudaEvent_t e0 = take_event(), e1 = take_event();
+  auto timed = [&](auto&& launch) {  // milliseconds per launch, after one warm-up
+    launch();
+    SUS2G_CUDA(cudaEventRecord(e0, s));
+    for (int r = 0; r < reps; ++r) launch();
+    SUS2G_CUDA(cudaEventRecord(e1, s));
+    SUS2G_CUDA(cudaEventSynchronize(e1));
+    float ms = 0.f;
+    SUS2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    return double(ms) / std::max(1, reps);
+  };
+  double gate_gain = 0.0;  // milliseconds the split gate passes save together
   for (int k = 0; k < nmodes; ++k) {
     const int mode = modes[k];
     double best = 0.0;
@@ -2242,14 +2500,7 @@ void Engine::autotune_passes(int reps, int* blocks_out, double* ms_out) {
             a.atom_order = order;
             a.h_bulk = stage;
             a.block_warps = wpb;
-            launch_shape<Real>(mode, a, blocks, false);
-            SUS2G_CUDA(cudaEventRecord(e0, s));
-            for (int r = 0; r < reps; ++r) launch_shape<Real>(mode, a, blocks, false);
-            SUS2G_CUDA(cudaEventRecord(e1, s));
-            SUS2G_CUDA(cudaEventSynchronize(e1));
-            float ms = 0.f;
-            SUS2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            const double per = double(ms) / std::max(1, reps);
+            const double per = timed([&] { launch_shape<Real>(mode, a, blocks, false); });
             double& slot = ms_out[2 * mode + (blocks - 3)];
             if (slot == 0.0 || per < slot) slot = per;
             if (choice == 0 || per < best) {
@@ -2267,46 +2518,35 @@ void Engine::autotune_passes(int reps, int* blocks_out, double* ms_out) {
     if ((mode == kModeStatic || mode == kModeOuter) && sizeof(Real) == 4 && m.B == 8) {
       // the fused energy pass (Static, or Effect outer) against its three-kernel split, in the
       // chosen grid and centre order, the split kernels with either register budget
-      static_split_ = true;
-      double split_best = 0.0;
-      int split_choice = 0;
-      for (int blocks = 3; blocks <= 4; ++blocks) {
-        split_blocks_ = blocks;
-        launch_static_split<Real>(a, false);
-        SUS2G_CUDA(cudaEventRecord(e0, s));
-        for (int r = 0; r < reps; ++r) launch_static_split<Real>(a, false);
-        SUS2G_CUDA(cudaEventRecord(e1, s));
-        SUS2G_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        SUS2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        const double per = double(ms) / std::max(1, reps);
-        if (split_choice == 0 || per < split_best) { split_best = per; split_choice = blocks; }
+      static_split_ = 0;
+      if (split_fits(false)) {
+        double split_best = 0.0;
+        int split_choice = 0;
+        for (int blocks = 3; blocks <= 4; ++blocks) {
+          split_blocks_ = blocks;
+          const double per = timed([&] { launch_static_split<Real>(a, false); });
+          if (split_choice == 0 || per < split_best) { split_best = per; split_choice = blocks; }
+        }
+        split_blocks_ = split_choice;
+        static_split_ = split_best < best ? 1 : 0;
       }
-      split_blocks_ = split_choice;
-      static_split_ = split_best < best;
     }
-    if ((mode == kModeGateForward || mode == kModeGateReverse) && sizeof(Real) == 4 && m.B == 8) {
+    if ((mode == kModeGateForward || mode == kModeGateReverse) && sizeof(Real) == 4 && m.B == 8 && split_fits(true)) {
       // each gate pass against its split (per-edge kernel with either budget, per-atom kernel)
       const int which = mode == kModeGateForward ? 0 : 1;
-      gate_split_[which] = true;
       double split_best = 0.0;
       int split_choice = 0;
       for (int blocks = 3; blocks <= 4; ++blocks) {
         gate_split_blocks_[which] = blocks;
-        launch_gate_split<Real>(which, a, false);
-        SUS2G_CUDA(cudaEventRecord(e0, s));
-        for (int r = 0; r < reps; ++r) launch_gate_split<Real>(which, a, false);
-        SUS2G_CUDA(cudaEventRecord(e1, s));
-        SUS2G_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        SUS2G_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        const double per = double(ms) / std::max(1, reps);
+        const double per = timed([&] { launch_gate_split<Real>(which, a, false); });
         if (split_choice == 0 || per < split_best) { split_best = per; split_choice = blocks; }
       }
       gate_split_blocks_[which] = split_choice;
-      gate_split_[which] = split_best < best;
+      gate_gain += best - split_best;
     }
   }
+  // the two gate passes take the same form (the split ones share the kept gate values)
+  gate_split_ = gate_gain > 0.0 ? 1 : 0;
   event_next_ = 0;
   reset_step_graph();  // a captured step holds the previous budgets
   // graphs captured elsewhere (a trainer's evaluation graph) hold them too: a new edge generation
@@ -2335,6 +2575,9 @@ void Engine::set_pass_shape(int mode, int blocks, int grid, int order, int stage
   pass_grid_[mode] = grid;
   pass_order_[mode] = order;
   pass_stage_[mode] = stage;
+  // a pinned shape is the fused pass's
+  if ((mode == kModeStatic || mode == kModeOuter) && static_split_ < 0) static_split_ = 0;
+  if ((mode == kModeGateForward || mode == kModeGateReverse) && gate_split_ < 0) gate_split_ = 0;
   reset_step_graph();
   ++edge_generation_;  // graphs captured by other owners hold the previous shape
 }

@@ -13,6 +13,7 @@ namespace sus2g {
 
 template <typename Real> struct PassArgs;  // efs_kernels.cuh
 struct HostProg;                            // engine.cu: a pass's graph program on the host
+struct HostBlockProg;                       // engine.cu: the same as a block program
 
 enum Precision : int { kFP64 = 0, kFP32 = 1 };
 
@@ -91,8 +92,8 @@ class Engine {
   // as three kernels) + 8 x h_j staging by bulk async copies, warps per block
   void pass_shape(int mode, int* shape4) const {
     shape4[0] = pass_blocks_[mode]; shape4[1] = pass_grid_[mode];
-    const bool gate_split = model_.gated && (mode == 1 || mode == 3) && gate_split_[mode == 1 ? 0 : 1];
-    const bool split = (static_split_ && mode == (model_.gated ? 2 : 0)) || gate_split;
+    const bool gate_split = model_.gated && (mode == 1 || mode == 3) && gate_split_ > 0;
+    const bool split = (static_split_ > 0 && mode == (model_.gated ? 2 : 0)) || gate_split;
     if (split) shape4[0] = gate_split ? gate_split_blocks_[mode == 1 ? 0 : 1] : split_blocks_;
     shape4[2] = pass_order_[mode] + (split ? 4 : 0) + (pass_stage_[mode] ? 8 : 0);
     shape4[3] = pass_wpb_[mode];
@@ -107,13 +108,13 @@ class Engine {
   // drops a captured step graph.
   // The per-atom passes split at the per-atom boundary instead of fused (FP32 engines, basis size
   // 8): the energy pass -- Static, or the Effect outer pass -- as three kernels (edge->moment
-  // forward, per-atom graph, per-edge adjoint), the Effect gate passes as two each; the
-  // autotuner chooses per pass; a change drops a captured step graph.
+  // forward, per-atom graph, per-edge adjoint), the Effect gate passes likewise.  Without this call
+  // the number of centres decides (auto_split), unless a pass's shape is pinned (fused) or the
+  // autotuner has chosen; a change drops a captured step graph.
   void set_static_split(bool on) {
-    if (on != static_split_ || on != gate_split_[0] || on != gate_split_[1]) reset_step_graph();
-    static_split_ = gate_split_[0] = gate_split_[1] = on;
+    if (static_split_ != (on ? 1 : 0) || gate_split_ != (on ? 1 : 0)) { reset_step_graph(); ++edge_generation_; }
+    static_split_ = gate_split_ = on ? 1 : 0;
   }
-  bool static_split() const { return static_split_; }
   // The outer and gate reverse parameter-gradient passes as two kernels each (per-atom part,
   // per-edge part; basis size 8) instead of one; a change drops a captured step graph and makes
   // graphs captured by other owners (a trainer) be captured again.
@@ -252,6 +253,8 @@ class Engine {
   // model tables (both precisions are packed into one buffer each)
   DevBuf tab_int_, tab_real_, tab_dbl_, tab_prog_;
   std::unique_ptr<HostProg> prog_[2];  // outer and gate graph programs (structure built once)
+  std::unique_ptr<HostBlockProg> block_prog_[2];
+  DevBuf tab_block_;
   void* dev_model_ = nullptr;  // host copy of DevModel<Real>
 
   // geometry
@@ -304,14 +307,18 @@ class Engine {
   static constexpr int kWorkInts = 32;  // work_: (next centre, warps done) per pass mode (< 16)
   DevBuf work_;                 // counters of the dynamic centre order
   template <typename Real> bool use_static_split() const;
-  template <typename Real> bool use_gate_split(int which) const;
+  bool split_fits(bool gate) const;  // the pass's nodes fit the block graph kernel
+  template <typename Real> bool use_gate_split() const;
+  bool auto_split() const;
   template <typename Real> int launch_gate_split(int which, PassArgs<Real> a, bool pdl);
   template <typename Real> int launch_static_split(PassArgs<Real> a, bool pdl);
-  bool static_split_ = false;   // energy pass as forward / per-atom graph / adjoint kernels
+  int static_split_ = -1;       // energy pass as forward / per-atom graph / adjoint kernels (-1: auto_split)
   int split_blocks_ = 0;        // register budget of the split's per-edge kernels (0 = default)
-  bool gate_split_[2] = {false, false};  // Effect gate forward / reverse passes split
+  int gate_split_ = -1;         // Effect gate forward and reverse passes split (together: gkeep_)
+  bool gate_ran_split_ = false; // the form of the last gate forward pass, which its reverse takes too
   int gate_split_blocks_[2] = {0, 0};    // their per-edge kernels' register budgets
   DevBuf mom_, amom_;           // the split pass's moments and adjoint moments [N][K H]
+  DevBuf hbar_, gkeep_;         // split gate passes: adjoints of h per centre [N][F], gate values kept for the reverse
   // second stream for independent work inside a step (reverse edges beside the first pass, the
   // frame reduction beside the force gather)
   cudaStream_t aux_stream_ = nullptr;

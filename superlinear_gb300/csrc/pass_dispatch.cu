@@ -4,6 +4,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "graph_block.cuh"
 #include "pass_launch.h"
 
 namespace sus2g {
@@ -68,32 +69,52 @@ cudaError_t upload_grad_constants() {
   return cudaSuccess;
 }
 
-template <typename Real>
-int launch_atom_graph(const PassArgs<Real>& a, int sm_count, cudaStream_t s, int gm) {
-  if (a.natoms == 0) return 0;
-  if (gm < 0 || gm > 2) throw std::runtime_error("graph kernel: unknown pass");
-  auto kern = gm == 0 ? atom_graph_kernel<Real, 0> : gm == 1 ? atom_graph_kernel<Real, 1> : atom_graph_kernel<Real, 2>;
-  const size_t smem =
-      sizeof(Real) * kGraphWarps * static_cast<size_t>(graph_warp_size(a.dm.M, a.dm.prog_parts, a.dm.F, a.dm.Q));
-  static size_t configured[3] = {0, 0, 0};
-  if (smem > configured[gm]) {
+namespace {
+template <int GM>
+int launch_graph(const PassArgs<float>& a, int sm_count, cudaStream_t s) {
+  const BlockProg& g = GM == 0 ? a.dm.outer.block : a.dm.gate.block;
+  auto kern = graph_block_kernel<GM>;
+  const size_t smem = graph_block_bytes(g.nslots, a.dm.F, a.dm.S);
+  static size_t configured = 0;
+  if (smem > configured) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) throw std::runtime_error(std::string("graph kernel shared memory: ") + cudaGetErrorString(err));
-    configured[gm] = smem;
+    configured = smem;
   }
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGraphWarps * kWarp, smem);
   if (per_sm < 1) throw std::runtime_error("graph kernel does not fit on an SM");
-  const int need = (a.natoms + kGraphWarps - 1) / kGraphWarps;
-  const int grid = std::max(1, std::min(need, per_sm * sm_count));
-  kern<<<grid, kGraphWarps * kWarp, smem, s>>>(a);
+  const int need = (a.natoms + kGraphAtoms - 1) / kGraphAtoms;
+  kern<<<std::max(1, std::min(need, per_sm * sm_count)), kGraphWarps * kWarp, smem, s>>>(a);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("graph kernel launch: ") + cudaGetErrorString(err));
   return 1;
 }
+}  // namespace
 
-template int launch_atom_graph<float>(const PassArgs<float>&, int, cudaStream_t, int);
-template int launch_atom_graph<double>(const PassArgs<double>&, int, cudaStream_t, int);
+bool graph_block_fits(const BlockProg& g, int F, int S) {
+  return g.nslots > 0 && graph_block_bytes(g.nslots, F, S) <= 227 * 1024;
+}
+
+int launch_atom_graph(const PassArgs<float>& a, int sm_count, cudaStream_t s, int gm) {
+  if (a.natoms == 0) return 0;
+  switch (gm) {
+    case 0: return launch_graph<0>(a, sm_count, s);
+    case 1: return launch_graph<1>(a, sm_count, s);
+    case 2: return launch_graph<2>(a, sm_count, s);
+  }
+  throw std::runtime_error("graph kernel: unknown pass");
+}
+
+int launch_hbar_sum(const PassArgs<float>& a, cudaStream_t s) {
+  if (a.natoms == 0) return 0;
+  const unsigned blocks = static_cast<unsigned>((static_cast<long long>(a.natoms) * kWarp + 255) / 256);
+  hbar_sum_kernel<<<blocks, 256, 0, s>>>(a);
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) throw std::runtime_error(std::string("gate-signal adjoint launch: ") + cudaGetErrorString(err));
+  return 1;
+}
+
 template int launch_atom_pass<float>(int, int, const PassArgs<float>&, int, cudaStream_t, int, bool);
 template int launch_atom_pass<double>(int, int, const PassArgs<double>&, int, cudaStream_t, int, bool);
 template GradLaunch grad_pass_config<float>(int, int, const DevModel<float>&, int, int, int);

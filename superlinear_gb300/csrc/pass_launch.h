@@ -31,10 +31,13 @@ template <typename Real>
 int launch_atom_pass(int L, int mode, const PassArgs<Real>& args, int sm_count, cudaStream_t stream,
                      int blocks = 0, bool pdl = false);
 
-// The per-atom graph kernel of a split pass (atom_graph_kernel<Real, gm>: 0 energy pass, 1 gate
-// forward, 2 gate reverse): returns 1 or throws.
-template <typename Real>
-int launch_atom_graph(const PassArgs<Real>& args, int sm_count, cudaStream_t stream, int gm = 0);
+// The per-atom graph kernel of a split pass (graph_block_kernel<gm>: 0 energy pass, 1 gate forward,
+// 2 gate reverse): returns 1 or throws.
+int launch_atom_graph(const PassArgs<float>& args, int sm_count, cudaStream_t stream, int gm);
+// Whether a pass's nodes fit that kernel's shared memory (the pass runs fused otherwise).
+bool graph_block_fits(const BlockProg& g, int F, int S);
+// The per-atom gate-signal adjoints a.hbar from the per-edge contributions (hbar_sum_kernel).
+int launch_hbar_sum(const PassArgs<float>& args, cudaStream_t stream);
 
 // Per-translation-unit constant-table upload (spherical-harmonic normalisation) of every unit.
 template <typename Real>

@@ -190,9 +190,9 @@ class Engine:
         check(load().sus2g_engine_set_grad_split(self._h, 1 if on else 0))
 
     def set_static_split(self, on: bool) -> None:
-        """FP32 engines, basis size 8: every per-atom pass split at the per-atom boundary (the
-        energy pass as forward / per-atom graph / adjoint kernels, the Effect gate passes as two
-        kernels each) instead of fused; the autotuner chooses per pass."""
+        """FP32 engines, basis size 8: every per-atom pass split at the per-atom boundary (forward /
+        per-atom graph / adjoint kernels) instead of fused.  Without this call the number of centres
+        decides (pinned pass shapes run fused), or the autotuner once it has run."""
         check(load().sus2g_engine_set_static_split(self._h, 1 if on else 0))
 
     def set_moment_mma(self, on: bool) -> None:

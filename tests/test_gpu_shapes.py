@@ -119,3 +119,22 @@ def test_efs_and_gradient_of_every_layout(engine_lib, oracle_lib, tmp_path, shap
                 assert np.max(np.abs(e - e0) / n) <= FP32_ENERGY
         grad = g.combination_grad(frs, ew, fw, sw)
         assert np.linalg.norm(grad - g0) <= GRAD_TOL[prec == sg.FP32] * np.linalg.norm(g0)
+
+
+def test_staged_evaluation_keeps_the_form_it_began_in(engine_lib, tmp_path):
+    """The split gate passes keep their values in another layout than the fused ones: a switch
+    between begin and finish takes effect with the next evaluation."""
+    import superlinear_gb300 as sg
+    path = write_model(tmp_path / "m.sus2", 3, 4, 2, 8, True, "K", 1.0, 5)
+    fr = frames(2, 9)[2]
+    g = sg.Engine(sg.Model(path), 0, sg.FP32)
+    e0, f0, _, _ = g.calc_efs([fr])
+    ei, ej, d = g.edges()
+    for begin in (False, True):
+        g.set_static_split(begin)
+        g.stage_begin(fr.natoms, fr.types, ei, ej, d)
+        g.set_static_split(not begin)
+        g.stage_outer()
+        e, s, f, v = g.stage_finish(fr.natoms, fr.natoms)
+        assert np.linalg.norm(f - f0) <= FP32_FORCE * np.linalg.norm(f0)
+        assert abs(e - e0[0]) / fr.natoms <= FP32_ENERGY
