@@ -115,19 +115,26 @@ __global__ void k_loss(int nframes, const int* fbegin, const double* E, const do
 // Effect gate-x L2 term of one frame (block per frame; MLMTPR::AddTwoLayerGateX2Penalty,
 // dev_src/mtpr_sh.cpp:5869-6047):  P_f = sum over edges (i -> j) of norm(t_j) sum_mu (alpha(t_j, mu)
 // h_j[mu])^2 with norm(t) = coeff / (active types x F x edges whose neighbour type is t).  Edges
-// are symmetric, so the edges with neighbour j number deg(j) = row_end[j] - row[j].  Adds P_f to
-// loss_f[f]; writes dP/dh_j to extra_h[j] (the gate-chain seed) and the frame's dP/dalpha to
-// agrad[f][t F + mu]; fixed-order sums throughout.
+// are symmetric, so the edges with neighbour j number deg(j) = row_end[j] - row[j].  The frames' sum
+// joins the loss; dP/dh_j goes to extra_h[j] (the gate-chain seed) and the frame's dP/dalpha to
+// agrad[f][t F + mu]; fixed-order sums throughout.  With S[t][mu] = sum_j of type t of deg(j) norm(t) h_j[mu]^2,
+// dP/dalpha = 2 alpha S and the term is sum alpha^2 S = sum alpha / 2 dP/dalpha, which k_gatex_alpha
+// forms from the frame sums.  Block (frame, kGatexMu functions), threads of a fixed mu taking the
+// frame's atoms in rows: h and extra_h move in whole sectors, an element costs a handful of FP64
+// operations (1/64 rate: what bounds it), and the largest frame's share is spread over several SMs.
+// One block per frame with a thread per atom, its own divisions and a second pass over the atoms
+// per alpha had taken 157 us for 256 frames of 8-216 atoms (F = 16), 277 us for 96 frames of 16-512
+// (F = 48); 28 and 56 us now.
+constexpr int kGatexThreads = 256, kGatexMu = 8, kGatexRows = kGatexThreads / kGatexMu;
 template <typename Real>
-__global__ void k_gatex_frame(int nframes, const int* fbegin, const int* row, const int* row_end, const int* types,
-                              const Real* h,
-                              const Real* alpha, int C, int F, double coeff, double* extra_h, double* loss_f,
-                              double* agrad) {
+__global__ void __launch_bounds__(kGatexThreads) k_gatex_frame(int nframes, const int* fbegin, const int* row,
+                                                               const int* row_end, const int* types, const Real* h,
+                                                               const Real* alpha, int C, int F, double coeff,
+                                                               double* extra_h, double* agrad) {
   const int f = blockIdx.x;
-  if (f >= nframes) return;
   const int a0 = fbegin[f], a1 = fbegin[f + 1];
   __shared__ unsigned long long count[64];
-  __shared__ double red[256];
+  __shared__ double red[kGatexThreads];
   for (int t = threadIdx.x; t < C; t += blockDim.x) count[t] = 0;
   __syncthreads();
   for (int j = a0 + threadIdx.x; j < a1; j += blockDim.x)
@@ -135,47 +142,46 @@ __global__ void k_gatex_frame(int nframes, const int* fbegin, const int* row, co
   __syncthreads();
   int active = 0;
   for (int t = 0; t < C; ++t) active += count[t] > 0;
-  auto weight = [&](int j) {  // deg(j) norm(t_j)
-    const int t = types[j], deg = row_end[j] - row[j];
-    return deg > 0 ? coeff * deg / (double(active) * F * double(count[t])) : 0.0;
-  };
-  double pen = 0.0;
-  for (int j = a0 + threadIdx.x; j < a1; j += blockDim.x) {
-    const double w = weight(j);
-    const int t = types[j];
-    for (int mu = 0; mu < F; ++mu) {
-      const double al = double(alpha[t * F + mu]), x = al * double(h[static_cast<size_t>(j) * F + mu]);
-      pen += w * x * x;
-      extra_h[static_cast<size_t>(j) * F + mu] = 2.0 * w * x * al;
+  const int r = threadIdx.x / kGatexMu, mu = blockIdx.y * kGatexMu + threadIdx.x % kGatexMu;
+  for (int t = 0; t < C; ++t) {
+    const double al = mu < F ? double(alpha[t * F + mu]) : 0.0;
+    const double norm = count[t] > 0 ? coeff / (double(active) * F * double(count[t])) : 0.0;
+    const double e2 = 2.0 * norm * al * al;
+    double sum = 0.0;
+    if (mu < F) {
+#pragma unroll 4
+      for (int j = a0 + r; j < a1; j += kGatexRows)
+        if (types[j] == t) {
+          const size_t at = static_cast<size_t>(j) * F + mu;
+          const double hj = double(h[at]), dh = double(row_end[j] - row[j]) * hj;
+          extra_h[at] = e2 * dh;
+          sum += dh * hj;
+        }
     }
-  }
-  red[threadIdx.x] = pen;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
     __syncthreads();
-  }
-  if (threadIdx.x == 0) loss_f[f] += red[0];
-  for (int q = threadIdx.x; q < C * F; q += blockDim.x) {
-    const int t = q / F, mu = q - t * F;
-    const double al = double(alpha[q]);
-    double g = 0.0;
-    for (int j = a0; j < a1; ++j)
-      if (types[j] == t) {
-        const double hj = double(h[static_cast<size_t>(j) * F + mu]);
-        g += 2.0 * weight(j) * al * hj * hj;
-      }
-    agrad[static_cast<size_t>(f) * C * F + q] = g;
+    red[threadIdx.x] = sum;
+    __syncthreads();
+    for (int st = kGatexRows / 2; st > 0; st >>= 1) {
+      if (r < st) red[threadIdx.x] += red[threadIdx.x + st * kGatexMu];
+      __syncthreads();
+    }
+    if (r == 0 && mu < F) agrad[static_cast<size_t>(f) * C * F + t * F + mu] = 2.0 * norm * al * red[threadIdx.x];
   }
 }
 
-// grad[q] += sum over frames of agrad[f][q] (frame order)
-__global__ void k_gatex_alpha(int nframes, int n, const double* agrad, double* grad) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+// grad[q] += sum over frames of agrad[f][q], a warp per entry (fixed order); pen[q] = the entry's
+// share of the term's value
+template <typename Real>
+__global__ void k_gatex_alpha(int nframes, int n, const double* agrad, const Real* alpha, double* grad, double* pen) {
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
   if (q >= n) return;
   double s = 0.0;
-  for (int f = 0; f < nframes; ++f) s += agrad[static_cast<size_t>(f) * n + q];
-  grad[q] += s;
+  for (int f = threadIdx.x % kWarp; f < nframes; f += kWarp) s += agrad[static_cast<size_t>(f) * n + q];
+  s = warp_sum(s);
+  if (threadIdx.x % kWarp == 0) {
+    grad[q] += s;
+    pen[q] = 0.5 * double(alpha[q]) * s;
+  }
 }
 
 // Error-metric partial sums of one frame (block per frame), as NonLinearRegression::AddLoss collects
@@ -336,14 +342,17 @@ __global__ void k_lin_normal(long long rows, int ncol, const double* cm, const d
   }
 }
 
-// loss = sum_f loss_f / K (fixed order), grad /= K
-__global__ void k_loss_finish(int nframes, const double* loss_f, double* loss, double* grad, int nparams) {
+// loss = (sum_f loss_f + sum_q pen_q) / K (fixed order, by the first warp), grad /= K
+__global__ void k_loss_finish(int nframes, const double* loss_f, int npen, const double* pen, double* loss, double* grad,
+                              int nparams) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const double inv = nframes > 0 ? 1.0 / nframes : 0.0;
-  if (t == 0) {
+  if (t < kWarp) {
     double s = 0.0;
-    for (int f = 0; f < nframes; ++f) s += loss_f[f];
-    *loss = s * inv;
+    for (int f = t; f < nframes; f += kWarp) s += loss_f[f];
+    for (int q = t; q < npen; q += kWarp) s += pen[q];
+    s = warp_sum(s);
+    if (t == 0) *loss = s * inv;
   }
   if (t < nparams) grad[t] *= inv;
 }
@@ -594,6 +603,7 @@ class Trainer {
       if (m.C > 64) throw Error(1, "gate-x term: more than 64 species");
       extra_h_.ensure(sizeof(double) * static_cast<size_t>(natoms_) * m.F);
       agrad_.ensure(sizeof(double) * static_cast<size_t>(std::max(1, nframes)) * m.C * m.F);
+      pen_.ensure(sizeof(double) * m.C * m.F);
     }
     TRAIN_CUDA(cudaMallocHost(&host_scalars_, sizeof(double) * 8));
     bind_edges();
@@ -634,31 +644,33 @@ class Trainer {
                                       E0_.as<double>(), F0_.as<double>(), S0_.as<double>(), has_.as<int>(), cfg_,
                                       ew_.as<double>(), fw_.as<double>(), sw_.as<double>(), lossf_.as<double>());
     const Model& m = eng_.model();
+    const int npen = gatex_ ? m.C * m.F : 0;
+    auto gatex_frames = [&](auto* h) {
+      using Real = typename std::remove_const<typename std::remove_pointer<decltype(h)>::type>::type;
+      k_gatex_frame<Real><<<dim3(nframes_, (m.F + kGatexMu - 1) / kGatexMu), kGatexThreads, 0, s>>>(
+          nframes_, fbegin_.as<int>(), eng_.d_row(), eng_.d_row_end(), types_.as<int>(), h,
+          static_cast<const Real*>(eng_.d_gate_additive()), m.C, m.F, cfg_.gate_x_l2, extra_h_.as<double>(), agrad_.as<double>());
+    };
+    auto gatex_alpha = [&](auto* alpha) {
+      using Real = typename std::remove_const<typename std::remove_pointer<decltype(alpha)>::type>::type;
+      k_gatex_alpha<Real><<<(npen * kWarp + 255) / 256, 256, 0, s>>>(nframes_, npen, agrad_.as<double>(), alpha,
+                                                                   grad_.as<double>() + eng_.gate_additive_offset(),
+                                                                   pen_.as<double>());
+    };
     if (gatex_) {
-      if (eng_.precision() == kFP32)
-        k_gatex_frame<float><<<nframes_, 256, 0, s>>>(nframes_, fbegin_.as<int>(), eng_.d_row(), eng_.d_row_end(),
-                                                      types_.as<int>(),
-                                                      static_cast<const float*>(eng_.d_gate_signal()),
-                                                      static_cast<const float*>(eng_.d_gate_additive()), m.C, m.F,
-                                                      cfg_.gate_x_l2, extra_h_.as<double>(), lossf_.as<double>(),
-                                                      agrad_.as<double>());
-      else
-        k_gatex_frame<double><<<nframes_, 256, 0, s>>>(nframes_, fbegin_.as<int>(), eng_.d_row(), eng_.d_row_end(),
-                                                       types_.as<int>(),
-                                                       static_cast<const double*>(eng_.d_gate_signal()),
-                                                       static_cast<const double*>(eng_.d_gate_additive()), m.C, m.F,
-                                                       cfg_.gate_x_l2, extra_h_.as<double>(), lossf_.as<double>(),
-                                                       agrad_.as<double>());
+      if (eng_.precision() == kFP32) gatex_frames(static_cast<const float*>(eng_.d_gate_signal()));
+      else gatex_frames(static_cast<const double*>(eng_.d_gate_signal()));
     }
     TRAIN_CUDA(cudaMemsetAsync(grad_.ptr, 0, sizeof(double) * nparams_, s));
     if (natoms_)
       eng_.combination_grad(ew_.as<double>(), fw_.as<double>(), sw_.as<double>(), grad_.as<double>(),
                             gatex_ ? extra_h_.as<double>() : nullptr);
-    if (gatex_)
-      k_gatex_alpha<<<(m.C * m.F + 255) / 256, 256, 0, s>>>(nframes_, m.C * m.F, agrad_.as<double>(),
-                                                           grad_.as<double>() + eng_.gate_additive_offset());
-    k_loss_finish<<<(nparams_ + 255) / 256, 256, 0, s>>>(nframes_, lossf_.as<double>(), loss_.as<double>(),
-                                                         grad_.as<double>(), nparams_);
+    if (gatex_) {
+      if (eng_.precision() == kFP32) gatex_alpha(static_cast<const float*>(eng_.d_gate_additive()));
+      else gatex_alpha(static_cast<const double*>(eng_.d_gate_additive()));
+    }
+    k_loss_finish<<<(nparams_ + 255) / 256, 256, 0, s>>>(nframes_, lossf_.as<double>(), npen, pen_.as<double>(),
+                                                         loss_.as<double>(), grad_.as<double>(), nparams_);
   }
 
   // Loss and gradient at the parameters already in the engine; results stay on the device.
@@ -1243,7 +1255,7 @@ class Trainer {
   DevBuf pos_, types_, E0_, F0_, S0_, has_, fbegin_;
   DevBuf E_, F_, V_, ew_, fw_, sw_, lossf_, loss_, grad_;
   bool gatex_ = false;
-  DevBuf extra_h_, agrad_;  // gate-x term: dP/dh per atom, dP/dalpha per frame
+  DevBuf extra_h_, agrad_, pen_;  // gate-x term: dP/dh per atom, dP/dalpha per frame
   DevBuf metric_part_;
   DevBuf lin_cm_, lin_alpha_, lin_rhs_, lin_A_, lin_b_;  // linear warm-up
   double* host_scalars_ = nullptr;
