@@ -78,7 +78,7 @@ struct GraphProg {
 
 // The same program for the block-per-32-centres kernel (graph_block.cuh; FP32 engines): node values
 // and adjoints in numbered slots, each step's target lists dealt to the block's warps.
-constexpr int kGraphWarps = 16;       // warps of a block
+constexpr int kGraphWarps = 16;       // warps of a block; twice as many where only one block fits an SM
 constexpr int kGraphAtoms = 32;       // centres of a block
 constexpr int kGraphMaxSlots = 4095;  // 12-bit slots in the packed records
 // A unit is two terms.  Words x and z hold a term's slots, a at bits 7-18 and b at bits 20-31 (a slot
@@ -89,9 +89,11 @@ constexpr unsigned kUnitChunkEnd = 1u << 5, kUnitListEnd = 1u << 6, kUnitStepEnd
 struct BlockProg {
   int nslots = 0;                         // 0: the pass has no such program (too many nodes)
   int one = 0;                            // slot of the constant 1
+  int warps = 0;                          // warps of a block (the lists are dealt to them)
   int nzero_v = 0, nzero_adj = 0, nkeep = 0;
   const int4* units = nullptr;            // term pairs (graph_block.cuh)
-  const int* begin = nullptr;             // [warps][3] the warp's stream: forward, reverse, end
+  const int* begin = nullptr;             // [warps][4] the warp's stream: forward, reverse, the
+                                          // contraction's reverse (gradient programs), end
   const int* basic_slot = nullptr;        // [K H] value slot of moment t, -1 when absent
   const int* basic_adj = nullptr;         // [K H] its adjoint slot
   const int* zero_v = nullptr;            // value slots that start at zero
@@ -99,6 +101,12 @@ struct BlockProg {
   const int* seed_v = nullptr;            // [S] (outer) / [Q] (gate): slots of the scalars
   const int* seed_adj = nullptr;
   const int* keep = nullptr;              // [nkeep] value slots the reverse reads
+  // gradient programs: adjoint slots zeroed before the contraction's reverse (until then they hold
+  // the values the rank-weight gradients read), and the slots of each rank-weight row
+  int nzero_late = 0;
+  const int* zero_late = nullptr;
+  const int* rank_v = nullptr;
+  const int* rank_adj = nullptr;
 };
 
 // Per-pass tables: the outer (energy) pass and the Effect gate pass share this layout.
@@ -135,6 +143,7 @@ struct PassTables {
   const Real* rprod_c;
   GraphProg<Real> prog;   // the same contraction and graph as a lane-balanced program (E/F/virial passes)
   BlockProg block;        // and as a block program (FP32 split passes)
+  BlockProg dual;         // and as one for values and tangents (FP32 split gradient)
 };
 
 // Parameter-vector offsets (the trainer's Coeff() order) and the gradient-only tables of one pass.

@@ -825,8 +825,8 @@ struct HostBlockProg {
   struct Term { int a, b, widx; double c; };
   struct Unit { Term t[2]; int target; bool chunk_end, list_end, step_end; };
   std::vector<Unit> units;
-  std::vector<int> begin, basic_slot, basic_adj, zero_v, zero_adj, seed_v, seed_adj, keep;
-  int nslots = 0, one = 0;
+  std::vector<int> begin, basic_slot, basic_adj, zero_v, zero_adj, seed_v, seed_adj, keep, zero_late, rank_v, rank_adj;
+  int nslots = 0, one = 0, warps = 0;
 };
 
 namespace {
@@ -1072,7 +1072,9 @@ HostProg build_prog(const Model& m, bool gate) {
   return hp;
 }
 
-HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::vector<int>& basic_of) {
+// dual: the gradient's program.  Its rank-weight gradients read the contraction's source values just
+// before the contraction's reverse, the last step, which the streams then set apart.
+HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::vector<int>& basic_of, bool dual) {
   HostBlockProg bp;
   const int nsteps = static_cast<int>(hp.steps.size());
   const std::vector<int>& seeds = hp.gate ? m.gate_nodes : m.scalar_map;
@@ -1080,12 +1082,21 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
   // each step's target lists from the lane streams: chunk = terms up to a flush, list = its chunks
   struct List { int target; std::vector<std::vector<HostProg::Rec>> chunks; };
   std::vector<std::vector<List>> steps(nsteps);
-  std::vector<char> in_v(m.M, 0), in_adj(m.M, 0), rev_b(m.M, 0);
+  std::vector<char> in_v(m.M, 0), in_adj(m.M, 0), rev_b(m.M, 0), early(m.M, 0), rank_src(m.M, 0);
+  const std::vector<ContractionRow>& rank_rows = hp.gate ? m.gate_rows : m.outer_rows;
+  const bool apart = dual && !rank_rows.empty();
+  if (dual)
+    for (const auto& r : rank_rows)
+      if (r.widx >= 0) rank_src[r.src] = 1;
   for (int st = 0; st < nsteps; ++st) {
     const auto& info = hp.steps[st];
     const bool rev = (info[3] & 1) != 0;
     std::map<int, std::vector<HostProg::Rec>> parts;
-    auto mark = [&](int target) { (rev ? in_adj : in_v)[target] = 1; };
+    const bool last = apart && st + 1 == nsteps;
+    auto mark = [&](int target) {
+      (rev ? in_adj : in_v)[target] = 1;
+      if (rev && !last) early[target] = 1;
+    };
     for (int lane = 0; lane < kWarp; ++lane) {
       std::vector<HostProg::Rec> chunk;
       for (int i = 0; i < info[1]; ++i) {
@@ -1094,7 +1105,7 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
         if (r.flush == kProgNoFlush) continue;
         for (const auto& t : chunk) {
           const int x = static_cast<int>(t.ab & 0xffffu), y = static_cast<int>(t.ab >> 16);
-          if (x != one) (rev ? in_adj : in_v)[x] = 1;
+          if (x != one) mark(x);
           if (y != one) { in_v[y] = 1; if (rev) rev_b[y] = 1; }
         }
         if (r.flush >= 0) {
@@ -1121,7 +1132,7 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
   std::vector<char> is_basic(m.M, 0), is_seed(m.M, 0);
   for (int b : basic_of)
     if (b >= 0) { is_basic[b] = 1; in_adj[b] = 1; if (vslot[b] < 0) vslot[b] = n++; }
-  for (int q : seeds) { is_seed[q] = 1; in_v[q] = in_adj[q] = 1; }
+  for (int q : seeds) { is_seed[q] = 1; in_v[q] = in_adj[q] = early[q] = 1; }
   for (int q = 0; q < m.M; ++q)
     if (in_v[q] && vslot[q] < 0) {
       vslot[q] = n++;
@@ -1130,22 +1141,32 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
   bp.one = n++;
   for (int q = 0; q < m.M; ++q)
     if (in_adj[q]) {
-      aslot[q] = vslot[q] >= 0 && !rev_b[q] ? vslot[q] : n++;
-      if (!is_seed[q]) bp.zero_adj.push_back(aslot[q]);
+      const bool share = vslot[q] >= 0 && !rev_b[q] && !(rank_src[q] && early[q]);
+      aslot[q] = share ? vslot[q] : n++;
+      if (share && rank_src[q]) bp.zero_late.push_back(aslot[q]);
+      else if (!is_seed[q]) bp.zero_adj.push_back(aslot[q]);
     }
   if (n > kGraphMaxSlots) return HostBlockProg{};
   bp.nslots = n;
+  const int warps = bp.warps = graph_program_warps(n, m.F, m.S);
   for (int b : basic_of) {
     bp.basic_slot.push_back(b >= 0 ? vslot[b] : -1);
     bp.basic_adj.push_back(b >= 0 ? aslot[b] : -1);
   }
   for (int q : seeds) { bp.seed_v.push_back(vslot[q]); bp.seed_adj.push_back(aslot[q]); }
   for (int q = 0; q < m.M; ++q)
-    if (rev_b[q]) bp.keep.push_back(vslot[q]);
+    if (rev_b[q] || rank_src[q]) bp.keep.push_back(vslot[q]);
+  if (dual)
+    for (int w = 0; w < static_cast<int>((hp.gate ? m.gate_w : m.outer_w).size()); ++w)
+      for (const auto& r : rank_rows)
+        if (r.widx == w) {
+          bp.rank_v.push_back(vslot[r.src]);
+          bp.rank_adj.push_back(aslot[r.dst]);
+        }
   // streams: lists longest first onto the least-loaded warp
   const HostBlockProg::Term pad{bp.one, bp.one, -1, 0.0};
-  std::vector<std::vector<HostBlockProg::Unit>> stream(kGraphWarps);
-  std::vector<int> fwd_end(kGraphWarps, 0);
+  std::vector<std::vector<HostBlockProg::Unit>> stream(warps);
+  std::vector<int> fwd_end(warps, 0), last_begin(warps, -1);
   auto fours = [&](std::vector<HostBlockProg::Unit>& v) {
     while (v.size() % 4) v.push_back({{pad, pad}, 0, false, false, false});
   };
@@ -1159,7 +1180,12 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
       cost.push_back(c);
     }
     std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return cost[x] > cost[y]; });
-    std::vector<size_t> load(kGraphWarps, 0);
+    if (apart && st + 1 == nsteps)
+      for (int w = 0; w < warps; ++w) {
+        fours(stream[w]);
+        last_begin[w] = static_cast<int>(stream[w].size());
+      }
+    std::vector<size_t> load(warps, 0);
     for (size_t q : order) {
       const int w = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
       load[w] += cost[q];
@@ -1182,7 +1208,7 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
       }
     }
     // the step's last unit carries the barrier (a unit of its own for a warp without lists)
-    for (int w = 0; w < kGraphWarps; ++w) {
+    for (int w = 0; w < warps; ++w) {
       if (load[w] == 0) stream[w].push_back({{pad, pad}, 0, false, false, false});
       stream[w].back().step_end = true;
       if (st + 1 == hp.nfwd) {
@@ -1191,11 +1217,12 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
       }
     }
   }
-  for (int w = 0; w < kGraphWarps; ++w) {
+  for (int w = 0; w < warps; ++w) {
     fours(stream[w]);
     const int first = static_cast<int>(bp.units.size());
     bp.begin.push_back(first);
     bp.begin.push_back(first + fwd_end[w]);
+    bp.begin.push_back(first + (last_begin[w] >= 0 ? last_begin[w] : static_cast<int>(stream[w].size())));
     bp.units.insert(bp.units.end(), stream[w].begin(), stream[w].end());
     bp.begin.push_back(static_cast<int>(bp.units.size()));
   }
@@ -1213,7 +1240,7 @@ void upload_block_progs(const Model& m, const HostBlockProg* const (&progs)[2], 
     if (n) std::memcpy(img.data() + o, p, n);
     return o;
   };
-  size_t off[2][9];
+  size_t off[2][12];
   for (int k = 0; k < 2; ++k) {
     const HostBlockProg& bp = *progs[k];
     const std::vector<double>& w = k ? m.gate_w : m.outer_w;
@@ -1237,8 +1264,8 @@ void upload_block_progs(const Model& m, const HostBlockProg* const (&progs)[2], 
     }
     off[k][0] = put(units.data(), sizeof(int4) * units.size());
     const std::vector<int>* lists[] = {&bp.begin, &bp.basic_slot, &bp.basic_adj, &bp.zero_v, &bp.zero_adj, &bp.seed_v, &bp.seed_adj,
-                                       &bp.keep};
-    for (int i = 0; i < 8; ++i) off[k][1 + i] = put(lists[i]->data(), sizeof(int) * lists[i]->size());
+                                       &bp.keep, &bp.zero_late, &bp.rank_v, &bp.rank_adj};
+    for (int i = 0; i < 11; ++i) off[k][1 + i] = put(lists[i]->data(), sizeof(int) * lists[i]->size());
   }
   buf.ensure(img.size());
   SUS2G_CUDA(cudaMemcpyAsync(buf.ptr, img.data(), img.size(), cudaMemcpyHostToDevice, s));
@@ -1248,14 +1275,15 @@ void upload_block_progs(const Model& m, const HostBlockProg* const (&progs)[2], 
     const HostBlockProg& bp = *progs[k];
     auto ints = [&](int i) { return reinterpret_cast<const int*>(base + off[k][i]); };
     BlockProg g;
-    g.nslots = bp.nslots; g.one = bp.one;
+    g.nslots = bp.nslots; g.one = bp.one; g.warps = bp.warps;
     g.nzero_v = static_cast<int>(bp.zero_v.size());
     g.nzero_adj = static_cast<int>(bp.zero_adj.size());
     g.nkeep = static_cast<int>(bp.keep.size());
     g.units = reinterpret_cast<const int4*>(base + off[k][0]);
     g.begin = ints(1); g.basic_slot = ints(2); g.basic_adj = ints(3); g.zero_v = ints(4); g.zero_adj = ints(5);
     g.seed_v = ints(6); g.seed_adj = ints(7);
-    g.keep = ints(8);
+    g.nzero_late = static_cast<int>(bp.zero_late.size());
+    g.keep = ints(8); g.zero_late = ints(9); g.rank_v = ints(10); g.rank_adj = ints(11);
     out[k] = g;
   }
 }
@@ -1380,15 +1408,23 @@ void Engine::wait_reverse() {
   rev_pending_ = false;
 }
 
+namespace {
+// basic index of (k, l, m) at k H + l l + l + m, -1 when absent
+std::vector<int> basic_table(const Model& m) {
+  std::vector<int> t(static_cast<size_t>(m.K) * m.H, -1);
+  for (int b = 0; b < m.NB; ++b) {
+    const auto& q = m.basic[b];
+    t[static_cast<size_t>(q[0]) * m.H + q[1] * q[1] + q[1] + q[2]] = b;
+  }
+  return t;
+}
+}  // namespace
+
 template <typename Real>
 void Engine::upload_tables() {
   const Model& m = model_;
   Packer pk;
-  std::vector<int> basic_of(static_cast<size_t>(m.K) * m.H, -1);
-  for (int b = 0; b < m.NB; ++b) {
-    const auto& q = m.basic[b];
-    basic_of[static_cast<size_t>(q[0]) * m.H + q[1] * q[1] + q[1] + q[2]] = b;
-  }
+  const std::vector<int> basic_of = basic_table(m);
   const int o_basic = pk.add_int(basic_of);
   PassOffsets po = pack_pass(m, false, pk);
   PassOffsets pg = m.gated ? pack_pass(m, true, pk) : po;
@@ -1489,17 +1525,6 @@ void Engine::upload_tables() {
     dm->outer.prog = bound[0];
     dm->gate.prog = m.gated ? bound[1] : bound[0];
     dm->prog_parts = std::max(bound[0].max_parts, m.gated ? bound[1].max_parts : 0);
-    if (sizeof(Real) == 4 && m.B == 8) {  // the engines that can run the split passes
-      if (!block_prog_[0]) {
-        block_prog_[0].reset(new HostBlockProg(build_block_prog(m, *prog_[0], basic_of)));
-        block_prog_[1].reset(new HostBlockProg(m.gated ? build_block_prog(m, *prog_[1], basic_of) : HostBlockProg{}));
-      }
-      BlockProg blocks[2];
-      const HostBlockProg* const hosts[2] = {block_prog_[0].get(), block_prog_[1].get()};
-      upload_block_progs(m, hosts, tab_block_, us, blocks);
-      dm->outer.block = blocks[0];
-      dm->gate.block = blocks[1];
-    }
   }
   dm->linear = R + o_lin;
   dm->species = tab_dbl_.as<double>();
@@ -1513,6 +1538,28 @@ void Engine::upload_tables() {
   dm->grad = gl;
   delete static_cast<DevModel<Real>*>(dev_model_);
   dev_model_ = dm;
+  if constexpr (sizeof(Real) == 4) {
+    if (block_prog_[0]) upload_block_programs(false);
+    if (dual_prog_[0]) upload_block_programs(true);
+  }
+}
+
+// The block programs of the split passes (dual: of the split gradient), from their first use on: the
+// structure is built once per engine, uploads refresh the rank weights.
+void Engine::upload_block_programs(bool dual) {
+  const Model& m = model_;
+  auto* dm = static_cast<DevModel<float>*>(dev_model_);
+  auto& host = dual ? dual_prog_ : block_prog_;
+  if (!host[0]) {
+    const std::vector<int> basic_of = basic_table(m);
+    host[0].reset(new HostBlockProg(build_block_prog(m, *prog_[0], basic_of, dual)));
+    host[1].reset(new HostBlockProg(m.gated ? build_block_prog(m, *prog_[1], basic_of, dual) : HostBlockProg{}));
+  }
+  BlockProg blocks[2];
+  const HostBlockProg* const hosts[2] = {host[0].get(), host[1].get()};
+  upload_block_progs(m, hosts, dual ? tab_dual_ : tab_block_, stream_ ? stream_ : own_stream_, blocks);
+  (dual ? dm->outer.dual : dm->outer.block) = blocks[0];
+  (dual ? dm->gate.dual : dm->gate.block) = blocks[1];
 }
 
 void Engine::upload_model() {
@@ -2006,7 +2053,8 @@ PassArgs<Real> Engine::pass_args() {
   if (m.gated) {
     hsig_.ensure(sizeof(Real) * static_cast<size_t>(std::max(1, N)) * m.F);
     hcontrib_.ensure(sizeof(Real) * E * m.F);
-    gmom_.ensure(sizeof(Real) * static_cast<size_t>(std::max(1, N)) * m.M);
+    // (a split gate pass keeps its own values, launch_gate_split)
+    if (!use_gate_split<Real>()) gmom_.ensure(sizeof(Real) * static_cast<size_t>(std::max(1, N)) * m.M);
     a.hsig = hsig_.as<Real>();
     a.hcontrib = hcontrib_.as<Real>();
     a.gmom = gmom_.as<Real>();
@@ -2019,6 +2067,8 @@ void Engine::run_efs(double* d_energy, double* d_forces, double* d_virial, doubl
   const Model& m = model_;
   cudaStream_t s = stream_;
   const int N = natoms_;
+  if (sizeof(Real) == 4 && m.B == 8 && !block_prog_[0] && (wants_split(static_split_) || (m.gated && wants_split(gate_split_))))
+    upload_block_programs(false);
   PassArgs<Real> a = pass_args<Real>();
   // stage 1: gate forward (Effect) -- gate signals of the centre atoms
   if (stages & kStageGate) {
@@ -2211,6 +2261,8 @@ void Engine::run_grad(const double* ew, const double* fw, const double* sw, doub
   cudaStream_t s = stream_;
   const int N = natoms_, P = m.param_count();
   const size_t E = std::max<long long>(1, nedges_);
+  if constexpr (sizeof(Real) == 4)
+    if (m.B == 8 && !dual_prog_[0]) upload_block_programs(true);
   const DevModel<Real>& dm = *static_cast<DevModel<Real>*>(dev_model_);
   GradArgs<Real> a{};
   a.dm = dm;
@@ -2228,21 +2280,57 @@ void Engine::run_grad(const double* ew, const double* fw, const double* sw, doub
   a.extra_h = extra_h;
   a.error = error_.as<int>();
   // the outer and gate reverse passes whole, or split into their per-atom and per-edge parts
-  // (basis size 8) through the moment adjoints in gabar_
+  // (basis size 8) through the moment adjoints in gabar_.  Split, the per-edge part runs as
+  // grad_edge_kernel where the model's warps are per channel and its sums fit in shared memory, and
+  // FP32 engines run the per-atom part as the edge->moment kernel and the block graph kernel where
+  // the nodes fit; the other forms of grad_pass_kernel cover what is left.
   const bool split = grad_split_ && m.B == 8;
   const int part1 = split ? kGradAtomPart : kGradWhole;
-  const GradLaunch co = grad_pass_config<Real>(m.L, kGradOuter, dm, ncentres_, sm_count_, part1);
-  GradLaunch co2 = co, cf = co, cr = co, cr2 = co;
-  if (split) co2 = grad_pass_config<Real>(m.L, kGradOuter, dm, ncentres_, sm_count_, kGradEdgePart);
-  if (m.gated) {
-    cf = grad_pass_config<Real>(m.L, kGradGateForward, dm, ncentres_, sm_count_);
-    cr = grad_pass_config<Real>(m.L, kGradGateReverse, dm, ncentres_, sm_count_, part1);
-    cr2 = split ? grad_pass_config<Real>(m.L, kGradGateReverse, dm, ncentres_, sm_count_, kGradEdgePart) : cr;
-  }
-  const int nslots = std::max({co.grid * co.warps, co2.grid * co2.warps, cf.grid * cf.warps, cr.grid * cr.warps,
-                               cr2.grid * cr2.warps});
+  bool dual = false;
+  if constexpr (sizeof(Real) == 4) dual = split && grad_graph_fits(dm, m.gated);
+  GradLaunch gm_o{}, gm_g{}, gg[3] = {}, ge_o{}, ge_g{}, gw{}, co{}, co2{}, cf{}, cr{}, cr2{};
+  int nslots = 0;
+  auto slices = [&](const GradLaunch& c, bool per_block) { nslots = std::max(nslots, per_block ? c.grid : c.grid * c.warps); };
   if (split) {
-    gabar_.ensure(sizeof(Real) * static_cast<size_t>(std::max(1, ncentres_)) * 2 * m.K * (m.L + 1) * (m.L + 1));
+    ge_o = grad_edge_config<Real>(m.L, kGradOuter, dm, ncentres_, sm_count_);
+    if (m.gated) ge_g = grad_edge_config<Real>(m.L, kGradGateReverse, dm, ncentres_, sm_count_);
+    slices(ge_o, true);
+    slices(ge_g, true);
+  }
+  if constexpr (sizeof(Real) == 4)
+    if (dual) {
+      gm_o = grad_moment_config(m.L, kGradOuter, dm, ncentres_, sm_count_);
+      for (int q = 0; q < (m.gated ? 3 : 1); ++q) {
+        gg[q] = grad_graph_config(q, dm, ncentres_, sm_count_);
+        slices(gg[q], true);
+      }
+      if (m.gated) {
+        gm_g = grad_moment_config(m.L, kGradGateForward, dm, ncentres_, sm_count_);
+        gw = grad_gate_weight_config(dm, ncentres_, sm_count_);
+        slices(gw, true);
+      }
+    }
+  if (!dual) {
+    co = grad_pass_config<Real>(m.L, kGradOuter, dm, ncentres_, sm_count_, part1);
+    slices(co, false);
+    if (m.gated) {
+      cf = grad_pass_config<Real>(m.L, kGradGateForward, dm, ncentres_, sm_count_);
+      cr = grad_pass_config<Real>(m.L, kGradGateReverse, dm, ncentres_, sm_count_, part1);
+      slices(cf, false);
+      slices(cr, false);
+    }
+  }
+  if (split && !ge_o.grid) {
+    co2 = grad_pass_config<Real>(m.L, kGradOuter, dm, ncentres_, sm_count_, kGradEdgePart);
+    slices(co2, false);
+  }
+  if (split && m.gated && !ge_g.grid) {
+    cr2 = grad_pass_config<Real>(m.L, kGradGateReverse, dm, ncentres_, sm_count_, kGradEdgePart);
+    slices(cr2, false);
+  }
+  const size_t NC = static_cast<size_t>(std::max(1, ncentres_)), KH2 = 2 * static_cast<size_t>(m.K) * m.H;
+  if (split) {
+    gabar_.ensure(sizeof(Real) * NC * KH2);
     a.abar = gabar_.as<Real>();
   }
   slots_.ensure(sizeof(double) * static_cast<size_t>(nslots) * P);
@@ -2252,37 +2340,67 @@ void Engine::run_grad(const double* ew, const double* fw, const double* sw, doub
     const size_t NF = static_cast<size_t>(std::max(1, N)) * m.F, NM = static_cast<size_t>(std::max(1, N)) * m.M;
     hsig_.ensure(sizeof(Real) * NF);
     hsigd_.ensure(sizeof(Real) * NF);
-    gmom_.ensure(sizeof(Real) * NM);
-    gmomd_.ensure(sizeof(Real) * NM);
     lhm_.ensure(sizeof(Real) * E * 2 * m.F);
     lh_atom_.ensure(sizeof(double) * 2 * NF);
     a.hsig = hsig_.as<Real>();
     a.hsigd = hsigd_.as<Real>();
-    a.gmom = gmom_.as<Real>();
-    a.gmomd = gmomd_.as<Real>();
     a.lhm = lhm_.as<Real>();
     a.lh_atom = lh_atom_.as<double>();
-    launches_ += launch_grad_pass<Real>(m.L, kGradGateForward, a, cf, s);
+    if (!dual) {
+      gmom_.ensure(sizeof(Real) * NM);
+      gmomd_.ensure(sizeof(Real) * NM);
+      a.gmom = gmom_.as<Real>();
+      a.gmomd = gmomd_.as<Real>();
+    }
+  }
+  if constexpr (sizeof(Real) == 4)
+    if (dual) {
+      const size_t blocks = (NC + kDualAtoms - 1) / kDualAtoms;
+      gdmom_.ensure(sizeof(Real) * NC * KH2);
+      a.mom = gdmom_.as<Real>();
+      if (m.gated) {
+        gdkeep_.ensure(sizeof(Real) * blocks * kWarp * std::max(1, dm.gate.dual.nkeep));
+        gdscal_.ensure(sizeof(Real) * blocks * kWarp * std::max(1, m.Q));
+        a.gkeep = gdkeep_.as<Real>();
+        a.gscal = gdscal_.as<Real>();
+        launches_ += launch_grad_moment(m.L, kGradGateForward, a, gm_g, s);
+        launches_ += launch_grad_graph(kGradGateForward, a, gg[kGradGateForward], s);
+      }
+      launches_ += launch_grad_moment(m.L, kGradOuter, a, gm_o, s);
+      launches_ += launch_grad_graph(kGradOuter, a, gg[kGradOuter], s);
+    }
+  if (!dual) {
+    if (m.gated) launches_ += launch_grad_pass<Real>(m.L, kGradGateForward, a, cf, s);
     launches_ += launch_grad_pass<Real>(m.L, kGradOuter, a, co, s);
-    if (split) launches_ += launch_grad_pass<Real>(m.L, kGradOuter, a, co2, s);
-    launches_ += launch_grad_pass<Real>(m.L, kGradGateReverse, a, cr, s);
-    if (split) launches_ += launch_grad_pass<Real>(m.L, kGradGateReverse, a, cr2, s);
+  }
+  if (ge_o.grid) launches_ += launch_grad_edge<Real>(m.L, kGradOuter, a, ge_o, s);
+  else if (split) launches_ += launch_grad_pass<Real>(m.L, kGradOuter, a, co2, s);
+  if (m.gated) {
+    if constexpr (sizeof(Real) == 4)
+      if (dual) {
+        launches_ += launch_lhm_sum(a, m.L + 1, s);
+        launches_ += launch_grad_graph(kGradGateReverse, a, gg[kGradGateReverse], s);
+      }
+    if (!dual) launches_ += launch_grad_pass<Real>(m.L, kGradGateReverse, a, cr, s);
+    if (ge_g.grid) launches_ += launch_grad_edge<Real>(m.L, kGradGateReverse, a, ge_g, s);
+    else if (split) launches_ += launch_grad_pass<Real>(m.L, kGradGateReverse, a, cr2, s);
     const int gw_off = dm.grad.gate_w_off;
     if (N && gw_off >= 0) {
-      const int blocks = std::max(1, std::min(nslots, (ncentres_ + kGwChunk - 1) / kGwChunk));
-      const size_t smem = sizeof(Real) * kGwChunk * 2 * (m.F + m.Q);
-      if (smem > 200 * 1024) throw Error(3, "gate weight gradient: radial functions + gate scalars exceed the shared-memory staging");
-      if (smem > 48 * 1024)
-        SUS2G_CUDA(cudaFuncSetAttribute(k_gate_weight_grad<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
-      k_gate_weight_grad<Real><<<blocks, kGwThreads, smem, s>>>(ncentres_, m.F, m.Q, m.M, dm.gate_nodes,
-                                                                lh_atom_.as<double>(), gmom_.as<Real>(),
-                                                                gmomd_.as<Real>(), slots_.as<double>(), P, gw_off);
-      ++launches_;
+      if constexpr (sizeof(Real) == 4)
+        if (dual) launches_ += launch_grad_gate_weight(a, gw, s);
+      if (!dual) {
+        const int blocks = std::max(1, std::min(nslots, (ncentres_ + kGwChunk - 1) / kGwChunk));
+        const size_t smem = sizeof(Real) * kGwChunk * 2 * (m.F + m.Q);
+        if (smem > 200 * 1024) throw Error(3, "gate weight gradient: radial functions + gate scalars exceed the shared-memory staging");
+        if (smem > 48 * 1024)
+          SUS2G_CUDA(cudaFuncSetAttribute(k_gate_weight_grad<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(smem)));
+        k_gate_weight_grad<Real><<<blocks, kGwThreads, smem, s>>>(ncentres_, m.F, m.Q, m.M, dm.gate_nodes,
+                                                                  lh_atom_.as<double>(), gmom_.as<Real>(),
+                                                                  gmomd_.as<Real>(), slots_.as<double>(), P, gw_off);
+        ++launches_;
+      }
     }
-  } else {
-    launches_ += launch_grad_pass<Real>(m.L, kGradOuter, a, co, s);
-    if (split) launches_ += launch_grad_pass<Real>(m.L, kGradOuter, a, co2, s);
   }
   slot_part_.ensure(sizeof(double) * kSlotGroups * static_cast<size_t>(P));
   k_slot_partial<<<dim3((P + 31) / 32, kSlotGroups), dim3(32, 8), 0, s>>>(slots_.as<double>(), nslots, P,
@@ -2344,7 +2462,7 @@ void Engine::efs(double* d_energy, double* d_forces, double* d_virial, double* d
 // tile shape.
 template <typename Real>
 bool Engine::use_static_split() const {
-  return sizeof(Real) == 4 && model_.B == 8 && (static_split_ < 0 ? auto_split() : static_split_ > 0) && split_fits(false);
+  return sizeof(Real) == 4 && model_.B == 8 && wants_split(static_split_) && split_fits(false);
 }
 bool Engine::split_fits(bool gate) const {
   if (precision_ != kFP32) return false;
@@ -2355,10 +2473,9 @@ template <typename Real>
 int Engine::launch_static_split(PassArgs<Real> a, bool pdl) {
   if constexpr (sizeof(Real) == 4) {
     const size_t n = static_cast<size_t>(std::max(1, ncentres_)) * model_.K * model_.H;
+    // a block of the graph kernel reads its centres' moments before it writes their adjoints
     mom_.ensure(sizeof(Real) * n);
-    amom_.ensure(sizeof(Real) * n);
-    a.mom = mom_.as<Real>();
-    a.amom = amom_.as<Real>();
+    a.mom = a.amom = mom_.as<Real>();
     const int mode = model_.gated ? kModeOuter : kModeStatic;
     a.grid_mode = pass_grid_[mode];
     a.atom_order = pass_order_[mode];
@@ -2379,8 +2496,7 @@ int Engine::launch_static_split(PassArgs<Real> a, bool pdl) {
 // fused pass's grid and centre order and their own register budget.
 template <typename Real>
 bool Engine::use_gate_split() const {
-  return sizeof(Real) == 4 && model_.B == 8 && model_.gated && (gate_split_ < 0 ? auto_split() : gate_split_ > 0) &&
-         split_fits(true);
+  return sizeof(Real) == 4 && model_.B == 8 && model_.gated && wants_split(gate_split_) && split_fits(true);
 }
 // Without a choice by the caller or the autotuner the passes run split from this many centres on.  A
 // fused pass whose centres all have a resident warp (12 to 16 per SM) hides the per-atom work
@@ -2401,22 +2517,19 @@ int Engine::launch_gate_split(int which, PassArgs<Real> a, bool pdl) {
     a.atom_order = pass_order_[mode];
     a.block_warps = pass_wpb_[mode];
     int k = 0;
-    gkeep_.ensure(sizeof(Real) * static_cast<size_t>((std::max(1, ncentres_) + kGraphAtoms - 1) / kGraphAtoms) * kGraphAtoms *
-                  std::max(1, a.dm.gate.block.nkeep));
+    // moments or their adjoints; the gate values kept for the reverse, then the adjoints of h
+    mom_.ensure(sizeof(Real) * n);
+    a.mom = a.amom = mom_.as<Real>();
+    const size_t nkeep = static_cast<size_t>((std::max(1, ncentres_) + kGraphAtoms - 1) / kGraphAtoms) * kGraphAtoms *
+                         std::max(1, a.dm.gate.block.nkeep);
+    gkeep_.ensure(sizeof(Real) * (nkeep + static_cast<size_t>(std::max(1, ncentres_)) * model_.F));
     a.gkeep = gkeep_.as<Real>();
+    a.hbar = gkeep_.as<Real>() + nkeep;
     if (which == 0) {
-      mom_.ensure(sizeof(Real) * n);
-      a.mom = mom_.as<Real>();
       k += launch_shape<Real>(kModeGateFwdEdges, a, gate_split_blocks_[0], pdl);
       k += launch_atom_graph(a, sm_count_, stream_, 1);
     } else {
-      amom_.ensure(sizeof(Real) * n);
-      a.amom = amom_.as<Real>();
-      if (!a.hbar_atom) {
-        hbar_.ensure(sizeof(Real) * static_cast<size_t>(std::max(1, ncentres_)) * model_.F);
-        a.hbar = hbar_.as<Real>();
-        k += launch_hbar_sum(a, stream_);
-      }
+      if (!a.hbar_atom) k += launch_hbar_sum(a, stream_);
       k += launch_atom_graph(a, sm_count_, stream_, 2);
       k += launch_shape<Real>(kModeGateRevEdges, a, gate_split_blocks_[1], false);
     }
@@ -2465,8 +2578,13 @@ void Engine::autotune_passes(int reps, int* blocks_out, double* ms_out) {
   const int N = natoms_;
   double* scratch = static_cast<double*>(io(7, sizeof(double) * (7 * static_cast<size_t>(std::max(1, nframes_)) +
                                                                   4 * static_cast<size_t>(std::max(1, N)))));
+  if (sizeof(Real) == 4 && m.B == 8 && !block_prog_[0]) upload_block_programs(false);
   run_efs<Real>(scratch, scratch + 7 * std::max(1, nframes_), scratch + std::max(1, nframes_), nullptr, kStageAll);
   PassArgs<Real> a = pass_args<Real>();
+  if (m.gated) {  // the fused gate passes are timed too
+    gmom_.ensure(sizeof(Real) * static_cast<size_t>(std::max(1, N)) * m.M);
+    a.gmom = gmom_.as<Real>();
+  }
   const int modes_static[] = {kModeStatic};
   const int modes_gated[] = {kModeGateForward, kModeOuter, kModeGateReverse};
   const int* modes = m.gated ? modes_gated : modes_static;

@@ -219,6 +219,7 @@ class Engine {
 
  private:
   template <typename Real> void upload_tables();
+  void upload_block_programs(bool dual);
   template <typename Real> PassArgs<Real> pass_args();
   template <typename Real> void autotune_passes(int reps, int* blocks_out, double* ms_out);
   enum : int { kStageGate = 1, kStageOuter = 2, kStageFinish = 4, kStageAll = 7 };
@@ -240,6 +241,7 @@ class Engine {
   void run_grad(const double* ew, const double* fw, const double* sw, double* grad, const double* extra_h);
   DevBuf slots_, slot_part_, hsigd_, gmomd_, lhm_, lh_atom_;
   DevBuf gabar_;                // moment adjoints between the parts of a split gradient pass
+  DevBuf gdmom_, gdkeep_, gdscal_;  // its moments, kept gate values and gate scalars (values, tangents)
   bool grad_split_ = true;      // gradient passes split at the per-atom boundary (basis size 8)
   void finalize_edges();
 
@@ -253,8 +255,8 @@ class Engine {
   // model tables (both precisions are packed into one buffer each)
   DevBuf tab_int_, tab_real_, tab_dbl_, tab_prog_;
   std::unique_ptr<HostProg> prog_[2];  // outer and gate graph programs (structure built once)
-  std::unique_ptr<HostBlockProg> block_prog_[2];
-  DevBuf tab_block_;
+  std::unique_ptr<HostBlockProg> block_prog_[2], dual_prog_[2];
+  DevBuf tab_block_, tab_dual_;
   void* dev_model_ = nullptr;  // host copy of DevModel<Real>
 
   // geometry
@@ -310,6 +312,7 @@ class Engine {
   bool split_fits(bool gate) const;  // the pass's nodes fit the block graph kernel
   template <typename Real> bool use_gate_split() const;
   bool auto_split() const;
+  bool wants_split(int choice) const { return choice < 0 ? auto_split() : choice > 0; }
   template <typename Real> int launch_gate_split(int which, PassArgs<Real> a, bool pdl);
   template <typename Real> int launch_static_split(PassArgs<Real> a, bool pdl);
   int static_split_ = -1;       // energy pass as forward / per-atom graph / adjoint kernels (-1: auto_split)
@@ -317,8 +320,8 @@ class Engine {
   int gate_split_ = -1;         // Effect gate forward and reverse passes split (together: gkeep_)
   bool gate_ran_split_ = false; // the form of the last gate forward pass, which its reverse takes too
   int gate_split_blocks_[2] = {0, 0};    // their per-edge kernels' register budgets
-  DevBuf mom_, amom_;           // the split pass's moments and adjoint moments [N][K H]
-  DevBuf hbar_, gkeep_;         // split gate passes: adjoints of h per centre [N][F], gate values kept for the reverse
+  DevBuf mom_;                  // the split pass's moments, then their adjoints [N][K H]
+  DevBuf gkeep_;                // split gate passes: gate values kept for the reverse, adjoints of h per centre [N][F]
   // second stream for independent work inside a step (reverse edges beside the first pass, the
   // frame reduction beside the force gather)
   cudaStream_t aux_stream_ = nullptr;

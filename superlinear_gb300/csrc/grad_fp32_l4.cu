@@ -2,4 +2,5 @@
 #include "grad_inst.cuh"
 namespace sus2g {
 SUS2G_INSTANTIATE_GRAD(float, 4)
+SUS2G_INSTANTIATE_GRAD_MOMENT(4)
 }  // namespace sus2g

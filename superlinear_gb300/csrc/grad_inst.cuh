@@ -5,6 +5,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "grad_edge.cuh"
 #include "pass_launch.h"
 
 namespace sus2g {
@@ -109,6 +110,86 @@ int launch_grad_pass_l(int mode, const GradArgs<Real>& a, const GradLaunch& cfg,
   return 1;
 }
 
+namespace grad_detail {
+// Blocks of up to max_warps warps of a kernel that needs `bytes(warps)` of shared memory: the most resident
+// warps per SM, four warps a block on ties (wider blocks level the warps' loads less, narrower ones
+// make more slices); grid 0 when it does not fit.
+template <typename Kern, typename Bytes>
+GradLaunch warp_launch(Kern kern, int max_warps, int natoms, int sm_count, Bytes&& bytes) {
+  int device = 0, optin = 0;
+  cudaGetDevice(&device);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  GradLaunch cfg;
+  int best = 0;
+  if (bytes(1) > static_cast<size_t>(optin)) return cfg;
+  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+  if (err != cudaSuccess) throw std::runtime_error(std::string("gradient shared memory: ") + cudaGetErrorString(err));
+  for (int q = 0; q < max_warps; ++q) {
+    const int w = q < kGradMaxWarps ? kGradMaxWarps - q : q + 1;  // 4 .. 1, then 5 up
+    if (bytes(w) > static_cast<size_t>(optin)) continue;
+    int blocks = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, w * kWarp, bytes(w));
+    if (blocks * w > best) {
+      best = blocks * w;
+      cfg.warps = w;
+      cfg.grid = blocks * sm_count;
+    }
+  }
+  if (best == 0) return GradLaunch{};
+  cfg.block = cfg.warps * kWarp;
+  cfg.smem = bytes(cfg.warps);
+  cfg.grid = std::max(1, std::min((natoms + cfg.warps - 1) / cfg.warps, cfg.grid));
+  return cfg;
+}
+template <typename Real, int L>
+GradKernel<Real> edge_kernel(int mode, bool gated) {
+  if (mode != kGradOuter) return grad_edge_kernel<L, Real, kGradGateReverse, 8, false>;
+  return gated ? grad_edge_kernel<L, Real, kGradOuter, 8, true> : grad_edge_kernel<L, Real, kGradOuter, 8, false>;
+}
+template <int L>
+GradKernel<float> moment_kernel(int mode) {
+  return mode == kGradOuter ? grad_moment_kernel<L, float, kGradOuter, 8> : grad_moment_kernel<L, float, kGradGateForward, 8>;
+}
+inline void check_launch(const char* what) {
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(err));
+}
+}  // namespace grad_detail
+
+template <typename Real, int L>
+GradLaunch grad_edge_config_l(int mode, const DevModel<Real>& dm, int natoms, int sm_count) {
+  // compiled for basis size 8 and one warp per radial channel (scaling maps "K" and "pair")
+  if (dm.B != 8 || (dm.scaling_mode != 2 && dm.scaling_mode != 0) || dm.K > kMaxK) return GradLaunch{};
+  const bool outer = mode == kGradOuter && dm.gated;
+  const size_t shared = sizeof(Real) * round4(pass_table_size<Real>(dm.C, dm.F, dm.B, dm.nblk)) + sizeof(int) * grad_edge_items(grad_items(L + 1, dm.B, dm.C, outer));
+  const size_t per_warp = sizeof(Real) * grad_edge_warp_floats<Real>(L, dm.K, dm.B, dm.C, outer);
+  return grad_detail::warp_launch(grad_detail::edge_kernel<Real, L>(mode, dm.gated), grad_max_warps(L, sizeof(Real) == 4), natoms, sm_count,
+                                  [&](int w) { return shared + w * per_warp; });
+}
+template <typename Real, int L>
+int launch_grad_edge_l(int mode, const GradArgs<Real>& a, const GradLaunch& cfg, cudaStream_t s) {
+  if (a.natoms == 0) return 0;
+  grad_detail::edge_kernel<Real, L>(mode, a.dm.gated)<<<cfg.grid, cfg.block, cfg.smem, s>>>(a);
+  grad_detail::check_launch("gradient edge launch");
+  return 1;
+}
+template <int L>
+GradLaunch grad_moment_config_l(int mode, const DevModel<float>& dm, int natoms, int sm_count) {
+  const size_t shared = sizeof(float) * round4(pass_table_size<float>(dm.C, dm.F, dm.B, dm.nblk));
+  const size_t per_warp = sizeof(float) * grad_moment_warp_size<float>(L, dm.K);
+  const GradLaunch cfg = grad_detail::warp_launch(grad_detail::moment_kernel<L>(mode), grad_max_warps(L, true), natoms, sm_count,
+                                                  [&](int w) { return shared + w * per_warp; });
+  if (!cfg.grid) throw std::runtime_error("gradient moment kernel does not fit on an SM");
+  return cfg;
+}
+template <int L>
+int launch_grad_moment_l(int mode, const GradArgs<float>& a, const GradLaunch& cfg, cudaStream_t s) {
+  if (a.natoms == 0) return 0;
+  grad_detail::moment_kernel<L>(mode)<<<cfg.grid, cfg.block, cfg.smem, s>>>(a);
+  grad_detail::check_launch("gradient moment launch");
+  return 1;
+}
+
 template <typename Real, int L>
 cudaError_t upload_grad_constants_l() { return sph_norm_upload(); }
 
@@ -117,4 +198,9 @@ cudaError_t upload_grad_constants_l() { return sph_norm_upload(); }
 #define SUS2G_INSTANTIATE_GRAD(REAL, L)                                                                  \
   template GradLaunch grad_pass_config_l<REAL, L>(int, const DevModel<REAL>&, int, int, int);            \
   template int launch_grad_pass_l<REAL, L>(int, const GradArgs<REAL>&, const GradLaunch&, cudaStream_t); \
+  template GradLaunch grad_edge_config_l<REAL, L>(int, const DevModel<REAL>&, int, int);                 \
+  template int launch_grad_edge_l<REAL, L>(int, const GradArgs<REAL>&, const GradLaunch&, cudaStream_t); \
   template cudaError_t upload_grad_constants_l<REAL, L>();
+#define SUS2G_INSTANTIATE_GRAD_MOMENT(L)                                                                 \
+  template GradLaunch grad_moment_config_l<L>(int, const DevModel<float>&, int, int);                    \
+  template int launch_grad_moment_l<L>(int, const GradArgs<float>&, const GradLaunch&, cudaStream_t);

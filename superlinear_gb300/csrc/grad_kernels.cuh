@@ -52,12 +52,15 @@ struct GradArgs {
   Real* hsigd;             // [N][F] tangent of h
   Real* gmom;              // [N][M] gate values
   Real* gmomd;             // [N][M] gate tangents
-  Real* lhm;               // [E][2F] dJ/dh, dJ/dhdot contributions stored at the reverse edge
+  Real* lhm;               // [E][2F] dJ/dh, dJ/dhdot contributions stored at the reverse edge: [k][lambda_l, mu_l]
   double* lh_atom;         // [N][2F] gathered per atom (gate reverse)
   const double* extra_h;   // [N][F] additional dJ/dh per atom (objective terms of h), or null
   double* slots;           // [warps in grid][nparams]
   Real* abar;              // [N][2][K][H] adjoints of the moments (values, tangents): the per-atom part
                            // of a split pass writes them, its per-edge part reads them
+  Real* mom;               // [N][2][K][H] moments (values, tangents) of the split per-atom part
+  Real* gkeep;             // [N / 16][nkeep][32] gate values its reverse reads (values, tangents)
+  Real* gscal;             // [N / 16][Q][32] gate scalars (values, tangents)
   int* error;
   int acc_cols;            // lane-private accumulator columns per k (0: shuffle-tree reductions)
 };
@@ -391,7 +394,8 @@ __global__ void __launch_bounds__(128, PART == kGradWhole ? 3 : 4) grad_pass_ker
     } else {
       // ---------------- gate reverse seeds from dJ/dh, dJ/dhdot ----------------
       for (int m_ = lane; m_ < 2 * F; m_ += kWarp) {
-        const Real s = column_sum<Real>(a.lhm + static_cast<size_t>(e0) * 2 * F + m_, 2 * F, e1 - e0);
+        const int k = (m_ % F) / Lp, col = k * 2 * Lp + (m_ % F) % Lp + (m_ < F ? 0 : Lp);
+        const Real s = column_sum<Real>(a.lhm + static_cast<size_t>(e0) * 2 * F + col, 2 * F, e1 - e0);
         double sd = double(s);
         if (a.extra_h && m_ < F) sd += a.extra_h[static_cast<size_t>(atom) * F + m_];
         hb[m_] = Real(sd);
@@ -538,9 +542,9 @@ __global__ void __launch_bounds__(128, PART == kGradWhole ? 3 : 4) grad_pass_ker
               for (int t = 0; t < C; ++t) slot_add<Real>(slot, gl.add_off + t * F + m_, tj == t ? dal : Real(0), lane);
           }
           if (effect_outer && valid) {
-            Real* dst = a.lhm + static_cast<size_t>(a.rev[e]) * 2 * F;
-            dst[m_] = on ? x0 * al * Qv : Real(0);
-            dst[F + m_] = on ? x0 * al * R * Tt : Real(0);
+            Real* dst = a.lhm + static_cast<size_t>(a.rev[e]) * 2 * F + k * 2 * Lp;
+            dst[l] = on ? x0 * al * Qv : Real(0);
+            dst[Lp + l] = on ? x0 * al * R * Tt : Real(0);
           }
         }
         if (COLS) {

@@ -9,7 +9,7 @@
 // 16-byte record serves one term of one centre, and its two node reads hit scattered banks.  Here
 // lanes are centres: node values lie [slot][32 centres] in shared memory, every node read is one
 // conflict-free row, a 16-byte unit serves two terms of 32 centres (about 9 instructions a term),
-// and a block's 16 warps share the target lists of a step, longest first, with a barrier per step.
+// and a block's 16 (or 32) warps share the target lists of a step, longest first, with a barrier per step.
 // Only the nodes of this pass take slots, and an adjoint takes its node's slot when the reverse
 // never reads the value, which keeps two blocks per SM at L4/K8.  Every list is summed chunk by
 // chunk in run_prog's order, so that split and fused passes give the same bits.
@@ -19,6 +19,9 @@
 #include "efs_kernels.cuh"
 
 namespace sus2g {
+
+// Warps of a block: 16, or 32 where shared memory admits one block per SM.
+__host__ __device__ inline int graph_block_warps(size_t bytes) { return bytes > 113 * 1024 ? 2 * kGraphWarps : kGraphWarps; }
 
 // Shared memory of a block: the slots, then hbar [F][32] (gate reverse) or the readout's scalars
 // [S][33] (energy pass).
@@ -71,15 +74,15 @@ __device__ __forceinline__ void run_block_steps(const int4* units, int p0, int p
 // Rows [32][n] of a per-centre array (row stride ld) into or out of slots: a lane moves its centre's
 // row in 16-byte units (the rows' lines stay in L1 between a warp's accesses).
 template <typename Put>
-__device__ __forceinline__ void centre_rows(const float* rows, int ld, int n, int na, int warp, int lane, Put&& put) {
+__device__ __forceinline__ void centre_rows(const float* rows, int ld, int n, int na, int warp, int warps, int lane, Put&& put) {
   const float* row = rows + static_cast<size_t>(min(lane, na - 1)) * ld;
   if (n % 4 == 0 && ld % 4 == 0) {
-    for (int t = 4 * warp; t < n; t += 4 * kGraphWarps) {
+    for (int t = 4 * warp; t < n; t += 4 * warps) {
       const float4 w = *reinterpret_cast<const float4*>(row + t);
       put(t, w.x); put(t + 1, w.y); put(t + 2, w.z); put(t + 3, w.w);
     }
   } else {
-    for (int t = warp; t < n; t += kGraphWarps) put(t, row[t]);
+    for (int t = warp; t < n; t += warps) put(t, row[t]);
   }
 }
 
@@ -87,17 +90,17 @@ __device__ __forceinline__ void centre_rows(const float* rows, int ld, int n, in
 // the gate reverse reads to a.gkeep, gate signals to a.hsig), 2 the gate reverse pass (per-atom
 // gate-signal adjoints in a.hbar, or a.hbar_atom for caller edges).
 template <int GM>
-__global__ void __launch_bounds__(kGraphWarps * kWarp, 2) graph_block_kernel(PassArgs<float> a) {
+__global__ void __launch_bounds__(2 * kGraphWarps * kWarp, 1) graph_block_kernel(PassArgs<float> a) {
   constexpr int A = kGraphAtoms;
   const DevModel<float>& dm = a.dm;
   const BlockProg& g = GM == 0 ? dm.outer.block : dm.gate.block;
   const int KH = dm.K * dm.H, C = dm.C, F = dm.F, Q = dm.Q;
-  const int warp = threadIdx.x / kWarp, lane = warp_lane();
+  const int warps = blockDim.x / kWarp, warp = threadIdx.x / kWarp, lane = warp_lane();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* s = reinterpret_cast<float*>(smem_raw);  // [nslots][32]
   float* more = s + g.nslots * A;                 // hbar [F][32], or the scalars [S][33]
   pdl_launch_dependents();
-  const int p0 = g.begin[3 * warp], p1 = g.begin[3 * warp + 1], p2 = g.begin[3 * warp + 2];
+  const int p0 = g.begin[4 * warp], p1 = g.begin[4 * warp + 1], p2 = g.begin[4 * warp + 3];
   pdl_wait();
   for (int blk = blockIdx.x; blk * A < a.natoms; blk += gridDim.x) {
     const int n0 = blk * A, na = min(A, a.natoms - n0);
@@ -106,16 +109,16 @@ __global__ void __launch_bounds__(kGraphWarps * kWarp, 2) graph_block_kernel(Pas
     if (warp == 0) s[g.one * A + lane] = 1.f;
     if constexpr (GM == 2) {
       if (a.hbar_atom) {
-        for (int mu = warp; mu < F; mu += kGraphWarps) more[mu * A + lane] = static_cast<float>(a.hbar_atom[n * F + mu]);
+        for (int mu = warp; mu < F; mu += warps) more[mu * A + lane] = static_cast<float>(a.hbar_atom[n * F + mu]);
       } else {
-        centre_rows(a.hbar + static_cast<size_t>(n0) * F, F, F, na, warp, lane,
+        centre_rows(a.hbar + static_cast<size_t>(n0) * F, F, F, na, warp, warps, lane,
                     [&](int mu, float x) { more[mu * A + lane] = x; });
       }
-      for (int q = warp; q < g.nkeep; q += kGraphWarps)
+      for (int q = warp; q < g.nkeep; q += warps)
         s[g.keep[q] * A + lane] = a.gkeep[(static_cast<size_t>(blk) * g.nkeep + q) * A + lane];
-      for (int q = warp; q < g.nzero_adj; q += kGraphWarps) s[g.zero_adj[q] * A + lane] = 0.f;
+      for (int q = warp; q < g.nzero_adj; q += warps) s[g.zero_adj[q] * A + lane] = 0.f;
       __syncthreads();
-      for (int q = warp; q < Q; q += kGraphWarps) {
+      for (int q = warp; q < Q; q += warps) {
         const float* w = dm.gate_wmat_t + static_cast<size_t>(q) * F;
         float sum = 0.f;
 #pragma unroll 8
@@ -124,19 +127,19 @@ __global__ void __launch_bounds__(kGraphWarps * kWarp, 2) graph_block_kernel(Pas
       }
       __syncthreads();
     } else {
-      centre_rows(a.mom + static_cast<size_t>(n0) * KH, KH, KH, na, warp, lane, [&](int t, float x) {
+      centre_rows(a.mom + static_cast<size_t>(n0) * KH, KH, KH, na, warp, warps, lane, [&](int t, float x) {
         const int slot = g.basic_slot[t];
         if (slot >= 0) s[slot * A + lane] = x;
       });
-      for (int q = warp; q < g.nzero_v; q += kGraphWarps) s[g.zero_v[q] * A + lane] = 0.f;
+      for (int q = warp; q < g.nzero_v; q += warps) s[g.zero_v[q] * A + lane] = 0.f;
       __syncthreads();
       run_block_steps(g.units, p0, p1, s, lane);
     }
     if constexpr (GM == 1) {
-      for (int q = warp; q < g.nkeep; q += kGraphWarps)
+      for (int q = warp; q < g.nkeep; q += warps)
         a.gkeep[(static_cast<size_t>(blk) * g.nkeep + q) * A + lane] = s[g.keep[q] * A + lane];
       // four signals at a time: each gate scalar is read once for them
-      for (int mu = 4 * warp; mu < F; mu += 4 * kGraphWarps) {
+      for (int mu = 4 * warp; mu < F; mu += 4 * warps) {
         float h[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
         for (int q = 0; q < Q; ++q) {
@@ -159,13 +162,13 @@ __global__ void __launch_bounds__(kGraphWarps * kWarp, 2) graph_block_kernel(Pas
       const int ti = C == 1 ? 0 : species_of(a.types, static_cast<int>(n), C);
       const float coef_r = static_cast<float>(dm.species_readout ? 1.0 : dm.species[ti]);
       const float* lin = dm.linear + (dm.species_readout ? ti * dm.S : 0);
-      for (int q = warp; q < dm.S; q += kGraphWarps) {
+      for (int q = warp; q < dm.S; q += warps) {
         more[q * (A + 1) + lane] = s[g.seed_v[q] * A + lane];
         s[g.seed_adj[q] * A + lane] = coef_r * lin[q];
       }
-      for (int q = warp; q < g.nzero_adj; q += kGraphWarps) s[g.zero_adj[q] * A + lane] = 0.f;
+      for (int q = warp; q < g.nzero_adj; q += warps) s[g.zero_adj[q] * A + lane] = 0.f;
       __syncthreads();
-      for (int c = warp; c < na; c += kGraphWarps) {
+      for (int c = warp; c < na; c += warps) {
         const int tc = __shfl_sync(0xffffffffu, ti, c);
         const int off = dm.species_readout ? tc * dm.S : 0;
         float ehi = 0.f, elo = 0.f;
@@ -187,10 +190,10 @@ __global__ void __launch_bounds__(kGraphWarps * kWarp, 2) graph_block_kernel(Pas
         return slot >= 0 ? s[slot * A + lane] : 0.f;
       };
       if (KH % 4 == 0) {
-        for (int t = 4 * warp; t < KH; t += 4 * kGraphWarps)
+        for (int t = 4 * warp; t < KH; t += 4 * warps)
           *reinterpret_cast<float4*>(row + t) = make_float4(get(t), get(t + 1), get(t + 2), get(t + 3));
       } else {
-        for (int t = warp; t < KH; t += kGraphWarps) row[t] = get(t);
+        for (int t = warp; t < KH; t += warps) row[t] = get(t);
       }
     }
   }
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(kGraphWarps * kWarp, 2) graph_block_kernel(Pas
 // edges by the outer pass) summed per column, warp per centre.  32 / W groups of W lanes take the
 // edges in turn, a lane reading one 16-byte unit of its row, four rows in flight; the groups'
 // sums are added in group order.  Bound by the read of the [E][F] contributions.
-__global__ void __launch_bounds__(256) hbar_sum_kernel(PassArgs<float> a) {
+static __global__ void __launch_bounds__(256) hbar_sum_kernel(PassArgs<float> a) {
   const int F = a.dm.F, lane = warp_lane();
   const int atom = static_cast<int>((static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kWarp);
   pdl_launch_dependents();

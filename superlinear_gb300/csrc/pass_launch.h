@@ -22,6 +22,31 @@ GradLaunch grad_pass_config(int L, int mode, const DevModel<Real>& dm, int natom
 template <typename Real>
 int launch_grad_pass(int L, int mode, const GradArgs<Real>& a, const GradLaunch& cfg, cudaStream_t stream);
 
+// The kernels of the split gradient (grad_edge.cuh, grad_graph.cuh).  Launch shapes: GradLaunch with
+// grid 0 where the kernel does not take the model; the edge, graph and gate-weight kernels write
+// one slice per block.
+constexpr int kDualAtoms = 16;  // centres per block of the graph kernel: half a row of 32
+template <typename Real>
+GradLaunch grad_edge_config(int L, int mode, const DevModel<Real>& dm, int natoms, int sm_count);
+template <typename Real>
+int launch_grad_edge(int L, int mode, const GradArgs<Real>& a, const GradLaunch& cfg, cudaStream_t stream);
+GradLaunch grad_moment_config(int L, int mode, const DevModel<float>& dm, int natoms, int sm_count);
+int launch_grad_moment(int L, int mode, const GradArgs<float>& a, const GradLaunch& cfg, cudaStream_t stream);
+bool grad_graph_fits(const DevModel<float>& dm, bool gated);
+GradLaunch grad_graph_config(int mode, const DevModel<float>& dm, int natoms, int sm_count);
+int launch_grad_graph(int mode, const GradArgs<float>& a, const GradLaunch& cfg, cudaStream_t stream);
+int launch_lhm_sum(const GradArgs<float>& a, int Lp, cudaStream_t stream);
+GradLaunch grad_gate_weight_config(const DevModel<float>& dm, int natoms, int sm_count);
+int launch_grad_gate_weight(const GradArgs<float>& a, const GradLaunch& cfg, cudaStream_t stream);
+template <typename Real, int L>
+GradLaunch grad_edge_config_l(int mode, const DevModel<Real>& dm, int natoms, int sm_count);
+template <typename Real, int L>
+int launch_grad_edge_l(int mode, const GradArgs<Real>& a, const GradLaunch& cfg, cudaStream_t stream);
+template <int L>
+GradLaunch grad_moment_config_l(int mode, const DevModel<float>& dm, int natoms, int sm_count);
+template <int L>
+int launch_grad_moment_l(int mode, const GradArgs<float>& a, const GradLaunch& cfg, cudaStream_t stream);
+
 // Launches atom_pass_kernel<L, Real, mode, Kahan = (Real is float)> sized as a multiple of the SM
 // count, with the register budget of `blocks` resident blocks per SM (3 or 4; 0 = the default),
 // as a programmatic dependent launch when pdl is set (the kernel stages its model tables while
@@ -34,6 +59,8 @@ int launch_atom_pass(int L, int mode, const PassArgs<Real>& args, int sm_count, 
 // The per-atom graph kernel of a split pass (graph_block_kernel<gm>: 0 energy pass, 1 gate forward,
 // 2 gate reverse): returns 1 or throws.
 int launch_atom_graph(const PassArgs<float>& args, int sm_count, cudaStream_t stream, int gm);
+// Warps per block of that kernel (and of the gradient's) for a program of so many slots.
+int graph_program_warps(int nslots, int F, int S);
 // Whether a pass's nodes fit that kernel's shared memory (the pass runs fused otherwise).
 bool graph_block_fits(const BlockProg& g, int F, int S);
 // The per-atom gate-signal adjoints a.hbar from the per-edge contributions (hbar_sum_kernel).
