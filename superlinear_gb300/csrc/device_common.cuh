@@ -117,31 +117,8 @@ struct PassTables {
   const Real* wcenter;    // C x F centre factor  (tau or gate type)
   const Real* wsource;    // C x F source factor  (tau or gate type)
   const Real* wadd;       // C x F Effect additive factor alpha (outer pass of gated models), else null
-  // ranked K contraction, forward grouped by destination node
-  int ndst;
-  const int* dst_node;    // [ndst]
-  const int* dst_begin;   // [ndst + 1]
-  const int* dst_src;     // basic index
-  const Real* dst_w;
-  // reverse grouped by basic index
-  const int* src_begin;   // [NB + 1]
-  const int* src_dst;
-  const Real* src_w;
-  // per-atom product graph schedule (see model.cpp build_schedule)
-  int levels;
-  const int* level_begin;   // [levels + 1]
-  const int* out_nodes;
-  const int* out_begin;
-  const int* fprod_a;
-  const int* fprod_b;
-  const Real* fprod_c;
-  const int* rlevel_begin;  // [levels + 1] (levels >= 1; level 0 holds sources)
-  const int* in_nodes;
-  const int* in_begin;
-  const int* rprod_out;
-  const int* rprod_other;
-  const Real* rprod_c;
-  GraphProg<Real> prog;   // the same contraction and graph as a lane-balanced program (E/F/virial passes)
+  int ndst;               // destination nodes of the ranked K contraction (0: none)
+  GraphProg<Real> prog;   // the rank contraction and product graph as a lane-balanced program
   BlockProg block;        // and as a block program (FP32 split passes)
   BlockProg dual;         // and as one for values and tangents (FP32 split gradient)
 };

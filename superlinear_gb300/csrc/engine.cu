@@ -557,15 +557,11 @@ __global__ void k_force_gather(const int* row, const int* row_end, const int* re
 
 // Caller edges: incoming lists.  in(j) = the edges whose neighbour is j, sorted by edge index, so
 // that per-atom sums over them run in a fixed order (no floating-point atomics).
-__global__ void k_count_in(const int* nbr, long long n, int* counts) {
-  const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e < n) atomicAdd(counts + nbr[e], 1);
-}
-__global__ void k_fill_in(const int* nbr, long long n, const int* in_row, int* cursor, int* in_tmp) {
-  const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= n) return;
+__global__ void k_fill_in(const int* nbr, const int* edges, const int* in_row, int* cursor, int* in_tmp) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= *edges) return;
   const int j = nbr[e];
-  in_tmp[in_row[j] + atomicAdd(cursor + j, 1)] = static_cast<int>(e);
+  in_tmp[in_row[j] + atomicSub(cursor + j, 1) - 1] = e;
 }
 // warp per atom: rank sort of the (unique) edge indices of in(j)
 __global__ void k_sort_in(const int* in_row, int nall, const int* in_tmp, int* in_edge) {
@@ -705,16 +701,26 @@ k_frame_reduce(const FramePlan* plans, int nframes, int S, const double* site, c
   if (threadIdx.x == 0) arrivals[f] = 0u;
 }
 
-// Caller-provided edges (owned centres, LAMMPS layout): count per centre.  An edge with a centre
-// or neighbour index out of range is flagged and left out here and by the scatter below alike,
-// so that no row keeps an unfilled slot.
-__global__ void k_count_centres(const int* ei, const int* ej, long long n, int* counts, int nowned, int nall,
-                                int* error) {
+// Caller-provided edges (owned centres, LAMMPS layout): *flag = 1 when an index is out of range or a
+// length is not well inside (0, 1e150).
+__global__ void k_check_user_edges(const int* ei, const int* ej, const double* d, long long n, int nowned, int nall, int* flag) {
+  const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const int i = ei[e], j = ej[e];
+  const double x = d[3 * e], y = d[3 * e + 1], z = d[3 * e + 2], r2 = x * x + y * y + z * z;
+  if (i < 0 || i >= nowned || j < 0 || j >= nall || !(r2 > 1e-290) || !(r2 < 1e299)) *flag = 1;
+}
+// Counts per centre and per neighbour.  An
+// edge with a centre or neighbour index out of range is flagged and left out here and by the
+// scatter below alike, so that no row keeps an unfilled slot.
+__global__ void k_count_user_edges(const int* ei, const int* ej, long long n, int* out_count, int* in_count, int nowned,
+                                   int nall, int* error) {
   const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const int i = ei[e], j = ej[e];
   if (i < 0 || i >= nowned || j < 0 || j >= nall) { record_error(error, kErrEdgeCapacity); return; }
-  atomicAdd(counts + i, 1);
+  atomicAdd(out_count + i, 1);
+  atomicAdd(in_count + j, 1);
 }
 
 template <typename Real>
@@ -727,8 +733,9 @@ __global__ void k_scatter_user_edges(const int* ei, const int* ej, const double*
   if (i < 0 || i >= nowned || j < 0 || j >= nall) { record_error(error, kErrEdgeCapacity); return; }
   const double x = d[3 * e], y = d[3 * e + 1], z = d[3 * e + 2];
   const double r2 = x * x + y * y + z * z;
-  if (!(r2 > 0) || !isfinite(r2)) record_error(error, kErrBadDistance);
-  const int p = row[i] + atomicAdd(cursor + i, 1);
+  if (!(r2 > 0) || !(r2 < 1e300)) record_error(error, kErrBadDistance);
+  // the counts run down to zero as the rows fill (the order within a row is made by the sort)
+  const int p = row[i] + atomicSub(cursor + i, 1) - 1;
   nbr[p] = j;
   typename Vec4<Real>::type v;
   v.x = Real(x); v.y = Real(y); v.z = Real(z);
@@ -741,10 +748,12 @@ __global__ void k_scatter_user_edges(const int* ei, const int* ej, const double*
   key[p] = (static_cast<unsigned long long>(j) << 32) | static_cast<unsigned long long>(e & 0xffffffffLL);
 }
 
-// Exclusive scan of n counts into row[0..n] on the device (one block; each thread scans a
-// contiguous chunk, then the chunk totals are scanned in shared memory).  Totals above 2^31 - 1
-// are flagged.
-__global__ void k_exclusive_scan(const int* counts, int n, int* row, int* error) {
+// Exclusive scans of n counts each into row[0..n] on the device: block 0 the out-edges, block 1 the
+// in-edges (each thread scans a contiguous chunk, then the chunk totals are scanned in shared
+// memory).  Totals above 2^31 - 1 are flagged.
+__global__ void k_exclusive_scans(const int* out_counts, const int* in_counts, int n, int* out_row, int* in_row, int* error) {
+  const int* counts = blockIdx.x ? in_counts : out_counts;
+  int* row = blockIdx.x ? in_row : out_row;
   __shared__ long long part[1024];
   const int t = threadIdx.x, T = blockDim.x;
   const long long chunk = (static_cast<long long>(n) + T - 1) / T;
@@ -768,23 +777,6 @@ __global__ void k_exclusive_scan(const int* counts, int n, int* row, int* error)
     if (part[t] > 2147483647LL) record_error(error, kErrEdgeCapacity);
     row[n] = static_cast<int>(min(part[t], 2147483647LL));
   }
-}
-
-void exclusive_scan_host_sync(const int* d_counts, int n, int* d_row, cudaStream_t s, long long* total) {
-  std::vector<int> h(n);
-  if (n) SUS2G_CUDA(cudaMemcpyAsync(h.data(), d_counts, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
-  SUS2G_CUDA(cudaStreamSynchronize(s));
-  std::vector<int> r(n + 1);
-  long long acc = 0;
-  for (int i = 0; i < n; ++i) {
-    r[i] = static_cast<int>(acc);
-    acc += h[i];
-    if (acc > 2000000000LL) throw Error(5, "edge count exceeds 2^31");
-  }
-  r[n] = static_cast<int>(acc);
-  SUS2G_CUDA(cudaMemcpyAsync(d_row, r.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
-  SUS2G_CUDA(cudaStreamSynchronize(s));
-  *total = acc;
 }
 
 void invert3(const double* c, double* inv) {
@@ -833,84 +825,69 @@ namespace {
 
 struct Packer {
   std::vector<int> ints;
-  std::vector<double> reals;
   int add_int(const std::vector<int>& v) { int o = static_cast<int>(ints.size()); ints.insert(ints.end(), v.begin(), v.end()); return o; }
-  int add_real(const std::vector<double>& v) { int o = static_cast<int>(reals.size()); reals.insert(reals.end(), v.begin(), v.end()); return o; }
 };
 
-struct PassOffsets {
-  int coeff, scal, wc, ws, wa;
-  int ndst, dst_node, dst_begin, dst_src, dst_w, src_begin, src_dst, src_w;
-  int levels, level_begin, out_nodes, out_begin, fa, fb, fc, rlevel_begin, in_nodes, in_begin, rout, rother, rc;
+// Offsets of a pass's parameter-dependent values in the value table.
+struct PassOffsets { int coeff, scal, wc, wa; };
+struct ValueOffsets {
+  PassOffsets outer, gate;
+  int linear, wmat, wmat_t, outer_w, gate_w;
 };
 
-PassOffsets pack_pass(const Model& m, bool gate, Packer& pk) {
-  PassOffsets o{};
+// The parameter-dependent values in the device table's order (offsets are the same at every call).
+template <typename Real>
+ValueOffsets pack_values(const Model& m, std::vector<Real>& out) {
+  out.clear();
   const int C = m.C, F = m.F, B = m.B;
-  std::vector<double> coeff(static_cast<size_t>(F) * B);
-  const bool own_radial = gate && m.gate_shared_radial;
-  for (int mu = 0; mu < F; ++mu)
-    for (int b = 0; b < B; ++b)
-      coeff[static_cast<size_t>(mu) * B + b] = own_radial ? m.gate_radial[static_cast<size_t>(mu) * B + b]
-                                                          : m.radial[static_cast<size_t>(mu) * (B + C) + b];
-  o.coeff = pk.add_real(coeff);
-  o.scal = pk.add_real(gate && m.gate_decoupled ? m.gate_scal : m.scal);
-  std::vector<double> wc(static_cast<size_t>(C) * F), wa(static_cast<size_t>(C) * F, 0.0);
-  for (int t = 0; t < C; ++t)
-    for (int mu = 0; mu < F; ++mu) {
-      const size_t idx = static_cast<size_t>(t) * F + mu;
-      wc[idx] = gate ? m.gate_type[idx] : m.radial[static_cast<size_t>(mu) * (B + C) + B + t];
-      if (!gate && m.gated) wa[idx] = m.gate_add[idx];
-    }
-  o.wc = pk.add_real(wc);
-  o.ws = o.wc;
-  o.wa = pk.add_real(wa);
-  // contraction
-  const auto& rows = gate ? m.gate_rows : m.outer_rows;
-  const auto& w = gate ? m.gate_w : m.outer_w;
-  std::vector<int> dsts;
-  for (const auto& r : rows) dsts.push_back(r.dst);
-  std::sort(dsts.begin(), dsts.end());
-  dsts.erase(std::unique(dsts.begin(), dsts.end()), dsts.end());
-  std::vector<int> dst_begin{0}, dst_src, src_begin{0}, src_dst;
-  std::vector<double> dst_w, src_w;
-  for (int d : dsts) {
-    for (const auto& r : rows)
-      if (r.dst == d) { dst_src.push_back(r.src); dst_w.push_back(r.widx < 0 ? 1.0 : w[r.widx]); }
-    dst_begin.push_back(static_cast<int>(dst_src.size()));
-  }
-  for (int b = 0; b < m.NB; ++b) {
-    for (const auto& r : rows)
-      if (r.src == b) { src_dst.push_back(r.dst); src_w.push_back(r.widx < 0 ? 1.0 : w[r.widx]); }
-    src_begin.push_back(static_cast<int>(src_dst.size()));
-  }
-  o.ndst = static_cast<int>(dsts.size());
-  o.dst_node = pk.add_int(dsts);
-  o.dst_begin = pk.add_int(dst_begin);
-  o.dst_src = pk.add_int(dst_src);
-  o.dst_w = pk.add_real(dst_w);
-  o.src_begin = pk.add_int(src_begin);
-  o.src_dst = pk.add_int(src_dst);
-  o.src_w = pk.add_real(src_w);
-  // graph
-  const GraphSchedule& g = gate ? m.gate_graph : m.outer_graph;
-  o.levels = g.levels;
-  o.level_begin = pk.add_int(g.level_begin);
-  o.out_nodes = pk.add_int(g.out_nodes);
-  o.out_begin = pk.add_int(g.out_begin);
-  std::vector<int> fa, fb;
-  std::vector<double> fc;
-  for (int p : g.fprod) { fa.push_back(m.products[p].a); fb.push_back(m.products[p].b); fc.push_back(m.products[p].c); }
-  o.fa = pk.add_int(fa);
-  o.fb = pk.add_int(fb);
-  o.fc = pk.add_real(fc);
-  o.rlevel_begin = pk.add_int(g.rlevel_begin);
-  o.in_nodes = pk.add_int(g.in_nodes);
-  o.in_begin = pk.add_int(g.in_begin);
-  o.rout = pk.add_int(g.rprod_out);
-  o.rother = pk.add_int(g.rprod_other);
-  o.rc = pk.add_real(g.rprod_c);
+  auto add = [&](const std::vector<double>& v) {
+    const int o = static_cast<int>(out.size());
+    for (double x : v) out.push_back(static_cast<Real>(x));
+    return o;
+  };
+  auto pass = [&](bool gate) {
+    PassOffsets o{};
+    const bool own_radial = gate && m.gate_shared_radial;
+    o.coeff = static_cast<int>(out.size());
+    for (int mu = 0; mu < F; ++mu)
+      for (int b = 0; b < B; ++b)
+        out.push_back(static_cast<Real>(own_radial ? m.gate_radial[static_cast<size_t>(mu) * B + b]
+                                                   : m.radial[static_cast<size_t>(mu) * (B + C) + b]));
+    o.scal = add(gate && m.gate_decoupled ? m.gate_scal : m.scal);
+    o.wc = static_cast<int>(out.size());
+    for (int t = 0; t < C; ++t)
+      for (int mu = 0; mu < F; ++mu)
+        out.push_back(static_cast<Real>(gate ? m.gate_type[static_cast<size_t>(t) * F + mu]
+                                             : m.radial[static_cast<size_t>(mu) * (B + C) + B + t]));
+    o.wa = static_cast<int>(out.size());
+    for (size_t q = 0; q < static_cast<size_t>(C) * F; ++q) out.push_back(static_cast<Real>(!gate && m.gated ? m.gate_add[q] : 0.0));
+    return o;
+  };
+  ValueOffsets o{};
+  o.outer = pass(false);
+  o.gate = m.gated ? pass(true) : o.outer;
+  o.linear = add(m.linear);
+  o.wmat = static_cast<int>(out.size());
+  if (m.gated)
+    for (int mu = 0; mu < F; ++mu)
+      for (int q = 0; q < m.Q; ++q) out.push_back(static_cast<Real>(m.gate_weight(mu, q)));
+  o.wmat_t = static_cast<int>(out.size());
+  if (m.gated)
+    for (int q = 0; q < m.Q; ++q)
+      for (int mu = 0; mu < F; ++mu) out.push_back(out[static_cast<size_t>(o.wmat) + static_cast<size_t>(mu) * m.Q + q]);
+  o.outer_w = add(m.outer_w);
+  o.gate_w = add(m.gate_w);
   return o;
+}
+
+// A program coefficient that is a rank weight: its place in the program image, and the weight.
+struct WeightPatch { size_t at; int widx; bool gate; };
+// One value of the device tables copied to its other places (rank weights into the programs).
+struct ValueCopy { void* to; const void* from; };
+template <typename Real>
+__global__ void k_copy_values(const ValueCopy* list, int n) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < n) *static_cast<Real*>(list[q].to) = *static_cast<const Real*>(list[q].from);
 }
 
 // ---- per-atom graph program (see GraphProg in device_common.cuh) ----
@@ -974,29 +951,42 @@ void add_prog_step(HostProg& hp, const std::vector<ProgGroup>& groups, bool reve
   for (int l = 0; l < kWarp; ++l) refill(l);
   const int first = static_cast<int>(hp.rows.size() / kWarp);
   const HostProg::Rec pad{static_cast<unsigned>(one) | (static_cast<unsigned>(one) << 16), kProgNoFlush, -1, 0.0};
-  auto seen = [](const std::vector<int>& nodes, int n) { return std::find(nodes.begin(), nodes.end(), n) != nodes.end(); };
+  struct Banks {  // distinct nodes read per bank in one row (at most one per lane)
+    int n[kWarp], node[kWarp][kWarp];
+    bool seen(int x) const {
+      const unsigned b = static_cast<unsigned>(x) % kWarp;
+      for (int q = 0; q < n[b]; ++q)
+        if (node[b][q] == x) return true;
+      return false;
+    }
+    int cost(int x) const { return n[static_cast<unsigned>(x) % kWarp] == 0 || seen(x) ? 0 : n[static_cast<unsigned>(x) % kWarp]; }
+    void read(int x) {
+      const unsigned b = static_cast<unsigned>(x) % kWarp;
+      if (!seen(x)) node[b][n[b]++] = x;
+    }
+  };
+  Banks bank_a, bank_b;
   int len = 0;
   for (;;) {
     bool any = false;
     for (int l = 0; l < kWarp; ++l) any = any || !pool[l].empty();
     if (!any) break;
-    std::vector<std::vector<int>> bank_a(kWarp), bank_b(kWarp);  // distinct nodes read per bank
+    std::fill(bank_a.n, bank_a.n + kWarp, 0);
+    std::fill(bank_b.n, bank_b.n + kWarp, 0);
     for (int l = 0; l < kWarp; ++l) {
       if (pool[l].empty()) { hp.rows.push_back(pad); continue; }
       const ProgGroup& g = groups[chs[cur[l]].g];
       size_t best = 0;
       int best_cost = 1 << 30;
-      for (size_t k = 0; k < pool[l].size(); ++k) {
-        const int a = g.ab[pool[l][k]][0], b = g.ab[pool[l][k]][1];
-        const int c = (seen(bank_a[a % kWarp], a) ? 0 : static_cast<int>(bank_a[a % kWarp].size())) +
-                      (seen(bank_b[b % kWarp], b) ? 0 : static_cast<int>(bank_b[b % kWarp].size()));
+      for (size_t k = 0; k < pool[l].size() && best_cost > 0; ++k) {  // (the first free one is best)
+        const int c = bank_a.cost(g.ab[pool[l][k]][0]) + bank_b.cost(g.ab[pool[l][k]][1]);
         if (c < best_cost) { best_cost = c; best = k; }
       }
       const int q = pool[l][best];
       pool[l].erase(pool[l].begin() + static_cast<long>(best));
       const int a = g.ab[q][0], b = g.ab[q][1];
-      if (!seen(bank_a[a % kWarp], a)) bank_a[a % kWarp].push_back(a);
-      if (!seen(bank_b[b % kWarp], b)) bank_b[b % kWarp].push_back(b);
+      bank_a.read(a);
+      bank_b.read(b);
       const bool last = pool[l].empty();
       hp.rows.push_back({static_cast<unsigned>(a) | (static_cast<unsigned>(b) << 16), last ? chs[cur[l]].flush : kProgNoFlush,
                          g.widx[q], g.c[q]});
@@ -1017,16 +1007,19 @@ HostProg build_prog(const Model& m, bool gate) {
   const int one = m.M;
   const auto& rows = gate ? m.gate_rows : m.outer_rows;
   const GraphSchedule& g = gate ? m.gate_graph : m.outer_graph;
+  std::vector<std::vector<int>> by_dst(m.M), by_src(m.M);
+  for (int q = 0; q < static_cast<int>(rows.size()); ++q) {
+    by_dst[rows[q].dst].push_back(q);
+    by_src[rows[q].src].push_back(q);
+  }
   std::vector<int> dsts;
-  for (const auto& r : rows) dsts.push_back(r.dst);
-  std::sort(dsts.begin(), dsts.end());
-  dsts.erase(std::unique(dsts.begin(), dsts.end()), dsts.end());
+  for (int d = 0; d < m.M; ++d)
+    if (!by_dst[d].empty()) dsts.push_back(d);
   {
     std::vector<ProgGroup> gs;
     for (int d : dsts) {
       ProgGroup pg{d, {}, {}, {}};
-      for (const auto& r : rows)
-        if (r.dst == d) { pg.ab.push_back({r.src, one}); pg.c.push_back(1.0); pg.widx.push_back(r.widx); }
+      for (int q : by_dst[d]) { pg.ab.push_back({rows[q].src, one}); pg.c.push_back(1.0); pg.widx.push_back(rows[q].widx); }
       gs.push_back(std::move(pg));
     }
     add_prog_step(hp, gs, false, one);
@@ -1063,8 +1056,7 @@ HostProg build_prog(const Model& m, bool gate) {
     std::vector<ProgGroup> gs;
     for (int b = 0; b < m.NB; ++b) {
       ProgGroup pg{b, {}, {}, {}};
-      for (const auto& r : rows)
-        if (r.src == b) { pg.ab.push_back({r.dst, one}); pg.c.push_back(1.0); pg.widx.push_back(r.widx); }
+      for (int q : by_src[b]) { pg.ab.push_back({rows[q].dst, one}); pg.c.push_back(1.0); pg.widx.push_back(rows[q].widx); }
       gs.push_back(std::move(pg));
     }
     add_prog_step(hp, gs, true, one);
@@ -1079,9 +1071,14 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
   const int nsteps = static_cast<int>(hp.steps.size());
   const std::vector<int>& seeds = hp.gate ? m.gate_nodes : m.scalar_map;
   const int one = m.M;
-  // each step's target lists from the lane streams: chunk = terms up to a flush, list = its chunks
-  struct List { int target; std::vector<std::vector<HostProg::Rec>> chunks; };
+  // each step's target lists from the lane streams: a chunk is a lane's terms up to a flush (rows
+  // first .. first + n - 1 of that lane), a list its chunks begin .. end - 1
+  struct Chunk { int lane, first, n; };
+  struct List { int target, begin, end; };
+  std::vector<Chunk> chunks;
   std::vector<std::vector<List>> steps(nsteps);
+  chunks.reserve(hp.rows.size() / 2);
+  auto rec = [&](const Chunk& c, int i) -> const HostProg::Rec& { return hp.rows[static_cast<size_t>(c.first + i) * kWarp + c.lane]; };
   std::vector<char> in_v(m.M, 0), in_adj(m.M, 0), rev_b(m.M, 0), early(m.M, 0), rank_src(m.M, 0);
   const std::vector<ContractionRow>& rank_rows = hp.gate ? m.gate_rows : m.outer_rows;
   const bool apart = dual && !rank_rows.empty();
@@ -1091,38 +1088,42 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
   for (int st = 0; st < nsteps; ++st) {
     const auto& info = hp.steps[st];
     const bool rev = (info[3] & 1) != 0;
-    std::map<int, std::vector<HostProg::Rec>> parts;
+    std::vector<Chunk> parts;
     const bool last = apart && st + 1 == nsteps;
     auto mark = [&](int target) {
       (rev ? in_adj : in_v)[target] = 1;
       if (rev && !last) early[target] = 1;
     };
     for (int lane = 0; lane < kWarp; ++lane) {
-      std::vector<HostProg::Rec> chunk;
+      Chunk c{lane, info[0], 0};
       for (int i = 0; i < info[1]; ++i) {
-        const HostProg::Rec& r = hp.rows[static_cast<size_t>(info[0] + i) * kWarp + lane];
-        chunk.push_back(r);
-        if (r.flush == kProgNoFlush) continue;
-        for (const auto& t : chunk) {
-          const int x = static_cast<int>(t.ab & 0xffffu), y = static_cast<int>(t.ab >> 16);
+        ++c.n;
+        const int flush = rec(c, c.n - 1).flush;
+        if (flush == kProgNoFlush) continue;
+        for (int k = 0; k < c.n; ++k) {
+          const unsigned ab = rec(c, k).ab;
+          const int x = static_cast<int>(ab & 0xffffu), y = static_cast<int>(ab >> 16);
           if (x != one) mark(x);
           if (y != one) { in_v[y] = 1; if (rev) rev_b[y] = 1; }
         }
-        if (r.flush >= 0) {
-          mark(r.flush);
-          steps[st].push_back({r.flush, {chunk}});
+        if (flush >= 0) {
+          mark(flush);
+          const int b = static_cast<int>(chunks.size());
+          chunks.push_back(c);
+          steps[st].push_back({flush, b, b + 1});
         } else {
-          parts[-r.flush - 2] = chunk;
+          if (static_cast<size_t>(-flush - 2) >= parts.size()) parts.resize(static_cast<size_t>(-flush - 1));
+          parts[-flush - 2] = c;
         }
-        chunk.clear();  // (what follows a lane's last flush is padding)
+        c = Chunk{lane, c.first + c.n, 0};  // (what follows a lane's last flush is padding)
       }
     }
     for (int q = info[2]; q < (info[3] >> 1); ++q) {
       const auto& c = hp.comb[q];
-      List l{c[0], {}};
-      for (int p = c[1]; p < c[2]; ++p) l.chunks.push_back(parts[p]);
+      const int b = static_cast<int>(chunks.size());
+      for (int p = c[1]; p < c[2]; ++p) chunks.push_back(parts[p]);
       mark(c[0]);
-      steps[st].push_back(std::move(l));
+      steps[st].push_back({c[0], b, static_cast<int>(chunks.size())});
     }
   }
   // slots: moments in (k, h) order, the other values, the constant, then adjoints; an adjoint takes
@@ -1156,13 +1157,16 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
   for (int q : seeds) { bp.seed_v.push_back(vslot[q]); bp.seed_adj.push_back(aslot[q]); }
   for (int q = 0; q < m.M; ++q)
     if (rev_b[q] || rank_src[q]) bp.keep.push_back(vslot[q]);
-  if (dual)
-    for (int w = 0; w < static_cast<int>((hp.gate ? m.gate_w : m.outer_w).size()); ++w)
-      for (const auto& r : rank_rows)
-        if (r.widx == w) {
-          bp.rank_v.push_back(vslot[r.src]);
-          bp.rank_adj.push_back(aslot[r.dst]);
-        }
+  if (dual) {
+    std::vector<const ContractionRow*> by_weight;
+    for (const auto& r : rank_rows)
+      if (r.widx >= 0 && r.widx < static_cast<int>((hp.gate ? m.gate_w : m.outer_w).size())) by_weight.push_back(&r);
+    std::stable_sort(by_weight.begin(), by_weight.end(), [](const ContractionRow* x, const ContractionRow* y) { return x->widx < y->widx; });
+    for (const ContractionRow* r : by_weight) {
+      bp.rank_v.push_back(vslot[r->src]);
+      bp.rank_adj.push_back(aslot[r->dst]);
+    }
+  }
   // streams: lists longest first onto the least-loaded warp
   const HostBlockProg::Term pad{bp.one, bp.one, -1, 0.0};
   std::vector<std::vector<HostBlockProg::Unit>> stream(warps);
@@ -1175,7 +1179,7 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
     std::vector<size_t> cost, order;
     for (const List& l : steps[st]) {
       size_t c = 1;
-      for (const auto& ch : l.chunks) c += (ch.size() + 1) / 2;
+      for (int q = l.begin; q < l.end; ++q) c += static_cast<size_t>((chunks[q].n + 1) / 2);
       order.push_back(cost.size());
       cost.push_back(c);
     }
@@ -1190,17 +1194,18 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
       const int w = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
       load[w] += cost[q];
       const List& l = steps[st][q];
-      for (size_t c = 0; c < l.chunks.size(); ++c) {
-        const auto& ch = l.chunks[c];
-        for (size_t i = 0; i < ch.size(); i += 2) {
+      for (int c = l.begin; c < l.end; ++c) {
+        const Chunk& ch = chunks[c];
+        for (int i = 0; i < ch.n; i += 2) {
           HostBlockProg::Unit u{{pad, pad}, 0, false, false, false};
-          for (size_t k = 0; k < 2 && i + k < ch.size(); ++k) {
-            const int x = static_cast<int>(ch[i + k].ab & 0xffffu), y = static_cast<int>(ch[i + k].ab >> 16);
-            u.t[k] = {x == one ? bp.one : (rev ? aslot : vslot)[x], y == one ? bp.one : vslot[y], ch[i + k].widx, ch[i + k].cfix};
+          for (int k = 0; k < 2 && i + k < ch.n; ++k) {
+            const HostProg::Rec& t = rec(ch, i + k);
+            const int x = static_cast<int>(t.ab & 0xffffu), y = static_cast<int>(t.ab >> 16);
+            u.t[k] = {x == one ? bp.one : (rev ? aslot : vslot)[x], y == one ? bp.one : vslot[y], t.widx, t.cfix};
           }
-          if (i + 2 >= ch.size()) {
+          if (i + 2 >= ch.n) {
             u.chunk_end = true;
-            u.list_end = c + 1 == l.chunks.size();
+            u.list_end = c + 1 == l.end;
             u.target = (rev ? aslot : vslot)[l.target];
           }
           stream[w].push_back(u);
@@ -1232,7 +1237,7 @@ HostBlockProg build_block_prog(const Model& m, const HostProg& hp, const std::ve
 
 // Serialises the block programs into one 16-byte aligned device image and binds them.
 void upload_block_progs(const Model& m, const HostBlockProg* const (&progs)[2], DevBuf& buf, cudaStream_t s,
-                        BlockProg (&out)[2]) {
+                        BlockProg (&out)[2], std::vector<WeightPatch>& patches) {
   std::vector<unsigned char> img;
   auto put = [&](const void* p, size_t n) {
     const size_t o = (img.size() + 15) & ~size_t(15);
@@ -1263,6 +1268,10 @@ void upload_block_progs(const Model& m, const HostBlockProg* const (&progs)[2], 
       units[q] = make_int4(static_cast<int>(x[0]), y[0], static_cast<int>(x[1]), y[1]);
     }
     off[k][0] = put(units.data(), sizeof(int4) * units.size());
+    for (size_t q = 0; q < units.size(); ++q)
+      for (int i = 0; i < 2; ++i)
+        if (bp.units[q].t[i].widx >= 0)
+          patches.push_back({off[k][0] + sizeof(int4) * q + sizeof(int) * (i ? 3 : 1), bp.units[q].t[i].widx, k == 1});
     const std::vector<int>* lists[] = {&bp.begin, &bp.basic_slot, &bp.basic_adj, &bp.zero_v, &bp.zero_adj, &bp.seed_v, &bp.seed_adj,
                                        &bp.keep, &bp.zero_late, &bp.rank_v, &bp.rank_adj};
     for (int i = 0; i < 11; ++i) off[k][1 + i] = put(lists[i]->data(), sizeof(int) * lists[i]->size());
@@ -1291,7 +1300,7 @@ void upload_block_progs(const Model& m, const HostBlockProg* const (&progs)[2], 
 // Serialises the programs of the passes into one 16-byte aligned device image and binds them.
 template <typename Real>
 void upload_progs(const Model& m, const std::vector<const HostProg*>& progs, DevBuf& buf, cudaStream_t s,
-                  std::vector<GraphProg<Real>>& out) {
+                  std::vector<GraphProg<Real>>& out, std::vector<WeightPatch>& patches) {
   std::vector<unsigned char> img;
   auto put = [&](const void* p, size_t n) {
     const size_t o = (img.size() + 15) & ~size_t(15);
@@ -1315,6 +1324,10 @@ void upload_progs(const Model& m, const std::vector<const HostProg*>& progs, Dev
       rows[q].c = static_cast<Real>(x.widx >= 0 ? w[x.widx] : x.cfix);
     }
     o.rows = put(rows.data(), sizeof(ProgRec<Real>) * rows.size());
+    for (size_t q = 0; q < rows.size(); ++q)
+      if (hp->rows[q].widx >= 0)
+        patches.push_back({o.rows + static_cast<size_t>(reinterpret_cast<const char*>(&rows[q].c) - reinterpret_cast<const char*>(rows.data())),
+                         hp->rows[q].widx, hp->gate});
     offs.push_back(o);
   }
   if (img.empty()) img.resize(16);
@@ -1336,15 +1349,10 @@ void upload_progs(const Model& m, const std::vector<const HostProg*>& progs, Dev
 }
 
 template <typename Real>
-PassTables<Real> bind_pass(const PassOffsets& o, const int* I, const Real* R) {
+PassTables<Real> bind_pass(const PassOffsets& o, int ndst, const Real* R) {
   PassTables<Real> t{};
-  t.coeff = R + o.coeff; t.scal = R + o.scal; t.wcenter = R + o.wc; t.wsource = R + o.ws; t.wadd = R + o.wa;
-  t.ndst = o.ndst; t.dst_node = I + o.dst_node; t.dst_begin = I + o.dst_begin; t.dst_src = I + o.dst_src; t.dst_w = R + o.dst_w;
-  t.src_begin = I + o.src_begin; t.src_dst = I + o.src_dst; t.src_w = R + o.src_w;
-  t.levels = o.levels; t.level_begin = I + o.level_begin; t.out_nodes = I + o.out_nodes; t.out_begin = I + o.out_begin;
-  t.fprod_a = I + o.fa; t.fprod_b = I + o.fb; t.fprod_c = R + o.fc;
-  t.rlevel_begin = I + o.rlevel_begin; t.in_nodes = I + o.in_nodes; t.in_begin = I + o.in_begin;
-  t.rprod_out = I + o.rout; t.rprod_other = I + o.rother; t.rprod_c = R + o.rc;
+  t.coeff = R + o.coeff; t.scal = R + o.scal; t.wcenter = t.wsource = R + o.wc; t.wadd = R + o.wa;
+  t.ndst = ndst;
   return t;
 }
 
@@ -1374,6 +1382,7 @@ Engine::Engine(const Model& model, int device, int precision) : model_(model), d
   if (model_.gated && !unique(model_.gate_nodes)) throw Error(3, "SUS2 model: duplicate gate scalar moments");
   if (model_.K > kMaxK) throw Error(3, "SUS2 model: sh_k_max above 8 is not supported by the GPU engine");
   plans_ = new std::vector<FramePlan>();
+  weight_copies_ = new std::vector<ValueCopy>();
   SUS2G_CUDA(cudaMallocHost(&host_total_, 8 * sizeof(int)));
   // [0] error code, [1] cell-list edge capacity overflow (largest count), [2] bin capacity overflow
   error_.ensure(3 * sizeof(int));
@@ -1387,6 +1396,7 @@ Engine::Engine(const Model& model, int device, int precision) : model_(model), d
 Engine::~Engine() {
   reset_step_graph();
   delete plans_;
+  delete static_cast<std::vector<ValueCopy>*>(weight_copies_);
   if (host_total_) cudaFreeHost(host_total_);
   if (pinned_) cudaFreeHost(pinned_);
   for (cudaEvent_t e : event_pool_) cudaEventDestroy(e);
@@ -1420,38 +1430,44 @@ std::vector<int> basic_table(const Model& m) {
 }
 }  // namespace
 
+// The device tables at the current parameters.  The first call builds and uploads the structure
+// (index lists, graph programs, gradient layout); later ones send the parameter-dependent values and
+// copy the rank weights into the programs on the device.
 template <typename Real>
 void Engine::upload_tables() {
   const Model& m = model_;
-  Packer pk;
-  const std::vector<int> basic_of = basic_table(m);
-  const int o_basic = pk.add_int(basic_of);
-  PassOffsets po = pack_pass(m, false, pk);
-  PassOffsets pg = m.gated ? pack_pass(m, true, pk) : po;
-  const int o_lin = pk.add_real(m.linear);
-  const int o_map = pk.add_int(m.scalar_map);
-  std::vector<double> wmat;
-  std::vector<int> nodes = m.gate_nodes;
-  if (m.gated) {
-    wmat.resize(static_cast<size_t>(m.F) * m.Q);
-    for (int mu = 0; mu < m.F; ++mu)
-      for (int q = 0; q < m.Q; ++q) wmat[static_cast<size_t>(mu) * m.Q + q] = m.gate_weight(mu, q);
+  const cudaStream_t us = stream_;
+  // species and shift (FP64), then the values; the host copies die at return, hence the
+  // synchronisation at the end (which also orders the tables before work on any later stream)
+  std::vector<Real> values;
+  const ValueOffsets vo = pack_values<Real>(m, values);
+  const size_t dbl_bytes = sizeof(double) * 2 * static_cast<size_t>(m.C), bytes = dbl_bytes + sizeof(Real) * values.size();
+  std::vector<unsigned char> img(bytes);
+  std::memcpy(img.data(), m.species.data(), dbl_bytes / 2);
+  std::memcpy(img.data() + dbl_bytes / 2, m.shift.data(), dbl_bytes / 2);
+  std::memcpy(img.data() + dbl_bytes, values.data(), sizeof(Real) * values.size());
+  tab_value_.ensure(bytes);
+  SUS2G_CUDA(cudaMemcpyAsync(tab_value_.ptr, img.data(), bytes, cudaMemcpyHostToDevice, us));
+  const Real* R = reinterpret_cast<const Real*>(tab_value_.as<unsigned char>() + dbl_bytes);
+  if (dev_model_) {
+    static_cast<DevModel<Real>*>(dev_model_)->scaling = Real(m.scaling);
+    copy_weights<Real>();
+    SUS2G_CUDA(cudaStreamSynchronize(us));
+    return;
   }
-  const int o_wmat = pk.add_real(wmat);
-  std::vector<double> wmat_t(wmat.size());
-  for (int mu = 0; mu < m.F && m.gated; ++mu)
-    for (int q = 0; q < m.Q; ++q) wmat_t[static_cast<size_t>(q) * m.F + mu] = wmat[static_cast<size_t>(mu) * m.Q + q];
-  const int o_wmat_t = pk.add_real(wmat_t);
-  const int o_nodes = pk.add_int(nodes);
+  Packer pk;
+  const int o_basic = pk.add_int(basic_table(m)), o_map = pk.add_int(m.scalar_map), o_nodes = pk.add_int(m.gate_nodes);
   // parameter-gradient layout: block offsets in the trainer's order and rank-weight row lists
   std::map<std::string, int> off;
   for (const auto& b : m.layout()) off[b.name] = b.offset;
   auto block = [&](const char* n) { auto it = off.find(n); return it == off.end() ? -1 : it->second; };
   auto weight_rows = [&](const std::vector<ContractionRow>& rows, int nw, int& o_begin, int& o_src, int& o_dst) {
+    std::vector<std::vector<const ContractionRow*>> of(nw);
+    for (const auto& r : rows)
+      if (r.widx >= 0 && r.widx < nw) of[r.widx].push_back(&r);
     std::vector<int> begin{0}, src, dst;
-    for (int w = 0; w < nw; ++w) {
-      for (const auto& r : rows)
-        if (r.widx == w) { src.push_back(r.src); dst.push_back(r.dst); }
+    for (const auto& list : of) {
+      for (const ContractionRow* r : list) { src.push_back(r->src); dst.push_back(r->dst); }
       begin.push_back(static_cast<int>(src.size()));
     }
     o_begin = pk.add_int(begin);
@@ -1487,79 +1503,136 @@ void Engine::upload_tables() {
     gl.gate.nw = static_cast<int>(m.gate_w.size());
     weight_rows(m.gate_rows, gl.gate.nw, gw_b, gw_s, gw_d);
   }
-  std::vector<double> dbl(m.species);
-  dbl.insert(dbl.end(), m.shift.begin(), m.shift.end());
-
-  std::vector<Real> reals(pk.reals.begin(), pk.reals.end());
   if (pk.ints.empty()) pk.ints.push_back(0);
-  if (reals.empty()) reals.push_back(Real(0));
   tab_int_.ensure(sizeof(int) * pk.ints.size());
-  tab_real_.ensure(sizeof(Real) * reals.size());
-  tab_dbl_.ensure(sizeof(double) * dbl.size());
   // stream-ordered copies: the engine stream is non-blocking, so a legacy-stream copy would not
-  // order against its next kernel; the host vectors die at return, hence the synchronisation
-  const cudaStream_t us = stream_ ? stream_ : own_stream_;
+  // order against its next kernel; the host vectors die at return, hence the synchronisation below
   SUS2G_CUDA(cudaMemcpyAsync(tab_int_.ptr, pk.ints.data(), sizeof(int) * pk.ints.size(), cudaMemcpyHostToDevice, us));
-  SUS2G_CUDA(cudaMemcpyAsync(tab_real_.ptr, reals.data(), sizeof(Real) * reals.size(), cudaMemcpyHostToDevice, us));
-  SUS2G_CUDA(cudaMemcpyAsync(tab_dbl_.ptr, dbl.data(), sizeof(double) * dbl.size(), cudaMemcpyHostToDevice, us));
-  SUS2G_CUDA(cudaStreamSynchronize(us));
   const int* I = tab_int_.as<int>();
-  const Real* R = tab_real_.as<Real>();
   auto* dm = new DevModel<Real>();
+  dev_model_ = dm;
   dm->C = m.C; dm->L = m.L; dm->K = m.K; dm->B = m.B; dm->F = m.F; dm->H = m.H; dm->M = m.M; dm->NB = m.NB;
   dm->S = m.S; dm->Q = m.Q; dm->nblk = m.nblk; dm->scaling_mode = m.scaling_mode;
   dm->rmax = Real(m.max_dist); dm->rang = Real(m.angular); dm->scaling = Real(m.scaling);
   dm->split = m.split; dm->poly = m.poly_cutoff; dm->cutoff_p = m.cutoff_p; dm->gated = m.gated;
   dm->species_readout = m.species_readout;
   dm->basic_of = I + o_basic;
-  dm->outer = bind_pass<Real>(po, I, R);
-  dm->gate = bind_pass<Real>(pg, I, R);
+  auto ndst = [](const std::vector<ContractionRow>& rows) {
+    std::vector<int> d;
+    for (const auto& r : rows) d.push_back(r.dst);
+    std::sort(d.begin(), d.end());
+    return static_cast<int>(std::unique(d.begin(), d.end()) - d.begin());
+  };
+  dm->outer = bind_pass<Real>(vo.outer, ndst(m.outer_rows), R);
+  dm->gate = m.gated ? bind_pass<Real>(vo.gate, ndst(m.gate_rows), R) : dm->outer;
+  weight_value_[0] = R + vo.outer_w;
+  weight_value_[1] = R + vo.gate_w;
+  prog_[0].reset(new HostProg(build_prog(m, false)));
+  prog_[1].reset(new HostProg(m.gated ? build_prog(m, true) : HostProg{}));
   {
-    // the programs' structure is built once per engine; uploads refresh the rank weights
-    if (!prog_[0]) {
-      prog_[0].reset(new HostProg(build_prog(m, false)));
-      prog_[1].reset(new HostProg(m.gated ? build_prog(m, true) : HostProg{}));
-    }
     std::vector<GraphProg<Real>> bound;
-    upload_progs<Real>(m, {prog_[0].get(), prog_[1].get()}, tab_prog_, us, bound);
+    std::vector<WeightPatch> patches;
+    upload_progs<Real>(m, {prog_[0].get(), prog_[1].get()}, tab_prog_, us, bound, patches);
+    add_weight_copies<Real>(tab_prog_.ptr, &patches);
     dm->outer.prog = bound[0];
     dm->gate.prog = m.gated ? bound[1] : bound[0];
     dm->prog_parts = std::max(bound[0].max_parts, m.gated ? bound[1].max_parts : 0);
   }
-  dm->linear = R + o_lin;
-  dm->species = tab_dbl_.as<double>();
-  dm->shift = tab_dbl_.as<double>() + m.C;
+  dm->linear = R + vo.linear;
+  dm->species = tab_value_.as<double>();
+  dm->shift = tab_value_.as<double>() + m.C;
   dm->scalar_map = I + o_map;
-  dm->gate_wmat = R + o_wmat;
-  dm->gate_wmat_t = R + o_wmat_t;
+  dm->gate_wmat = R + vo.wmat;
+  dm->gate_wmat_t = R + vo.wmat_t;
   dm->gate_nodes = I + o_nodes;
   gl.outer.w_begin = I + ow_b; gl.outer.w_src = I + ow_s; gl.outer.w_dst = I + ow_d;
   gl.gate.w_begin = I + gw_b; gl.gate.w_src = I + gw_s; gl.gate.w_dst = I + gw_d;
   dm->grad = gl;
-  delete static_cast<DevModel<Real>*>(dev_model_);
-  dev_model_ = dm;
-  if constexpr (sizeof(Real) == 4) {
-    if (block_prog_[0]) upload_block_programs(false);
-    if (dual_prog_[0]) upload_block_programs(true);
-  }
+  if (sizeof(Real) == 4 && m.B == 8) upload_block_programs(false);
+  SUS2G_CUDA(cudaStreamSynchronize(us));
 }
 
-// The block programs of the split passes (dual: of the split gradient), from their first use on: the
-// structure is built once per engine, uploads refresh the rank weights.
+// The places of a program image that hold rank weights join the list of copies (sent to the device
+// at the next parameter upload: an engine that never gets one needs no list there).
+template <typename Real>
+void Engine::add_weight_copies(void* image, const void* weight_patches) {
+  auto& list = *static_cast<std::vector<ValueCopy>*>(weight_copies_);
+  for (const WeightPatch& p : *static_cast<const std::vector<WeightPatch>*>(weight_patches))
+    list.push_back({static_cast<unsigned char*>(image) + p.at, static_cast<const Real*>(weight_value_[p.gate ? 1 : 0]) + p.widx});
+}
+template <typename Real>
+void Engine::copy_weights() {
+  const auto& list = *static_cast<std::vector<ValueCopy>*>(weight_copies_);
+  const int n = static_cast<int>(list.size());
+  if (n == 0) return;
+  if (copies_sent_ != list.size()) {
+    tab_copies_.ensure(sizeof(ValueCopy) * list.size());
+    SUS2G_CUDA(cudaMemcpyAsync(tab_copies_.ptr, list.data(), sizeof(ValueCopy) * list.size(), cudaMemcpyHostToDevice, stream_));
+    copies_sent_ = list.size();
+  }
+  k_copy_values<Real><<<(n + 255) / 256, 256, 0, stream_>>>(tab_copies_.as<ValueCopy>(), n);
+  SUS2G_CUDA(cudaGetLastError());
+}
+
+// The block programs of the split passes, built with the tables, or (dual) of the split gradient,
+// built at its first use.
 void Engine::upload_block_programs(bool dual) {
   const Model& m = model_;
   auto* dm = static_cast<DevModel<float>*>(dev_model_);
-  auto& host = dual ? dual_prog_ : block_prog_;
-  if (!host[0]) {
-    const std::vector<int> basic_of = basic_table(m);
-    host[0].reset(new HostBlockProg(build_block_prog(m, *prog_[0], basic_of, dual)));
-    host[1].reset(new HostBlockProg(m.gated ? build_block_prog(m, *prog_[1], basic_of, dual) : HostBlockProg{}));
-  }
+  const std::vector<int> basic_of = basic_table(m);
+  HostBlockProg host[2];
+  host[0] = build_block_prog(m, *prog_[0], basic_of, dual);
+  if (m.gated) host[1] = build_block_prog(m, *prog_[1], basic_of, dual);
   BlockProg blocks[2];
-  const HostBlockProg* const hosts[2] = {host[0].get(), host[1].get()};
-  upload_block_progs(m, hosts, dual ? tab_dual_ : tab_block_, stream_ ? stream_ : own_stream_, blocks);
+  const HostBlockProg* const hosts[2] = {&host[0], &host[1]};
+  DevBuf& buf = dual ? tab_dual_ : tab_block_;
+  std::vector<WeightPatch> patches;
+  upload_block_progs(m, hosts, buf, stream_, blocks, patches);
+  add_weight_copies<float>(buf.ptr, &patches);
   (dual ? dm->outer.dual : dm->outer.block) = blocks[0];
   (dual ? dm->gate.dual : dm->gate.block) = blocks[1];
+  if (dual) have_dual_ = true;
+}
+
+// Takes the parameters (and scaling) of a model of the same structure, as a new engine for it would
+// start: settings at their defaults, no geometry, the caller's stream released.
+bool Engine::take_params(const Model& m) {
+  if (!model_.same_structure(m)) return false;
+  SUS2G_CUDA(cudaSetDevice(device_));
+  SUS2G_CUDA(cudaStreamSynchronize(stream_));
+  SUS2G_CUDA(cudaStreamSynchronize(aux_stream_));
+  rev_pending_ = false;
+  reset_step_graph();
+  stream_ = own_stream_;
+  std::vector<double> p(static_cast<size_t>(m.param_count()));
+  m.get_params(p.data());
+  model_.set_params(p.data());
+  model_.scaling = m.scaling;
+  step_graphs_ = true;
+  pdl_ = default_pdl();
+  moment_mma_ = false;
+  grad_split_ = true;
+  set_timing(false);
+  open_stage_ = -1;
+  for (int q = 0; q < 4; ++q) {
+    pass_blocks_[q] = pass_grid_[q] = pass_order_[q] = pass_stage_[q] = 0;
+    pass_wpb_[q] = 4;
+  }
+  static_split_ = gate_split_ = -1;
+  split_blocks_ = gate_split_blocks_[0] = gate_split_blocks_[1] = 0;
+  gate_ran_split_ = false;
+  staged_ = 0;
+  desc_out_ = nullptr;
+  natoms_ = nframes_ = ncentres_ = bins_frames_ = 0;
+  nedges_ = exact_edges_ = 0;
+  nedges_exact_ = true;
+  user_edges_ = padded_ = clear_bins_ = false;
+  plans_->clear();
+  launches_ = 0;
+  ++edge_generation_;
+  SUS2G_CUDA(cudaMemsetAsync(error_.ptr, 0, 3 * sizeof(int), stream_));
+  upload_model();
+  return true;
 }
 
 void Engine::upload_model() {
@@ -1573,6 +1646,13 @@ void Engine::upload_model() {
 
 long long Engine::nedges() {
   wait_reverse();
+  if (!nedges_exact_ && user_edges_) {
+    int total = 0;
+    SUS2G_CUDA(cudaMemcpyAsync(&total, row_.as<int>() + natoms_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    SUS2G_CUDA(cudaStreamSynchronize(stream_));
+    exact_edges_ = total;
+    nedges_exact_ = true;
+  }
   if (!nedges_exact_) {
     // padded layout: the sum of the per-centre counts
     std::vector<int> counts(static_cast<size_t>(std::max(0, ncentres_)));
@@ -1926,22 +2006,14 @@ void Engine::finalize_edges() {
   }
   if (user_edges_) {
     const int nall = natoms_;
-    in_row_.ensure(sizeof(int) * (nall + 1));
-    in_edge_.ensure(sizeof(int) * std::max<long long>(1, nedges_));
-    counts_.ensure(sizeof(int) * (nall + 1));
-    SUS2G_CUDA(cudaMemsetAsync(counts_.ptr, 0, sizeof(int) * (nall + 1), s));
     if (nedges_) {
       const unsigned eb = static_cast<unsigned>((nedges_ + 255) / 256);
-      k_iota<<<eb, 256, 0, s>>>(rev_.as<int>(), nedges_);
-      k_count_in<<<eb, 256, 0, s>>>(nbr_.as<int>(), nedges_, counts_.as<int>());
-      launches_ += 2;
-    }
-    k_exclusive_scan<<<1, 1024, 0, s>>>(counts_.as<int>(), nall, in_row_.as<int>(), error_.as<int>());
-    ++launches_;
-    if (nedges_) {
-      const unsigned eb = static_cast<unsigned>((nedges_ + 255) / 256);
-      SUS2G_CUDA(cudaMemsetAsync(counts_.ptr, 0, sizeof(int) * (nall + 1), s));
-      k_fill_in<<<eb, 256, 0, s>>>(nbr_.as<int>(), nedges_, in_row_.as<int>(), counts_.as<int>(), tmp_nbr_.as<int>());
+      if (model_.gated) {  // the outer pass stores its gate-signal adjoints at the edges themselves
+        k_iota<<<eb, 256, 0, s>>>(rev_.as<int>(), nedges_);
+        ++launches_;
+      }
+      k_fill_in<<<eb, 256, 0, s>>>(nbr_.as<int>(), row_.as<int>() + nall, in_row_.as<int>(), counts_.as<int>() + nall + 1,
+                                   tmp_nbr_.as<int>());
       k_sort_in<<<static_cast<unsigned>((static_cast<long long>(nall) * kWarp + 255) / 256), 256, 0, s>>>(
           in_row_.as<int>(), nall, tmp_nbr_.as<int>(), in_edge_.as<int>());
       launches_ += 2;
@@ -1970,6 +2042,18 @@ void Engine::finalize_edges() {
   }
 }
 
+bool Engine::edges_plain(int nowned, int nall, int nedges, const int* d_i, const int* d_j, const double* d_d) {
+  if (nedges <= 0) return true;
+  SUS2G_CUDA(cudaSetDevice(device_));
+  edge_flag_.ensure(sizeof(int));
+  SUS2G_CUDA(cudaMemsetAsync(edge_flag_.ptr, 0, sizeof(int), stream_));
+  k_check_user_edges<<<static_cast<unsigned>((static_cast<long long>(nedges) + 255) / 256), 256, 0, stream_>>>(
+      d_i, d_j, d_d, nedges, nowned, nall, edge_flag_.as<int>());
+  SUS2G_CUDA(cudaGetLastError());
+  SUS2G_CUDA(cudaMemcpyAsync(host_total_ + 7, edge_flag_.ptr, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+  SUS2G_CUDA(cudaStreamSynchronize(stream_));
+  return host_total_[7] == 0;
+}
 void Engine::set_edges(int nowned, int nall, const int* d_types, int nedges, const int* d_i, const int* d_j, const double* d_d) {
   SUS2G_CUDA(cudaSetDevice(device_));
   ++edge_generation_;
@@ -1988,42 +2072,39 @@ void Engine::set_edges(int nowned, int nall, const int* d_types, int nedges, con
   plans[0].a1 = nowned;
   plan_.ensure(sizeof(FramePlan));
   SUS2G_CUDA(cudaMemcpyAsync(plan_.ptr, plans.data(), sizeof(FramePlan), cudaMemcpyHostToDevice, s));
-  counts_.ensure(sizeof(int) * (nowned + 1));
-  row_.ensure(sizeof(int) * (nall + 1));
-  SUS2G_CUDA(cudaMemsetAsync(counts_.ptr, 0, sizeof(int) * (nowned + 1), s));
-  if (nedges) {
-    k_count_centres<<<(nedges + 255) / 256, 256, 0, s>>>(d_i, d_j, nedges, counts_.as<int>(), nowned, nall,
-                                                         error_.as<int>());
-    ++launches_;
-  }
-  long long total = 0;
-  exclusive_scan_host_sync(counts_.as<int>(), nowned, row_.as<int>(), s, &total);
-  nedges_ = exact_edges_ = total;
-  nedges_exact_ = true;
-  const size_t E = std::max<long long>(1, total);
+  // counts of out- and in-edges, both rows by one scan launch (ghosts have no out-edges), then the
+  // scatter; the row ends -- the edges that are in range -- stay on the device
+  const size_t E = std::max(1, nedges);
   const size_t rsz = precision_ == kFP32 ? sizeof(EdgeF) : sizeof(EdgeD);
+  counts_.ensure(sizeof(int) * 2 * (nall + 1));
+  row_.ensure(sizeof(int) * (nall + 1));
+  in_row_.ensure(sizeof(int) * (nall + 1));
+  in_edge_.ensure(sizeof(int) * E);
   nbr_.ensure(sizeof(int) * E); tmp_nbr_.ensure(sizeof(int) * E);
-  rev_.ensure(sizeof(int) * E);
+  if (model_.gated) rev_.ensure(sizeof(int) * E);
   d4_.ensure(rsz * E); tmp_d4_.ensure(rsz * E);
   key_.ensure(sizeof(unsigned long long) * E); tmp_key_.ensure(sizeof(unsigned long long) * E);
-  DevBuf cursor;
-  cursor.ensure(sizeof(int) * (nowned + 1));
-  SUS2G_CUDA(cudaMemsetAsync(cursor.ptr, 0, sizeof(int) * (nowned + 1), s));
+  int* out_count = counts_.as<int>();
+  int* in_count = out_count + nall + 1;
+  SUS2G_CUDA(cudaMemsetAsync(counts_.ptr, 0, sizeof(int) * 2 * (nall + 1), s));
+  const unsigned eb = static_cast<unsigned>((static_cast<long long>(nedges) + 255) / 256);
+  if (nedges) {
+    k_count_user_edges<<<eb, 256, 0, s>>>(d_i, d_j, nedges, out_count, in_count, nowned, nall, error_.as<int>());
+    ++launches_;
+  }
+  k_exclusive_scans<<<2, 1024, 0, s>>>(out_count, in_count, nall, row_.as<int>(), in_row_.as<int>(), error_.as<int>());
+  ++launches_;
   if (nedges) {
     if (precision_ == kFP32)
-      k_scatter_user_edges<float><<<(nedges + 255) / 256, 256, 0, s>>>(d_i, d_j, d_d, nedges, row_.as<int>(), cursor.as<int>(),
+      k_scatter_user_edges<float><<<eb, 256, 0, s>>>(d_i, d_j, d_d, nedges, row_.as<int>(), out_count,
           tmp_nbr_.as<int>(), tmp_d4_.as<EdgeF>(), tmp_key_.as<unsigned long long>(), nowned, nall, error_.as<int>());
     else
-      k_scatter_user_edges<double><<<(nedges + 255) / 256, 256, 0, s>>>(d_i, d_j, d_d, nedges, row_.as<int>(), cursor.as<int>(),
+      k_scatter_user_edges<double><<<eb, 256, 0, s>>>(d_i, d_j, d_d, nedges, row_.as<int>(), out_count,
           tmp_nbr_.as<int>(), tmp_d4_.as<EdgeD>(), tmp_key_.as<unsigned long long>(), nowned, nall, error_.as<int>());
     ++launches_;
   }
-  // rows of ghost atoms are empty
-  if (nall > nowned) {
-    std::vector<int> tail(nall - nowned, static_cast<int>(total));
-    SUS2G_CUDA(cudaMemcpyAsync(row_.as<int>() + nowned + 1, tail.data(), sizeof(int) * tail.size(), cudaMemcpyHostToDevice, s));
-    SUS2G_CUDA(cudaStreamSynchronize(s));
-  }
+  nedges_ = nedges;
+  nedges_exact_ = false;
   finalize_edges();
 }
 
@@ -2067,8 +2148,6 @@ void Engine::run_efs(double* d_energy, double* d_forces, double* d_virial, doubl
   const Model& m = model_;
   cudaStream_t s = stream_;
   const int N = natoms_;
-  if (sizeof(Real) == 4 && m.B == 8 && !block_prog_[0] && (wants_split(static_split_) || (m.gated && wants_split(gate_split_))))
-    upload_block_programs(false);
   PassArgs<Real> a = pass_args<Real>();
   // stage 1: gate forward (Effect) -- gate signals of the centre atoms
   if (stages & kStageGate) {
@@ -2262,7 +2341,7 @@ void Engine::run_grad(const double* ew, const double* fw, const double* sw, doub
   const int N = natoms_, P = m.param_count();
   const size_t E = std::max<long long>(1, nedges_);
   if constexpr (sizeof(Real) == 4)
-    if (m.B == 8 && !dual_prog_[0]) upload_block_programs(true);
+    if (m.B == 8 && !have_dual_) upload_block_programs(true);
   const DevModel<Real>& dm = *static_cast<DevModel<Real>*>(dev_model_);
   GradArgs<Real> a{};
   a.dm = dm;
@@ -2578,7 +2657,6 @@ void Engine::autotune_passes(int reps, int* blocks_out, double* ms_out) {
   const int N = natoms_;
   double* scratch = static_cast<double*>(io(7, sizeof(double) * (7 * static_cast<size_t>(std::max(1, nframes_)) +
                                                                   4 * static_cast<size_t>(std::max(1, N)))));
-  if (sizeof(Real) == 4 && m.B == 8 && !block_prog_[0]) upload_block_programs(false);
   run_efs<Real>(scratch, scratch + 7 * std::max(1, nframes_), scratch + std::max(1, nframes_), nullptr, kStageAll);
   PassArgs<Real> a = pass_args<Real>();
   if (m.gated) {  // the fused gate passes are timed too

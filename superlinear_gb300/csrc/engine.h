@@ -13,7 +13,6 @@ namespace sus2g {
 
 template <typename Real> struct PassArgs;  // efs_kernels.cuh
 struct HostProg;                            // engine.cu: a pass's graph program on the host
-struct HostBlockProg;                       // engine.cu: the same as a block program
 
 enum Precision : int { kFP64 = 0, kFP32 = 1 };
 
@@ -47,6 +46,9 @@ class Engine {
   // Replace the engine's parameter vector (trainer order) and re-upload the device tables.
   void set_params(const double* params) { model_.set_params(params); upload_model(); }
   void set_scaling(double s) { model_.set_scaling(s); upload_model(); }
+  // Parameters and scaling of m when it has this model's structure (false otherwise): the engine is
+  // then as a new one for m, with this one's buffers and programs.
+  bool take_params(const Model& m);
   // Incremented by every build_edges / set_edges: a caller that captured work on this engine's
   // buffers (a CUDA graph) must rebuild it when the generation it recorded has changed, since a
   // rebuild may reallocate the edge and step buffers.
@@ -61,6 +63,9 @@ class Engine {
   // nall atoms; edges need not be sorted; rev is computed from (i, j, d) pairing.
   void set_edges(int nowned, int nall, const int* d_types, int nedges, const int* d_i, const int* d_j,
                  const double* d_d);
+  // Whether every caller edge (device arrays) has its indices in range and a length far from zero
+  // and overflow; waits for the stream and leaves the engine's geometry as it is.
+  bool edges_plain(int nowned, int nall, int nedges, const int* d_i, const int* d_j, const double* d_d);
 
   // One E/F/virial step of periodic frames with device positions / types / outputs (build_edges +
   // efs).  For cell-list batches the second consecutive step of a layout -- frame sizes, cells,
@@ -220,6 +225,8 @@ class Engine {
  private:
   template <typename Real> void upload_tables();
   void upload_block_programs(bool dual);
+  template <typename Real> void add_weight_copies(void* image, const void* weight_patches);
+  template <typename Real> void copy_weights();
   template <typename Real> PassArgs<Real> pass_args();
   template <typename Real> void autotune_passes(int reps, int* blocks_out, double* ms_out);
   enum : int { kStageGate = 1, kStageOuter = 2, kStageFinish = 4, kStageAll = 7 };
@@ -253,10 +260,13 @@ class Engine {
   unsigned long long edge_generation_ = 0;
 
   // model tables (both precisions are packed into one buffer each)
-  DevBuf tab_int_, tab_real_, tab_dbl_, tab_prog_;
+  DevBuf tab_int_, tab_value_, tab_prog_, tab_copies_;
+  const void* weight_value_[2] = {nullptr, nullptr};  // the rank weights in it (outer, gate)
+  void* weight_copies_ = nullptr;           // their copies in the programs (host list)
+  size_t copies_sent_ = 0;                  // its length on the device
   std::unique_ptr<HostProg> prog_[2];  // outer and gate graph programs (structure built once)
-  std::unique_ptr<HostBlockProg> block_prog_[2], dual_prog_[2];
   DevBuf tab_block_, tab_dual_;
+  bool have_dual_ = false;
   void* dev_model_ = nullptr;  // host copy of DevModel<Real>
 
   // geometry
@@ -275,7 +285,7 @@ class Engine {
   DevBuf bin_count_, bin_rec_, bin_pos_, bin_posf_, rec_of_;
   const int* d_types_ = nullptr;
   bool user_edges_ = false;     // caller-supplied edges: no reverse partners, scatter instead of gather
-  DevBuf hbar_atom_, bin_of_, frac_, off_, in_row_, in_edge_;  // in_*: caller edges grouped by neighbour
+  DevBuf edge_flag_, hbar_atom_, bin_of_, frac_, off_, in_row_, in_edge_;  // in_*: caller edges grouped by neighbour
   DevBuf pad_nbr_, pad_d4_, pad_key_;  // padded single-pass staging of cell-list frames
   double cap_scale_ = 2.0;      // padded capacity = cap_scale x mean neighbour count + 64 (grows on overflow)
   double bin_cap_scale_ = 2.0;  // bin capacity = bin_cap_scale x mean atoms per bin + 8 (grows on overflow)

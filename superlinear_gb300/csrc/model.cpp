@@ -524,9 +524,27 @@ void Model::set_params(const double* in) {
     auto* v = block_ptr(b.name);
     std::copy(in + b.offset, in + b.offset + b.size, v->begin());
   }
-  outer_rows.clear();
-  gate_rows.clear();
-  derive();
+}
+
+bool Model::same_structure(const Model& o) const {
+  auto products_equal = [](const std::vector<Product>& a, const std::vector<Product>& b) {
+    return a.size() == b.size() && std::equal(a.begin(), a.end(), b.begin(), [](const Product& x, const Product& y) {
+             return x.a == y.a && x.b == y.b && x.out == y.out && x.c == y.c;
+           });
+  };
+  const std::vector<Block> la = layout(), lb = o.layout();
+  const bool blocks = la.size() == lb.size() && std::equal(la.begin(), la.end(), lb.begin(), [](const Block& x, const Block& y) {
+                        return x.name == y.name && x.offset == y.offset && x.size == y.size;
+                      });
+  return blocks && C == o.C && L == o.L && K == o.K && B == o.B && F == o.F && M == o.M && S == o.S && Q == o.Q &&
+         scaling_mode == o.scaling_mode && min_dist == o.min_dist && max_dist == o.max_dist && angular == o.angular &&
+         poly_cutoff == o.poly_cutoff && cutoff_p == o.cutoff_p && species_readout == o.species_readout && basic == o.basic &&
+         products_equal(products, o.products) && scalar_map == o.scalar_map && outer_rank == o.outer_rank &&
+         outer_begin == o.outer_begin && outer_product == o.outer_product && gate_rank == o.gate_rank &&
+         gate_begin == o.gate_begin && gate_product_begin == o.gate_product_begin && gate_product_end == o.gate_product_end &&
+         gated == o.gated && body_combo == o.body_combo && gate_decoupled == o.gate_decoupled &&
+         gate_shared_radial == o.gate_shared_radial && gate_nodes == o.gate_nodes && gate_body == o.gate_body &&
+         body_count == o.body_count;
 }
 
 }  // namespace sus2g

@@ -91,6 +91,8 @@ struct Model {
   int param_count() const;
   void get_params(double* out) const;
   void set_params(const double* in);
+  // Whether o differs from this model in parameter values and the radial scaling only.
+  bool same_structure(const Model& o) const;
   // The global radial scaling (the `scaling` field, MLMTPR::scaling): not a trained coefficient,
   // set by the trainer's rescale step and written back by save().
   void set_scaling(double s);
