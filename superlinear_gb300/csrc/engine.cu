@@ -66,8 +66,8 @@ __global__ void k_frame_of(const FramePlan* plans, int nframes, int* frame_of, c
 // its count; the host then grows bcap and repeats the step.  With find_frame the atom's frame is
 // found here (binary search over the frames' first atoms) and written to frame_of.
 __global__ void k_bin_place(const FramePlan* plans, int nframes, bool find_frame, int* frame_of, const double* pos,
-                            int natoms, int bcap, int* bin_of, int* rec_of, int* bin_count, AtomFrac* frac,
-                            AtomOff* off, BinAtom* bin_rec, BinPos* bin_pos, BinPosF* bin_posf, int* bin_over,
+                            int natoms, int bcap, int* rec_of, int* bin_count, AtomOff* off, AtomOff* bin_off,
+                            BinPos* bin_pos, BinPosF* bin_posf, int* bin_over,
                             int* error, const int* types, int C) {
   pdl_launch_dependents();  // the fill kernel's blocks may become resident while this grid runs
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -87,7 +87,7 @@ __global__ void k_bin_place(const FramePlan* plans, int nframes, bool find_frame
   }
   const FramePlan& fp = plans[f];
   if (types[i] < 0 || types[i] >= C) record_error(error, kErrBadSpecies);
-  if (!fp.use_bins) { bin_of[i] = -1; return; }
+  if (!fp.use_bins) return;
   const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
   // fractional coordinates, checked before any conversion to an integer: a non-finite coordinate,
   // or one more than 2^30 cells from the home cell, is reported and the atom binned inertly at
@@ -100,23 +100,19 @@ __global__ void k_bin_place(const FramePlan* plans, int nframes, bool find_frame
   }
   if (!finite) record_error(error, kErrBadPosition);
   int b[3], o[3];
-  float w32[3];
   for (int q = 0; q < 3; ++q) {
     const double fl = finite ? floor(sq[q]) : 0.0;
     const double w = finite ? sq[q] - fl : 0.0;
     o[q] = static_cast<int>(fl);
-    w32[q] = static_cast<float>(w);
     b[q] = max(0, min(static_cast<int>(w * fp.nb[q]), fp.nb[q] - 1));
   }
-  frac[i] = AtomFrac{w32[0], w32[1], w32[2], 0};
-  off[i] = AtomOff{o[0], o[1], o[2], 0};
+  off[i] = AtomOff{o[0], o[1], o[2], (b[0] << 20) | (b[1] << 10) | b[2]};
   const int bin = fp.bin0 + (b[0] * fp.nb[1] + b[1]) * fp.nb[2] + b[2];
-  bin_of[i] = bin;
   const int slot = atomicAdd(bin_count + bin, 1);
   if (slot >= bcap) { atomicMax(bin_over, slot + 1); rec_of[i] = 0; return; }
   const long long rec = static_cast<long long>(bin) * bcap + slot;
   rec_of[i] = static_cast<int>(rec);
-  bin_rec[rec] = BinAtom{w32[0], w32[1], w32[2], i, o[0], o[1], o[2], 0};
+  bin_off[rec] = AtomOff{o[0], o[1], o[2], 0};
   const double* c = fp.cell;
   const double a0 = o[0], a1 = o[1], a2 = o[2];
   const double bad = finite ? 0.0 : nan("");
@@ -127,17 +123,6 @@ __global__ void k_bin_place(const FramePlan* plans, int nframes, bool find_frame
   const float hx = static_cast<float>(wx), hy = static_cast<float>(wy), hz = static_cast<float>(wz);
   bin_posf[rec] = BinPosF{hx, hy, hz, i, static_cast<float>(wx - hx), static_cast<float>(wy - hy),
                           static_cast<float>(wz - hz), 0};
-}
-
-// One cell-list edge record: components and distance already in the record's precision.
-template <typename Real>
-__device__ __forceinline__ void write_edge_rec(long long e, int j, int a, int b, int c, Real x, Real y, Real z, Real r,
-                                               int* nbr, typename Vec4<Real>::type* d4, unsigned long long* key) {
-  nbr[e] = j;
-  typename Vec4<Real>::type v;
-  v.x = x; v.y = y; v.z = z; v.w = r;
-  d4[e] = v;
-  key[e] = edge_key(j, a, b, c);
 }
 
 template <typename Real>
@@ -199,22 +184,69 @@ __device__ __forceinline__ void sort_centre_edges(int lane, int n, long long pad
   }
 }
 
+// A centre's edges between the walk and the sort: the first kStage of them in shared memory, the
+// rest in its padded slots of the staging buffers.
+template <typename Real> struct EdgeStage {
+  static constexpr int kStage = sizeof(Real) == 4 ? 128 : 64;
+  typename Vec4<Real>::type d4[kStage];
+  int j[kStage], image[kStage];
+};
+
+// rank[u] = how many of the centre's n neighbours come before neighbour mine[u].  A cell-list frame
+// is at least 3 r_c wide, so a neighbour appears once per centre and its index alone is the order.
+template <int U, typename Real>
+__device__ __forceinline__ void rank_neighbours(int n, const EdgeStage<Real>& st, const int* rest, const int (&mine)[U],
+                                                int (&rank)[U]) {
+  const int staged = min(n, EdgeStage<Real>::kStage);
+#pragma unroll
+  for (int u = 0; u < U; ++u) rank[u] = 0;
+  int t = 0;
+  for (; t + 4 <= staged; t += 4) {
+    const int4 o = *reinterpret_cast<const int4*>(st.j + t);
+#pragma unroll
+    for (int u = 0; u < U; ++u) rank[u] += (o.x < mine[u]) + (o.y < mine[u]) + (o.z < mine[u]) + (o.w < mine[u]);
+  }
+  for (; t < n; ++t) {
+    const int o = t < staged ? st.j[t] : rest[t];
+#pragma unroll
+    for (int u = 0; u < U; ++u) rank[u] += o < mine[u];
+  }
+}
+
+// The order of a centre's n <= 128 edges: perm[rank] = place in the stage (32 U places).
+template <int U, typename Real>
+__device__ __forceinline__ void order_edges(int lane, int n, const EdgeStage<Real>& st, const int* rest, int* perm) {
+  int mine[U], rank[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int q = u * kWarp + lane;
+    mine[u] = q >= n ? 0 : q < EdgeStage<Real>::kStage ? st.j[q] : rest[q];
+  }
+  rank_neighbours<U, Real>(n, st, rest, mine, rank);
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (u * kWarp + lane < n) perm[rank[u]] = u * kWarp + lane;
+}
+
 // Cell-list frames: one warp per centre over its 125 stencil bins (warp_bin_edges), one pass.  The
-// centre's edges go to its padded slots pad0 + (i - a0) cap .. + cap of the staging buffers; a
-// count above cap is clamped to cap and raises *overflow to the full count, which the host reads
-// with the step's error check (it then grows the capacity and repeats the step).  With row_end the
-// kernel then sorts the centre's edges into the final arrays at the same slots.
+// centre's edges are staged, put in order by neighbour and written once, coalesced, to its padded
+// slots pad0 + (i - a0) cap .. + cap; a count above cap is clamped to cap and raises *overflow to
+// the full count, which the host reads with the step's error check (it then grows the capacity and
+// repeats the step).
+// Bound by the instructions of the walk and the sort.  32,768 atoms of 92 edges: 164 us with 64-bit
+// keys ranked four per lane for any count, staging in global memory and a fractional prefilter; 118 us
+// so.
 template <typename Real>
 __global__ void __launch_bounds__(kFillWarps * kWarp, 4)
 k_edge_fill_bins(const FramePlan* plans, const int* frame_of, const double* pos, int natoms, double rc2,
-                 const int* bin_count, int bin_cap, const BinAtom* bin_rec, const BinPos* bin_pos,
-                 const BinPosF* bin_posf, const int* bin_of, const int* rec_of, const AtomFrac* frac, const AtomOff* off,
+                 const int* bin_count, int bin_cap, const AtomOff* bin_off, const BinPos* bin_pos,
+                 const BinPosF* bin_posf, const int* rec_of, const AtomOff* off,
                  int* counts, int* nbr,
                  typename Vec4<Real>::type* d4, unsigned long long* key, int* overflow, int* error, int* row,
                  int* row_end, unsigned long long* key_out, int* nbr_out, typename Vec4<Real>::type* d4_out) {
-  __shared__ int2 queue[kFillWarps][kEdgeQueue];
-  __shared__ BinWalk walk[kFillWarps];
-  __shared__ unsigned long long skeys[kFillWarps][kFillSortStage];
+  using Stage = EdgeStage<Real>;
+  __shared__ __align__(16) BinWalk<Real> walks[kFillWarps];
+  __shared__ __align__(16) Stage stages[kFillWarps];
   pdl_wait();  // the bins and frame map of the previous kernel
   pdl_launch_dependents();
   const int i = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kWarp);
@@ -225,15 +257,22 @@ k_edge_fill_bins(const FramePlan* plans, const int* frame_of, const double* pos,
   const unsigned below = (1u << lane) - 1u;
   const long long pad = fp.pad0 + static_cast<long long>(i - fp.a0) * fp.cap;
   const int cap = fp.cap;
+  Stage& st = stages[w];
   int cursor = 0;
-  warp_bin_edges<Real>(i, fp, pos, rc2, bin_count, bin_cap, bin_rec, bin_pos, bin_posf, bin_of, rec_of, frac, off, error,
-                       queue[w], walk[w],
-                       [&](unsigned mask, bool ok, int j, int a, int b, int c, Real x, Real y, Real z, Real r) {
+  warp_bin_edges<Real>(i, fp, pos, rc2, bin_count, bin_cap, bin_off, bin_pos, bin_posf, rec_of, off, error, walks[w],
+                       [&](unsigned mask, bool ok, int j, int image, Real x, Real y, Real z, Real r) {
                          if (ok) {
                            const int k = cursor + __popc(mask & below);
-                           if (k < cap) {
-                             write_edge_rec<Real>(pad + k, j, a, b, c, x, y, z, r, nbr, d4, key);
-                             if (k < kFillSortStage) skeys[w][k] = edge_key(j, a, b, c);
+                           typename Vec4<Real>::type v;
+                           v.x = x; v.y = y; v.z = z; v.w = r;
+                           if (k < Stage::kStage) {
+                             st.d4[k] = v;
+                             st.j[k] = j;
+                             st.image[k] = image;
+                           } else if (k < cap) {
+                             d4[pad + k] = v;
+                             nbr[pad + k] = j;
+                             key[pad + k] = static_cast<unsigned long long>(image);
                            }
                          }
                          cursor += __popc(mask);
@@ -242,13 +281,36 @@ k_edge_fill_bins(const FramePlan* plans, const int* frame_of, const double* pos,
   if (lane == 0) {
     counts[i] = n;
     if (cursor > cap) atomicMax(overflow, cursor);
-  }
-  if (!row_end) return;
-  __syncwarp();
-  sort_centre_edges<Real>(lane, n, pad, skeys[w], key, nbr, d4, key_out, nbr_out, d4_out);
-  if (lane == 0) {
     row[i] = static_cast<int>(pad);
     row_end[i] = static_cast<int>(pad) + n;
+  }
+  const int* rest = nbr + pad;
+  auto write = [&](int to, int from) {
+    const bool staged = from < Stage::kStage;
+    const int j = staged ? st.j[from] : rest[from];
+    const unsigned long long image = staged ? static_cast<unsigned long long>(st.image[from]) : key[pad + from];
+    key_out[pad + to] = (static_cast<unsigned long long>(j) << 21) | image;
+    nbr_out[pad + to] = j;
+    d4_out[pad + to] = staged ? st.d4[from] : d4[pad + from];
+  };
+  if (n <= 4 * kWarp) {
+    int* perm = reinterpret_cast<int*>(walks[w].queue);  // (the ring is empty)
+    switch ((n + kWarp - 1) / kWarp) {
+      case 0: break;
+      case 1: order_edges<1, Real>(lane, n, st, rest, perm); break;
+      case 2: order_edges<2, Real>(lane, n, st, rest, perm); break;
+      case 3: order_edges<3, Real>(lane, n, st, rest, perm); break;
+      default: order_edges<4, Real>(lane, n, st, rest, perm);
+    }
+    __syncwarp();
+    for (int q = lane; q < n; q += kWarp) write(q, perm[q]);
+  } else {
+    for (int q = lane; q < n; q += kWarp) {
+      const int mine[1] = {q < Stage::kStage ? st.j[q] : rest[q]};
+      int rank[1];
+      rank_neighbours<1, Real>(n, st, rest, mine, rank);
+      write(rank[0], q);
+    }
   }
 }
 
@@ -1834,8 +1896,10 @@ void Engine::build_edges(int nframes, const int* frame_natoms, const double* cel
       // bins at least r_c / 2 wide (the 5 x 5 x 5 stencil of the fill kernel); widths >= 3 r_c
       // give at least 6 bins per axis, so the periodic stencil never holds a bin twice
       for (int q = 0; q < 3; ++q) fp.nb[q] = std::max(6, std::min(512, static_cast<int>(width[q] / (0.5 * rc))));
-      // FP32 prefilter: |error of r^2| <= 2 r_c |error of d|, with |error of d| bounded by the
-      // rounding of the wrapped fractions (< 2^-24 each, three terms) times the cell row norms
+      // FP32 prefilter: |error of r^2| <= 2 r_c |error of d| near the cutoff; d is the rounded wrapped
+      // position (below the row norms' sum S per component) plus the rounded shift (below 2 S):
+      // |error of d| <= 3^1/2 2^-24 (3 S + r_c) < 3.3e-7 S (the widths give S >= 9 r_c); the band is
+      // more than twice what that and r^2's own rounding need
       double rows = 0;
       for (int q = 0; q < 3; ++q)
         rows += std::sqrt(fp.cell[3 * q] * fp.cell[3 * q] + fp.cell[3 * q + 1] * fp.cell[3 * q + 1] + fp.cell[3 * q + 2] * fp.cell[3 * q + 2]);
@@ -1888,8 +1952,6 @@ void Engine::build_edges(int nframes, const int* frame_natoms, const double* cel
     bin_count_.ensure(sizeof(int) * (bins + 1));
     if (bin_count_.ptr != before) bin_zeroed_ = 0;
   }
-  DevBuf& bin_of = bin_of_;
-  bin_of.ensure(sizeof(int) * std::max(1, a));
   // batches with cell lists only: the binning kernel finds each atom's frame itself
   const bool find_frame = bins && bins_frames_ == nframes;
   if (nframes && !find_frame) {
@@ -1903,19 +1965,17 @@ void Engine::build_edges(int nframes, const int* frame_natoms, const double* cel
     if (bin_zeroed_ < bins + 1) SUS2G_CUDA(cudaMemsetAsync(bin_count_.ptr, 0, sizeof(int) * (bins + 1), s));
     bin_zeroed_ = 0;          // counted into from here on
     bins_used_ = bins + 1;    // cleared again by this step's reverse-edge kernel
-    frac_.ensure(sizeof(AtomFrac) * a);
     off_.ensure(sizeof(AtomOff) * a);
     rec_of_.ensure(sizeof(int) * a);
     const size_t slots = static_cast<size_t>(bins) * bin_cap;
-    bin_rec_.ensure(sizeof(BinAtom) * slots);
+    bin_off_.ensure(sizeof(AtomOff) * slots);
     bin_pos_.ensure(sizeof(BinPos) * slots);
     bin_posf_.ensure(sizeof(BinPosF) * slots);
     // one warp per block: each atom costs ~40 FP64 operations (1/64 of the FP32 rate on this
     // GPU), so small frames are spread over as many SMs as possible (4,096 atoms: 128 SMs)
     k_bin_place<<<(a + kWarp - 1) / kWarp, kWarp, 0, s>>>(plan_.as<FramePlan>(), nframes, find_frame, frame_of_.as<int>(), d_pos, a,
-                                               bin_cap, bin_of.as<int>(), rec_of_.as<int>(), bin_count_.as<int>(),
-                                               frac_.as<AtomFrac>(),
-                                               off_.as<AtomOff>(), bin_rec_.as<BinAtom>(), bin_pos_.as<BinPos>(),
+                                               bin_cap, rec_of_.as<int>(), bin_count_.as<int>(),
+                                               off_.as<AtomOff>(), bin_off_.as<AtomOff>(), bin_pos_.as<BinPos>(),
                                                bin_posf_.as<BinPosF>(), error_.as<int>() + 2, error_.as<int>(), d_types,
                                                model_.C);
     ++launches_;
@@ -1924,11 +1984,9 @@ void Engine::build_edges(int nframes, const int* frame_natoms, const double* cel
   const size_t rsz = precision_ == kFP32 ? sizeof(EdgeF) : sizeof(EdgeD);
   const FramePlan* P = plan_.as<FramePlan>();
   const int* FO = frame_of_.as<int>();
-  const int* BO = bin_of.as<int>();
-  const BinAtom* BR = bin_rec_.as<BinAtom>();
+  const AtomOff* BO = bin_off_.as<AtomOff>();
   const BinPos* BP = bin_pos_.as<BinPos>();
   const BinPosF* BPF = bin_posf_.as<BinPosF>();
-  const AtomFrac* FR = frac_.as<AtomFrac>();
   const AtomOff* OF = off_.as<AtomOff>();
   int* overflow = error_.as<int>() + 1;
   // every periodic batch: the fill kernels (cell lists and image scan) write each centre's edges
@@ -1953,12 +2011,12 @@ void Engine::build_edges(int nframes, const int* frame_natoms, const double* cel
     if (bins) {
       if (precision_ == kFP32)
         SUS2G_CUDA(launch_kernel((pdl_ & kPdlFill) != 0, k_edge_fill_bins<float>, dim3(warp_blocks), dim3(kFillWarps * kWarp), 0, s,
-            P, FO, d_pos, a, rc2, bin_count_.as<int>(), bin_cap, BR, BP, BPF, BO, rec_of_.as<int>(), FR, OF,
+            P, FO, d_pos, a, rc2, bin_count_.as<int>(), bin_cap, BO, BP, BPF, rec_of_.as<int>(), OF,
             counts_.as<int>(), pad_nbr_.as<int>(), pad_d4_.as<EdgeF>(), pad_key_.as<unsigned long long>(), overflow,
             error_.as<int>(), RW, RE, KO, NO, d4_.as<EdgeF>()));
       else
         SUS2G_CUDA(launch_kernel((pdl_ & kPdlFill) != 0, k_edge_fill_bins<double>, dim3(warp_blocks), dim3(kFillWarps * kWarp), 0, s,
-            P, FO, d_pos, a, rc2, bin_count_.as<int>(), bin_cap, BR, BP, BPF, BO, rec_of_.as<int>(), FR, OF,
+            P, FO, d_pos, a, rc2, bin_count_.as<int>(), bin_cap, BO, BP, BPF, rec_of_.as<int>(), OF,
             counts_.as<int>(), pad_nbr_.as<int>(), pad_d4_.as<EdgeD>(), pad_key_.as<unsigned long long>(), overflow,
             error_.as<int>(), RW, RE, KO, NO, d4_.as<EdgeD>()));
       ++launches_;

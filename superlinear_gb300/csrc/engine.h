@@ -282,10 +282,10 @@ class Engine {
   int bin_zeroed_ = 0;          // leading bin counters known to be zero on the device
   int bins_used_ = 0;           // bin counters used by the current cell-list build
   DevBuf posf_;  // double-float positions of image-scan batches (FP32 engines)
-  DevBuf bin_count_, bin_rec_, bin_pos_, bin_posf_, rec_of_;
+  DevBuf bin_count_, bin_off_, bin_pos_, bin_posf_, rec_of_;
   const int* d_types_ = nullptr;
   bool user_edges_ = false;     // caller-supplied edges: no reverse partners, scatter instead of gather
-  DevBuf edge_flag_, hbar_atom_, bin_of_, frac_, off_, in_row_, in_edge_;  // in_*: caller edges grouped by neighbour
+  DevBuf edge_flag_, hbar_atom_, off_, in_row_, in_edge_;  // in_*: caller edges grouped by neighbour
   DevBuf pad_nbr_, pad_d4_, pad_key_;  // padded single-pass staging of cell-list frames
   double cap_scale_ = 2.0;      // padded capacity = cap_scale x mean neighbour count + 64 (grows on overflow)
   double bin_cap_scale_ = 2.0;  // bin capacity = bin_cap_scale x mean atoms per bin + 8 (grows on overflow)

@@ -36,18 +36,15 @@ struct FramePlan {
   float invf[9], reachf[3], rc2f;  // FP32 copies for the image scan's FP32 ranges and bound
 };
 
-// Per-atom wrapped fractional coordinates (FP32, in [0,1)) and the integer cell offsets
-// floor(frac) (FP64 arithmetic), written by the binning kernel for cell-list frames.
-struct AtomFrac { float x, y, z; int pad; };
-struct AtomOff { int x, y, z, pad; };
-// One bin slot (atoms grouped by bin): fractional coordinates, the atom's index and its integer
-// cell offset, so that a candidate is one 32-byte load.
-struct __align__(16) BinAtom { float x, y, z; int j; int ox, oy, oz, pad; };
-// The same slot's exact position wrapped into the home cell, x - floor(frac) . cell (FP64), and the
-// atom's index: the exact test forms x_j + n.cell - x_i as wrapped x_j + ((w + off_i) . cell - x_i),
-// whose second term is one constant per (centre, neighbouring bin).
+// Per-atom integer cell offsets floor(frac) (FP64 arithmetic) and bin coordinates (10 bits each),
+// written by the binning kernel for cell-list frames; the offsets also per bin slot.
+struct __align__(16) AtomOff { int x, y, z, bin; };
+// One bin slot (atoms grouped by bin): the exact position wrapped into the home cell,
+// x - floor(frac) . cell (FP64), and the atom's index: the exact test forms x_j + n.cell - x_i as
+// wrapped x_j + ((w + off_i) . cell - x_i), whose second term is one constant per (centre,
+// neighbouring bin).
 struct __align__(16) BinPos { double x, y, z; int j, pad; };
-// FP32 engines: the wrapped position as double-float parts x = xh + xl (xh = fl32(x)).
+// The wrapped position as double-float parts x = xh + xl (xh = fl32(x)).
 struct __align__(16) BinPosF { float xh, yh, zh; int j; float xl, yl, zl; int pad; };
 
 __device__ __forceinline__ unsigned long long edge_key(int j, int n0, int n1, int n2) {
@@ -59,28 +56,24 @@ __device__ __forceinline__ unsigned long long edge_key(int j, int n0, int n1, in
 
 // Cell-list frames, one warp per centre i.  Bins are at least r_c / 2 wide, so every neighbour lies
 // in the 5 x 5 x 5 bins around the centre's bin (about 2.3x fewer candidates than 27 bins of width
-// r_c).  Each lane owns four of those 125 bins and walks their atoms, two candidates per
-// iteration (independent loads in flight); candidates that pass the FP32 prefilter are appended
-// to a per-warp queue in shared memory (`queue`, 128 entries) and whenever 32 are queued the warp
-// tests a full warp of them:
+// r_c).  Each lane owns four of those 125 bins and walks them two at a time (independent loads in
+// flight): a candidate is one 16-byte load, and the FP32 prefilter adds the bin's wrap shift to the
+// wrapped position's leading part.  Candidates that pass are appended to a per-warp ring in shared
+// memory and whenever 32 are queued the warp tests a full warp of them:
 //   * FP64 engines: x_j + n.cell - x_i and r^2 in FP64;
 //   * FP32 engines: the same vector from double-float (hi, lo) parts in FP32 arithmetic, with the
 //     FP64 test only for the rare entries whose FP32 r^2 lies within 1e-4 relative of r_c^2
 //     (FP64 runs at 1/64 of the FP32 rate on this GPU).
 // Either way the accepted set is exactly {r^2 < r_c^2} in FP64.  The vector's periodic part
-// depends only on the wrap w in {-1, 0, 1}^3 of the neighbouring bin: lane k < 27 holds the shift
-// (w_k + off_i) . cell - x_i of wrap k.  Accepted edges of each round are reported through
-// Round(mask, lane_accepted, j, n0, n1, n2, x, y, z, r) (Real components and distance), so the
+// depends only on the wrap w in {-1, 0, 1}^3 of the neighbouring bin: entry k < 27 of the shift
+// table holds (w_k + off_i) . cell - x_i.  Accepted edges of each round are reported through
+// Round(mask, lane_accepted, j, packed image, x, y, z, r) (Real components and distance), so the
 // caller can count or write them with one ballot per round.
-constexpr int kEdgeQueue = 128;
+constexpr int kEdgeQueue = 128;                    // ring entries: at most 31 + 64 are waiting
 constexpr int kBinReach = 2;                       // bins on each side of the centre's bin
 constexpr int kBinSpan = 2 * kBinReach + 1;        // 5
 constexpr int kBinStencil = kBinSpan * kBinSpan * kBinSpan;  // 125
 constexpr int kBinsPerLane = 4;                    // 32 x 4 >= 125
-__device__ __forceinline__ int pack_image(int n0, int n1, int n2) {
-  return ((n0 + 64) << 14) | ((n1 + 64) << 7) | (n2 + 64);
-}
-
 // double-float sum (ah + al) + (bh + bl), rounded to FP32 (two-sum of the high parts)
 __device__ __forceinline__ float df_add(float ah, float al, float bh, float bl) {
   const float s = ah + bh;
@@ -106,52 +99,45 @@ __device__ __forceinline__ void df_acc_mul(float& h, float& l, float m, float ch
   df_acc(h, l, p, fmaf(m, cl, pe));
 }
 
-// Per-warp shared tables of the fill: the 27 wrap shifts (FP64 and double-float parts) and the
-// lanes' bins (start, length).
-// Per wrap w in {-1, 0, 1}^3 of a neighbouring bin (index (w0 + 1) 9 + (w1 + 1) 3 + (w2 + 1)):
-// the exact shift (w + off_i) . cell - x_i in FP64 and as double-float parts, the image base
-// w + off_i and the FP32 fractional shift w - frac_i of the prefilter.
-struct __align__(16) WrapShift {
-  double x, y, z;
-  float hx, hy, hz, lx, ly, lz;
-  int4 nb;      // (w0 + off_i.x, w1 + off_i.y, w2 + off_i.z, -)
-  float4 df;    // (w0 - frac_i.x, w1 - frac_i.y, w2 - frac_i.z, -)
-};
-struct BinWalk {
-  WrapShift shift[27];
+// Per-warp shared tables of the fill.  Per wrap w in {-1, 0, 1}^3 of a neighbouring bin (index
+// (w0 + 1) 9 + (w1 + 1) 3 + (w2 + 1)) the exact shift (w + off_i) . cell - x_i: its leading FP32
+// part, and the trailing part (FP32 engines) or the FP64 value.  The ring: (bin slot, wrap index |
+// (w0 + 1) << 5 | (w1 + 1) << 7 | (w2 + 1) << 9).
+template <typename Real> struct BinWalk {
+  float4 hi[27];
+  typename Vec4<Real>::type lo[27];
+  int2 queue[kEdgeQueue];
 };
 
 template <typename Real, typename Round>
 __device__ __forceinline__ void warp_bin_edges(int i, const FramePlan& fp, const double* pos, double rc2,
-                                               const int* bin_count, int bin_cap, const BinAtom* bin_rec,
-                                               const BinPos* bin_pos,
-                                               const BinPosF* bin_posf, const int* bin_of, const int* rec_of,
-                                               const AtomFrac* frac, const AtomOff* off, int* error, int2* queue,
-                                               BinWalk& walk, Round&& round) {
+                                               const int* bin_count, int bin_cap, const AtomOff* bin_off,
+                                               const BinPos* bin_pos, const BinPosF* bin_posf, const int* rec_of,
+                                               const AtomOff* off, int* error, BinWalk<Real>& walk, Round&& round) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
-  const int local = bin_of[i] - fp.bin0;
-  const int bi0 = local / (fp.nb[1] * fp.nb[2]), bi1 = (local / fp.nb[2]) % fp.nb[1], bi2 = local % fp.nb[2];
-  const AtomFrac fi = frac[i];
   const AtomOff oi = off[i];
+  const int bi0 = oi.bin >> 20, bi1 = (oi.bin >> 10) & 1023, bi2 = oi.bin & 1023;
   const double* c = fp.cell;
-  const float* cf = fp.cellf;
-  const int self_rec = rec_of[i];  // the centre's own bin record
-  // lane k < 27: wrap k = (w0 + 1) 9 + (w1 + 1) 3 + (w2 + 1).  Its shift (w + off_i) . cell - x_i =
-  // w . cell - (x_i wrapped into the home cell): FP64 engines in FP64; FP32 engines as double-float
-  // parts from the cell's and the centre record's (hi, lo) parts in FP32 arithmetic (their exact
-  // FP64 shift is formed only for the rare entries near the cutoff)
+  const int self_rec = rec_of[i];  // the centre's own bin slot
+  // lane k < 27: wrap k.  Its shift (w + off_i) . cell - x_i = w . cell - (x_i wrapped into the home
+  // cell): FP64 engines in FP64; FP32 engines as double-float parts from the cell's and the centre
+  // slot's (hi, lo) parts in FP32 arithmetic (their exact FP64 shift is formed only for the rare
+  // entries near the cutoff)
   if (lane < 27) {
     const int w0 = lane / 9 - 1, w1 = (lane / 3) % 3 - 1, w2 = lane % 3 - 1;
-    WrapShift w;
+    typename Vec4<Real>::type lo;
+    float4 hi;
+    lo.w = 0;
     if constexpr (sizeof(Real) == 8) {
       const double a0 = w0 + oi.x, a1 = w1 + oi.y, a2 = w2 + oi.z;
-      w.x = a0 * c[0] + a1 * c[3] + a2 * c[6] - pos[3 * i];
-      w.y = a0 * c[1] + a1 * c[4] + a2 * c[7] - pos[3 * i + 1];
-      w.z = a0 * c[2] + a1 * c[5] + a2 * c[8] - pos[3 * i + 2];
-      w.hx = w.hy = w.hz = w.lx = w.ly = w.lz = 0.f;
+      lo.x = a0 * c[0] + a1 * c[3] + a2 * c[6] - pos[3 * i];
+      lo.y = a0 * c[1] + a1 * c[4] + a2 * c[7] - pos[3 * i + 1];
+      lo.z = a0 * c[2] + a1 * c[5] + a2 * c[8] - pos[3 * i + 2];
+      hi = make_float4(static_cast<float>(lo.x), static_cast<float>(lo.y), static_cast<float>(lo.z), 0.f);
     } else {
       const BinPosF me = bin_posf[self_rec];
+      const float* cf = fp.cellf;
       const float* cl = fp.celll;
       float h[3], l[3];
 #pragma unroll
@@ -165,99 +151,60 @@ __device__ __forceinline__ void warp_bin_edges(int i, const FramePlan& fp, const
           const float th = static_cast<float>(wq[r]) * cf[3 * r + q], tl = static_cast<float>(wq[r]) * cl[3 * r + q];
           const float s2 = sh + th, v = s2 - sh;
           const float e = (sh - (s2 - v)) + (th - v);
-          const float lo = e + (sl + tl);
-          sh = s2 + lo;
-          sl = lo - (sh - s2);
+          const float rest = e + (sl + tl);
+          sh = s2 + rest;
+          sl = rest - (sh - s2);
         }
         h[q] = sh;
         l[q] = sl;
       }
-      w.x = w.y = w.z = 0.0;
-      w.hx = h[0]; w.hy = h[1]; w.hz = h[2];
-      w.lx = l[0]; w.ly = l[1]; w.lz = l[2];
+      hi = make_float4(h[0], h[1], h[2], 0.f);
+      lo.x = l[0]; lo.y = l[1]; lo.z = l[2];
     }
-    w.nb = make_int4(w0 + oi.x, w1 + oi.y, w2 + oi.z, 0);
-    w.df = make_float4(static_cast<float>(w0) - fi.x, static_cast<float>(w1) - fi.y, static_cast<float>(w2) - fi.z, 0.f);
-    walk.shift[lane] = w;
+    walk.hi[lane] = hi;
+    walk.lo[lane] = lo;
   }
-  // the lane's bins (stencil slots 4 lane + u) laid end to end: record offset start_u - excl_u,
-  // exclusive ends excl_1..3 and the wraps packed 5 bits each
-  int off0 = 0, off1 = 0, off2 = 0, off3 = 0, ex1 = 0, ex2 = 0, ex3 = 0, kpack = 0, mine = 0;
-#pragma unroll
-  for (int u = 0; u < kBinsPerLane; ++u) {
-    const int sl = kBinsPerLane * lane + u;
-    int bstart = 0, blen = 0, wk = 13;
-    if (sl < kBinStencil) {
-      const int raw0 = bi0 + sl / (kBinSpan * kBinSpan) - kBinReach;
-      const int raw1 = bi1 + (sl / kBinSpan) % kBinSpan - kBinReach;
-      const int raw2 = bi2 + sl % kBinSpan - kBinReach;
-      const int w0 = raw0 < 0 ? -1 : (raw0 >= fp.nb[0] ? 1 : 0);
-      const int w1 = raw1 < 0 ? -1 : (raw1 >= fp.nb[1] ? 1 : 0);
-      const int w2 = raw2 < 0 ? -1 : (raw2 >= fp.nb[2] ? 1 : 0);
-      const int bin = fp.bin0 + ((raw0 - w0 * fp.nb[0]) * fp.nb[1] + (raw1 - w1 * fp.nb[1])) * fp.nb[2] +
-                      (raw2 - w2 * fp.nb[2]);
-      bstart = bin * bin_cap;
-      blen = min(bin_count[bin], bin_cap);
-      wk = (w0 + 1) * 9 + (w1 + 1) * 3 + (w2 + 1);
-    }
-    const int o = bstart - mine;
-    if (u == 0) off0 = o;
-    if (u == 1) { off1 = o; ex1 = mine; }
-    if (u == 2) { off2 = o; ex2 = mine; }
-    if (u == 3) { off3 = o; ex3 = mine; }
-    kpack |= wk << (5 * u);
-    mine += blen;
-  }
-  int most = mine;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-  // the FP32 cell rows of the prefilter, in registers
-  float cr[9];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) cr[q] = cf[q];
   __syncwarp();
   const float screen = fp.screen2, lo2 = fp.lo2, hi2 = fp.hi2;
-  int queued = 0;  // warp-uniform
-  // test of queue entries [0, n) (one per lane) and the round callback
-  // queue entry: (bin record index, packed image | wrap index k << 21)
+  int head = 0, tail = 0;  // warp-uniform ring positions
+  // test of the ring's first n entries (one per lane) and the round callback
   auto drain = [&](int n) {
     bool ok = false;
-    int j = 0, n0 = 0, n1 = 0, n2 = 0, k = 0;
-    int2 q = make_int2(0, 0);
+    int j = 0, image = 0;
+    Real vx = 0, vy = 0, vz = 0, r2 = 0;
     if (lane < n) {
-      q = queue[lane];
-      k = q.y >> 21;
-      n0 = ((q.y >> 14) & 127) - 64; n1 = ((q.y >> 7) & 127) - 64; n2 = (q.y & 127) - 64;
-    }
-    if constexpr (sizeof(Real) == 8) {
-      double vx = 0, vy = 0, vz = 0, r2 = 0;
-      if (lane < n) {
+      const int2 q = walk.queue[(head + lane) & (kEdgeQueue - 1)];
+      const int k = q.y & 31;
+      const AtomOff oj = bin_off[q.x];
+      const int n0 = ((q.y >> 5) & 3) - 1 + oi.x - oj.x, n1 = ((q.y >> 7) & 3) - 1 + oi.y - oj.y,
+                n2 = ((q.y >> 9) & 3) - 1 + oi.z - oj.z;
+      image = ((n0 + 64) << 14) | ((n1 + 64) << 7) | (n2 + 64);
+      const bool self = q.x == self_rec && k == 13;
+      const bool packable = (((n0 + 64) | (n1 + 64) | (n2 + 64)) & ~127) == 0;
+      if (!packable) record_error(error, kErrImageRange);
+      if constexpr (sizeof(Real) == 8) {
         const BinPos bp = bin_pos[q.x];
-        const WrapShift& w = walk.shift[k];
+        const auto w = walk.lo[k];
         j = bp.j;
         vx = bp.x + w.x;
         vy = bp.y + w.y;
         vz = bp.z + w.z;
         r2 = vx * vx + vy * vy + vz * vz;
         ok = r2 < rc2;
-      }
-      const unsigned mask = __ballot_sync(0xffffffffu, ok);
-      round(mask, ok, j, n0, n1, n2, Real(vx), Real(vy), Real(vz), Real(sqrt(r2)));
-    } else {
-      float vx = 0, vy = 0, vz = 0, r2 = 0;
-      if (lane < n) {
+      } else {
         const BinPosF bp = bin_posf[q.x];
-        const WrapShift& w = walk.shift[k];
+        const float4 h = walk.hi[k];
+        const EdgeF l = walk.lo[k];
         j = bp.j;
-        vx = df_add(bp.xh, bp.xl, w.hx, w.lx);
-        vy = df_add(bp.yh, bp.yl, w.hy, w.ly);
-        vz = df_add(bp.zh, bp.zl, w.hz, w.lz);
+        vx = df_add(bp.xh, bp.xl, h.x, l.x);
+        vy = df_add(bp.yh, bp.yl, h.y, l.y);
+        vz = df_add(bp.zh, bp.zl, h.z, l.z);
         r2 = vx * vx + vy * vy + vz * vz;
         ok = r2 < lo2;
         if (!ok && r2 < hi2) {
           // near the cutoff: the FP64 test decides, x_j + (w + off_i) . cell - x_i in FP64
           const BinPos bd = bin_pos[q.x];
-          const double a0 = k / 9 - 1 + oi.x, a1 = (k / 3) % 3 - 1 + oi.y, a2 = k % 3 - 1 + oi.z;
+          const double a0 = n0 + oj.x, a1 = n1 + oj.y, a2 = n2 + oj.z;
           const double dx = bd.x + (a0 * c[0] + a1 * c[3] + a2 * c[6] - pos[3 * i]);
           const double dy = bd.y + (a0 * c[1] + a1 * c[4] + a2 * c[7] - pos[3 * i + 1]);
           const double dz = bd.z + (a0 * c[2] + a1 * c[5] + a2 * c[8] - pos[3 * i + 2]);
@@ -267,63 +214,59 @@ __device__ __forceinline__ void warp_bin_edges(int i, const FramePlan& fp, const
           r2 = static_cast<float>(d2);
         }
       }
-      const unsigned mask = __ballot_sync(0xffffffffu, ok);
-      round(mask, ok, j, n0, n1, n2, vx, vy, vz, sqrtf(r2));
+      ok = ok && !self && packable;
     }
+    head += n;
+    const unsigned mask = __ballot_sync(0xffffffffu, ok);
+    if constexpr (sizeof(Real) == 8) round(mask, ok, j, image, vx, vy, vz, sqrt(r2));
+    else round(mask, ok, j, image, vx, vy, vz, sqrtf(r2));
   };
-  // FP32 prefilter of the lane's candidate t (0 <= t < mine, else -1): packed image with the wrap
-  // index, and the bin record index
-  auto screen_candidate = [&](int t, int& rec_index) -> int {
-    if (t >= mine) return -1;
-    const int u1 = t >= ex1, u2 = t >= ex2, u3 = t >= ex3;
-    rec_index = t + (u3 ? off3 : (u2 ? off2 : (u1 ? off1 : off0)));
-    const int k = (kpack >> (5 * (u1 + u2 + u3))) & 31;
-    const BinAtom rec = bin_rec[rec_index];
-    const float4 df = walk.shift[k].df;
-    const float sx32 = rec.x + df.x, sy32 = rec.y + df.y, sz32 = rec.z + df.z;
-    const float fx = sx32 * cr[0] + sy32 * cr[3] + sz32 * cr[6];
-    const float fy = sx32 * cr[1] + sy32 * cr[4] + sz32 * cr[7];
-    const float fz = sx32 * cr[2] + sy32 * cr[5] + sz32 * cr[8];
-    if (fx * fx + fy * fy + fz * fz >= screen) return -1;
-    const int4 nb = walk.shift[k].nb;
-    const int n0 = nb.x - rec.ox, n1 = nb.y - rec.oy, n2 = nb.z - rec.oz;
-    if (i == rec.j && n0 == 0 && n1 == 0 && n2 == 0) return -1;
-    if (n0 < -64 || n0 > 63 || n1 < -64 || n1 > 63 || n2 < -64 || n2 > 63) {
-      record_error(error, kErrImageRange);
-      return -1;
+  // prefilter of slot `rec` of a bin with shift h, and its place in the ring
+  auto screen_candidate = [&](bool have, int rec, const float4& h, int wrap) {
+    bool pass = false;
+    if (have) {
+      const float4 p = *reinterpret_cast<const float4*>(bin_posf + rec);
+      const float x = p.x + h.x, y = p.y + h.y, z = p.z + h.z;
+      pass = x * x + y * y + z * z < screen;
     }
-    return pack_image(n0, n1, n2) | (k << 21);
+    const unsigned m = __ballot_sync(0xffffffffu, pass);
+    if (pass) walk.queue[(tail + __popc(m & below)) & (kEdgeQueue - 1)] = make_int2(rec, wrap);
+    tail += __popc(m);
   };
-  auto push = [&](int packed, int rec_index) {
-    const bool pre = packed >= 0;
-    const unsigned m = __ballot_sync(0xffffffffu, pre);
-    if (pre) queue[queued + __popc(m & below)] = make_int2(rec_index, packed);
-    queued += __popc(m);
-  };
-  // two candidates per lane per iteration (their loads overlap)
-  for (int t = 0; t < most; t += 2) {
-    int ra = 0, rb = 0;
-    const int pa = screen_candidate(t, ra);
-    const int pb = screen_candidate(t + 1, rb);
-    push(pa, ra);
-    push(pb, rb);
-    __syncwarp();
-    while (queued >= 32) {
-      drain(32);
-      __syncwarp();
-      // move the remainder (< 96 entries) to the front, 32 at a time in order
-      for (int q0 = 32; q0 < queued; q0 += 32) {
-        int2 rest = make_int2(0, 0);
-        const bool have = q0 + lane < queued;
-        if (have) rest = queue[q0 + lane];
-        __syncwarp();
-        if (have) queue[q0 - 32 + lane] = rest;
-        __syncwarp();
+#pragma unroll 1
+  for (int u = 0; u < kBinsPerLane; u += 2) {
+    int first[2], len[2], wrap[2];
+    float4 h[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const int sl = kBinsPerLane * lane + u + p;
+      first[p] = 0; len[p] = 0; wrap[p] = 13;
+      if (sl < kBinStencil) {
+        int w[3], at[3] = {bi0 + sl / (kBinSpan * kBinSpan) - kBinReach, bi1 + (sl / kBinSpan) % kBinSpan - kBinReach,
+                           bi2 + sl % kBinSpan - kBinReach};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          w[q] = 1;
+          if (at[q] < 0) { w[q] = 0; at[q] += fp.nb[q]; }
+          else if (at[q] >= fp.nb[q]) { w[q] = 2; at[q] -= fp.nb[q]; }
+        }
+        const int bin = fp.bin0 + (at[0] * fp.nb[1] + at[1]) * fp.nb[2] + at[2];
+        first[p] = bin * bin_cap;
+        len[p] = min(bin_count[bin], bin_cap);
+        wrap[p] = (w[0] * 9 + w[1] * 3 + w[2]) | (w[0] << 5) | (w[1] << 7) | (w[2] << 9);
       }
-      queued -= 32;
+      h[p] = walk.hi[wrap[p] & 31];
+    }
+    const int most = __reduce_max_sync(0xffffffffu, max(len[0], len[1]));
+    for (int t = 0; t < most; ++t) {
+      screen_candidate(t < len[0], first[0] + t, h[0], wrap[0]);
+      screen_candidate(t < len[1], first[1] + t, h[1], wrap[1]);
+      __syncwarp();
+      while (tail - head >= 32) drain(32);
+      __syncwarp();  // the ring's read entries may be overwritten
     }
   }
-  if (queued > 0) drain(queued);
+  if (tail > head) drain(tail - head);
   __syncwarp();
 }
 
