@@ -4,13 +4,18 @@
 // Real Y_lm.  Same convention as the reference engine (interfaces/lammps/ML-SUS2/sus2_sl_kernel.cpp:
 // 12-42: orthonormal, Condon-Shortley phase folded so that Y_l,+m ~ +Re (x+iy)^m, index
 // h = l*l + l + m).  Formulated here on the unit vector u = d/r:
-//     Y_l,0  = N_l0 Pi_l0(u_z)
-//     Y_l,+m = sqrt(2) N_lm Pi_lm(u_z) Re (u_x + i u_y)^m,   Y_l,-m = ... Im (u_x + i u_y)^m
-// where Pi_mm = (2m-1)!!, Pi_m+1,m = (2m+1) u_z Pi_mm and
-//     Pi_lm = ((2l-1) u_z Pi_l-1,m - (l+m-1) Pi_l-2,m) / (l-m)
-// is the associated-Legendre recurrence with |u| = 1 substituted, and
-// N_lm = sqrt((2l+1)/(4 pi) (l-m)!/(l+m)!).  The gradient with respect to d only needs tangential
-// derivatives, so any smooth extension Yhat(u) off the sphere gives
+//     Y_l,0  = f_l0(u_z)
+//     Y_l,+m = f_lm(u_z) Re (u_x + i u_y)^m,   Y_l,-m = f_lm(u_z) Im (u_x + i u_y)^m
+// where f_lm = N_lm Pi_lm (times sqrt(2) for m > 0), N_lm = sqrt((2l+1)/(4 pi) (l-m)!/(l+m)!),
+// Pi_mm = (2m-1)!! and Pi_lm = ((2l-1) u_z Pi_l-1,m - (l+m-1) Pi_l-2,m) / (l-m) (the
+// associated-Legendre recurrence with |u| = 1 substituted).  The normalisation is folded into the
+// coefficients at compile time; up to l = m + 3 f_lm is its polynomial in u_z, above it the
+// recurrence.  Sums over l come before the products with (u_x + i u_y)^m.  Every pass evaluates
+// these per edge and is bound by its instructions (FP64: by the FP64 pipe); terms times constant
+// zeros and ones, which the compiler has to keep, are left out (with the virial's halving sums: adjoint
+// of Static L3/K4/O2, 32,768 atoms, 138.5 -> 129.1 us; gate reverse of Effect L4/K8/R2/O3, 8,000
+// atoms, 112.5 -> 104.6 us).  The gradient with respect to d
+// only needs tangential derivatives, so any smooth extension Yhat(u) off the sphere gives
 //     dY/dd = (1/r) (I - u u^T) grad_u Yhat(u),
 // which the reverse and tangent helpers below use with the polynomial extension above.
 //
@@ -21,139 +26,141 @@
 // l > 0 functions use angular_max_dist (RB_CalcForCutoff, sus2_sl_radial_math.cpp:296-336).
 #pragma once
 #include <cmath>
+#include <type_traits>
+#include <utility>
 
 #include "device_common.cuh"
 
 namespace sus2g {
 
-// N_lm (times sqrt 2 for m > 0), index l*l + l + m for m >= 0, in FP64 and rounded to FP32 (the
-// FP32 form reads its own table: converting the FP64 entries at run time would occupy the FP64
-// pipe, 1/64 of the FP32 rate on this GPU).  Each translation unit that includes this header owns
-// a copy and fills it once per device through sph_norm_upload().
-static __constant__ double c_sph_norm[64];
-static __constant__ float c_sph_norm_f[64];
-
-static inline cudaError_t sph_norm_upload() {
-  double n[64] = {0};
-  float nf[64] = {0};
-  const double pi = 3.14159265358979323846;
-  for (int l = 0; l <= 6; ++l)
-    for (int m = 0; m <= l; ++m) {
-      double ratio = 1.0;
-      for (int a = l - m + 1; a <= l + m; ++a) ratio /= a;
-      n[l * l + l + m] = std::sqrt((2 * l + 1) * ratio / (4 * pi)) * (m ? std::sqrt(2.0) : 1.0);
-    }
-  for (int q = 0; q < 64; ++q) nf[q] = static_cast<float>(n[q]);
-  cudaError_t err = cudaMemcpyToSymbol(c_sph_norm, n, sizeof(n));
-  if (err != cudaSuccess) return err;
-  return cudaMemcpyToSymbol(c_sph_norm_f, nf, sizeof(nf));
-}
-
-template <int L> struct Sph { static constexpr int Lp = L + 1, H = Lp * Lp; };
-
 __host__ __device__ constexpr int sh_index(int l, int m) { return l * l + l + m; }
 
-// (2m-1)!! and 1/n as literals of type T: with the unrolled (l, m) loops the argument is a
-// compile-time value and these fold to immediates (a constexpr double recursion would be
-// evaluated at run time in FP64).
-template <typename T>
-__device__ __forceinline__ T sph_dfact(int m) {
-  switch (m) {
-    case 0: case 1: return T(1);
-    case 2: return T(3);
-    case 3: return T(15);
-    case 4: return T(105);
-    case 5: return T(945);
-    case 6: return T(10395);
-    default: return T(135135);
-  }
+// sqrt by Newton's method (from above, until it stops falling), for constants only
+__host__ __device__ constexpr double const_sqrt(double x) {
+  double r = x > 1.0 ? x : 1.0;
+  for (double n = 0.5 * (r + x / r); n < r; n = 0.5 * (r + x / r)) r = n;
+  return r;
 }
-template <typename T>
-__device__ __forceinline__ T sph_inv(int n) {
-  switch (n) {
-    case 1: return T(1);
-    case 2: return T(0.5);
-    case 3: return T(0.33333333333333333333);
-    case 4: return T(0.25);
-    case 5: return T(0.2);
-    case 6: return T(0.16666666666666666667);
-    default: return T(0.14285714285714285714);
+// N_lm, times sqrt(2) for m > 0, times (2m-1)!!
+__host__ __device__ constexpr double sph_norm(int l, int m) {
+  double ratio = 1.0, dfact = 1.0;
+  for (int a = l - m + 1; a <= l + m; ++a) ratio /= a;
+  for (int a = 3; a <= 2 * m - 1; a += 2) dfact *= a;
+  return const_sqrt((2 * l + 1) * ratio / (4 * 3.14159265358979323846) * (m ? 2.0 : 1.0)) * dfact;
+}
+
+// f(A), f(A + 1) .. f(N - 1) with the index as a compile-time constant.
+template <int A, int N, typename Fn>
+__device__ __forceinline__ void unroll(Fn&& fn) {
+  if constexpr (A < N) {
+    fn(std::integral_constant<int, A>{});
+    unroll<A + 1, N>(fn);
   }
 }
 
-template <typename T> __device__ __forceinline__ T norm_lm(int idx) { return T(c_sph_norm[idx]); }
-template <> __device__ __forceinline__ float norm_lm<float>(int idx) { return c_sph_norm_f[idx]; }
+// f_lm(z) for l = m .. L into f[l - m], and df_lm/dz into d[l - m] (DERIV).
+template <int L, int m, bool DERIV, typename T>
+__device__ __forceinline__ void legendre_column(T z, T z2, T* f, T* d) {
+  unroll<m, L + 1>([&](auto lc) {
+    constexpr int l = decltype(lc)::value, q = l - m;
+    constexpr double n = sph_norm(l, m);
+    if constexpr (q == 0) {
+      f[0] = T(n);
+      if (DERIV) d[0] = T(0);
+    } else if constexpr (q == 1) {
+      constexpr double c = n * (2 * m + 1);
+      f[1] = T(c) * z;
+      if (DERIV) d[1] = T(c);
+    } else if constexpr (q == 2) {
+      constexpr double c = n * (2 * m + 1) / 2, a = c * (2 * m + 3), a2 = 2 * a;
+      f[2] = T(a) * z2 - T(c);
+      if (DERIV) d[2] = T(a2) * z;
+    } else if constexpr (q == 3) {
+      constexpr double b = n * (2 * m + 1) * (2 * m + 3) / 6, a = b * (2 * m + 5), a3 = 3 * a, b3 = 3 * b;
+      f[3] = z * (T(a) * z2 - T(b3));
+      if (DERIV) d[3] = T(a3) * z2 - T(b3);
+    } else {
+      constexpr double a = n / sph_norm(l - 1, m) * (2 * l - 1) / q, b = n / sph_norm(l - 2, m) * (l + m - 1) / q;
+      f[q] = T(a) * z * f[q - 1] - T(b) * f[q - 2];
+      if (DERIV) d[q] = T(a) * (z * d[q - 1] + f[q - 1]) - T(b) * d[q - 2];
+    }
+  });
+}
+
+// (u_x + i u_y)^m for m = 0 .. L
+template <int L, typename T>
+__device__ __forceinline__ void azimuth_powers(T ux, T uy, T* Cm, T* Sm) {
+  Cm[0] = T(1); Sm[0] = T(0);
+  if (L >= 1) { Cm[1] = ux; Sm[1] = uy; }
+#pragma unroll
+  for (int m = 2; m <= L; ++m) {
+    Cm[m] = ux * Cm[m - 1] - uy * Sm[m - 1];
+    Sm[m] = ux * Sm[m - 1] + uy * Cm[m - 1];
+  }
+}
 
 // Values Y[h] for h < (L+1)^2 at unit vector (ux, uy, uz).
 template <int L, typename T>
 __device__ __forceinline__ void sph_values(T ux, T uy, T uz, T* Y) {
   T Cm[L + 1], Sm[L + 1];
-  Cm[0] = T(1); Sm[0] = T(0);
-#pragma unroll
-  for (int m = 1; m <= L; ++m) {
-    Cm[m] = ux * Cm[m - 1] - uy * Sm[m - 1];
-    Sm[m] = ux * Sm[m - 1] + uy * Cm[m - 1];
-  }
-#pragma unroll
-  for (int m = 0; m <= L; ++m) {
-    T p2 = T(0), p1 = T(0), p0 = sph_dfact<T>(m);
+  azimuth_powers<L>(ux, uy, Cm, Sm);
+  const T z2 = uz * uz;
+  unroll<0, L + 1>([&](auto mc) {
+    constexpr int m = decltype(mc)::value;
+    T f[L + 1 - m];
+    legendre_column<L, m, false, T>(uz, z2, f, nullptr);
 #pragma unroll
     for (int l = m; l <= L; ++l) {
-      T p;
-      if (l == m) p = p0;
-      else if (l == m + 1) p = T(2 * m + 1) * uz * p0;
-      else p = (T(2 * l - 1) * uz * p1 - T(l + m - 1) * p2) * sph_inv<T>(l - m);
-      if (l == m) { p1 = p; }
-      else { p2 = p1; p1 = p; }
-      const T n = norm_lm<T>(sh_index(l, m)) * p;
       if (m == 0) {
-        Y[sh_index(l, 0)] = n;
+        Y[sh_index(l, 0)] = f[l];
       } else {
-        Y[sh_index(l, m)] = n * Cm[m];
-        Y[sh_index(l, -m)] = n * Sm[m];
+        Y[sh_index(l, m)] = f[l - m] * Cm[m];
+        Y[sh_index(l, -m)] = f[l - m] * Sm[m];
       }
     }
-  }
+  });
 }
 
 // grad_u of sum_h P[h] Yhat_h(u) (polynomial extension), accumulated into (gx, gy, gz).
 template <int L, typename T>
 __device__ __forceinline__ void sph_grad_dot(T ux, T uy, T uz, const T* P, T& gx, T& gy, T& gz) {
   T Cm[L + 1], Sm[L + 1];
-  Cm[0] = T(1); Sm[0] = T(0);
+  azimuth_powers<L>(ux, uy, Cm, Sm);
+  const T z2 = uz * uz;
+  unroll<0, L + 1>([&](auto mc) {
+    constexpr int m = decltype(mc)::value;
+    T f[L + 1 - m], d[L + 1 - m];
+    legendre_column<L, m, true, T>(uz, z2, f, d);
+    if constexpr (m == 0) {
 #pragma unroll
-  for (int m = 1; m <= L; ++m) {
-    Cm[m] = ux * Cm[m - 1] - uy * Sm[m - 1];
-    Sm[m] = ux * Sm[m - 1] + uy * Cm[m - 1];
-  }
+      for (int l = 1; l <= L; ++l) gz += P[sh_index(l, 0)] * d[l];
+    } else {
+      // sums over l, then d/dux (C_m, S_m) = m (C_m-1, S_m-1), d/duy (C_m, S_m) = m (-S_m-1, C_m-1)
+      T fc = f[0] * P[sh_index(m, m)], fs = f[0] * P[sh_index(m, -m)], dc = T(0), ds = T(0);
 #pragma unroll
-  for (int m = 0; m <= L; ++m) {
-    const T pmm = sph_dfact<T>(m);
-    T p1 = T(0), p2 = T(0), d1 = T(0), d2 = T(0);
-#pragma unroll
-    for (int l = m; l <= L; ++l) {
-      T p, d;
-      if (l == m) { p = pmm; d = T(0); }
-      else if (l == m + 1) { p = T(2 * m + 1) * uz * pmm; d = T(2 * m + 1) * pmm; }
-      else {
-        const T inv = sph_inv<T>(l - m);
-        p = (T(2 * l - 1) * uz * p1 - T(l + m - 1) * p2) * inv;
-        d = (T(2 * l - 1) * (p1 + uz * d1) - T(l + m - 1) * d2) * inv;
+      for (int l = m + 1; l <= L; ++l) {
+        fc += f[l - m] * P[sh_index(l, m)];
+        fs += f[l - m] * P[sh_index(l, -m)];
+        if (l == m + 1) {
+          dc = d[1] * P[sh_index(l, m)];
+          ds = d[1] * P[sh_index(l, -m)];
+        } else {
+          dc += d[l - m] * P[sh_index(l, m)];
+          ds += d[l - m] * P[sh_index(l, -m)];
+        }
       }
-      p2 = p1; p1 = p; d2 = d1; d1 = d;
-      const T n = norm_lm<T>(sh_index(l, m));
-      if (m == 0) {
-        gz += P[sh_index(l, 0)] * n * d;
+      if constexpr (m == 1) {
+        gx += fc;
+        gy += fs;
       } else {
-        const T pc = P[sh_index(l, m)] * n, ps = P[sh_index(l, -m)] * n;
-        const T mf = T(m);
-        // d/dux (Cm, Sm) = m (C_m-1, S_m-1); d/duy (Cm, Sm) = m (-S_m-1, C_m-1)
-        gx += p * mf * (pc * Cm[m - 1] + ps * Sm[m - 1]);
-        gy += p * mf * (ps * Cm[m - 1] - pc * Sm[m - 1]);
-        gz += d * (pc * Cm[m] + ps * Sm[m]);
+        fc *= T(m);
+        fs *= T(m);
+        gx += fc * Cm[m - 1] + fs * Sm[m - 1];
+        gy += fs * Cm[m - 1] - fc * Sm[m - 1];
       }
+      if constexpr (m < L) gz += dc * Cm[m] + ds * Sm[m];
     }
-  }
+  });
 }
 
 // Tangent of Yhat along a tangential direction t (already projected, divided by r):
@@ -161,37 +168,30 @@ __device__ __forceinline__ void sph_grad_dot(T ux, T uy, T uz, const T* P, T& gx
 template <int L, typename T>
 __device__ __forceinline__ void sph_tangent(T ux, T uy, T uz, T tx, T ty, T tz, T* Ydot) {
   T Cm[L + 1], Sm[L + 1];
-  Cm[0] = T(1); Sm[0] = T(0);
+  azimuth_powers<L>(ux, uy, Cm, Sm);
+  const T z2 = uz * uz;
+  unroll<0, L + 1>([&](auto mc) {
+    constexpr int m = decltype(mc)::value;
+    T f[L + 1 - m], d[L + 1 - m];
+    legendre_column<L, m, true, T>(uz, z2, f, d);
+    if constexpr (m == 0) {
+      Ydot[0] = T(0);
 #pragma unroll
-  for (int m = 1; m <= L; ++m) {
-    Cm[m] = ux * Cm[m - 1] - uy * Sm[m - 1];
-    Sm[m] = ux * Sm[m - 1] + uy * Cm[m - 1];
-  }
+      for (int l = 1; l <= L; ++l) Ydot[sh_index(l, 0)] = d[l] * tz;
+    } else {
+      // the tangents of C_m and S_m, and tz C_m, tz S_m
+      const T ct = m == 1 ? tx : T(m) * (Cm[m - 1] * tx - Sm[m - 1] * ty);
+      const T st = m == 1 ? ty : T(m) * (Sm[m - 1] * tx + Cm[m - 1] * ty);
+      const T cz = Cm[m] * tz, sz = Sm[m] * tz;
+      Ydot[sh_index(m, m)] = f[0] * ct;
+      Ydot[sh_index(m, -m)] = f[0] * st;
 #pragma unroll
-  for (int m = 0; m <= L; ++m) {
-    const T pmm = sph_dfact<T>(m);
-    T p1 = T(0), p2 = T(0), d1 = T(0), d2 = T(0);
-#pragma unroll
-    for (int l = m; l <= L; ++l) {
-      T p, d;
-      if (l == m) { p = pmm; d = T(0); }
-      else if (l == m + 1) { p = T(2 * m + 1) * uz * pmm; d = T(2 * m + 1) * pmm; }
-      else {
-        const T inv = sph_inv<T>(l - m);
-        p = (T(2 * l - 1) * uz * p1 - T(l + m - 1) * p2) * inv;
-        d = (T(2 * l - 1) * (p1 + uz * d1) - T(l + m - 1) * d2) * inv;
-      }
-      p2 = p1; p1 = p; d2 = d1; d1 = d;
-      const T n = norm_lm<T>(sh_index(l, m));
-      if (m == 0) {
-        Ydot[sh_index(l, 0)] = n * d * tz;
-      } else {
-        const T mf = T(m);
-        Ydot[sh_index(l, m)] = n * (p * mf * (Cm[m - 1] * tx - Sm[m - 1] * ty) + d * Cm[m] * tz);
-        Ydot[sh_index(l, -m)] = n * (p * mf * (Sm[m - 1] * tx + Cm[m - 1] * ty) + d * Sm[m] * tz);
+      for (int l = m + 1; l <= L; ++l) {
+        Ydot[sh_index(l, m)] = f[l - m] * ct + d[l - m] * cz;
+        Ydot[sh_index(l, -m)] = f[l - m] * st + d[l - m] * sz;
       }
     }
-  }
+  });
 }
 
 // Raw Chebyshev values and r-derivatives (envelope 1, scaling 1) for B <= NBM <= kMaxB (NBM is

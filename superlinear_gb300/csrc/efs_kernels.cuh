@@ -1041,28 +1041,19 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
         vir[3] -= dx * double(Gy); vir[4] -= dx * double(Gz); vir[5] -= dy * double(Gz);
       }
     }
-    // per-atom virial: lane c < 6 writes component c (FP32 bulk: the compensated warp totals of
-    // all six components in FP32, then one conversion to FP64 for the whole warp)
+    // per-atom virial: one lane of four writes a component (FP32 bulk: compensated warp totals in
+    // FP32, then one conversion to FP64)
     double* vo = a.virial + (size_t)atom * 6;
+    const int vc = warp_sums_index(lane);
+    double total;
     if (sizeof(Real) == 4) {
-      float h = 0.f, l = 0.f;
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        warp_csum_pair(vhi[c], vlo[c]);
-        if (lane == c) { h = vhi[c]; l = vlo[c]; }
-      }
-      const double vc = double(h) + double(l);
-      if (lane < 6) vo[lane] = kGateRev ? vo[lane] + vc : vc;
+      float h, l;
+      warp_csums(vhi, vlo, lane, h, l);
+      total = double(h) + double(l);
     } else {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) vir[c] = warp_sum(vir[c]);
-      if (lane == 0) {
-        if (kGateRev)
-          for (int c = 0; c < 6; ++c) vo[c] += vir[c];
-        else
-          for (int c = 0; c < 6; ++c) vo[c] = vir[c];
-      }
+      total = warp_sums(vir, lane);
     }
+    if ((lane & 3) == 0 && vc < 6) vo[vc] = kGateRev ? vo[vc] + total : total;
     __syncwarp();
   }
   finish_dynamic();

@@ -1434,10 +1434,6 @@ Engine::Engine(const Model& model, int device, int precision) : model_(model), d
   SUS2G_CUDA(cudaStreamCreateWithPriority(&aux_stream_, cudaStreamNonBlocking, urgent_priority_));
   for (cudaEvent_t* e : {&ev_fork_, &ev_rev_, &ev_fork2_, &ev_join2_})
     SUS2G_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-  SUS2G_CUDA(upload_pass_constants<float>());
-  SUS2G_CUDA(upload_pass_constants<double>());
-  SUS2G_CUDA(upload_grad_constants<float>());
-  SUS2G_CUDA(upload_grad_constants<double>());
   // scalar readout and gate nodes are written with plain stores; duplicates would race
   auto unique = [](std::vector<int> v) { std::sort(v.begin(), v.end()); return std::adjacent_find(v.begin(), v.end()) == v.end(); };
   if (!unique(model_.scalar_map)) throw Error(3, "SUS2 model: duplicate entries in alpha_moment_mapping");

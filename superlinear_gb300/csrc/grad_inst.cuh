@@ -190,17 +190,13 @@ int launch_grad_moment_l(int mode, const GradArgs<float>& a, const GradLaunch& c
   return 1;
 }
 
-template <typename Real, int L>
-cudaError_t upload_grad_constants_l() { return sph_norm_upload(); }
-
 }  // namespace sus2g
 
 #define SUS2G_INSTANTIATE_GRAD(REAL, L)                                                                  \
   template GradLaunch grad_pass_config_l<REAL, L>(int, const DevModel<REAL>&, int, int, int);            \
   template int launch_grad_pass_l<REAL, L>(int, const GradArgs<REAL>&, const GradLaunch&, cudaStream_t); \
   template GradLaunch grad_edge_config_l<REAL, L>(int, const DevModel<REAL>&, int, int);                 \
-  template int launch_grad_edge_l<REAL, L>(int, const GradArgs<REAL>&, const GradLaunch&, cudaStream_t); \
-  template cudaError_t upload_grad_constants_l<REAL, L>();
+  template int launch_grad_edge_l<REAL, L>(int, const GradArgs<REAL>&, const GradLaunch&, cudaStream_t);
 #define SUS2G_INSTANTIATE_GRAD_MOMENT(L)                                                                 \
   template GradLaunch grad_moment_config_l<L>(int, const DevModel<float>&, int, int);                    \
   template int launch_grad_moment_l<L>(int, const GradArgs<float>&, const GradLaunch&, cudaStream_t);

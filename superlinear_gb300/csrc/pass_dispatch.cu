@@ -51,26 +51,6 @@ int launch_grad_pass(int L, int mode, const GradArgs<Real>& a, const GradLaunch&
   throw std::runtime_error("sh_l_max above 5 is not supported");
 }
 
-template <typename Real>
-cudaError_t upload_pass_constants() {
-  cudaError_t errs[6] = {upload_pass_constants_l<Real, 0>(), upload_pass_constants_l<Real, 1>(),
-                         upload_pass_constants_l<Real, 2>(), upload_pass_constants_l<Real, 3>(),
-                         upload_pass_constants_l<Real, 4>(), upload_pass_constants_l<Real, 5>()};
-  for (cudaError_t e : errs)
-    if (e != cudaSuccess) return e;
-  return cudaSuccess;
-}
-
-template <typename Real>
-cudaError_t upload_grad_constants() {
-  cudaError_t errs[6] = {upload_grad_constants_l<Real, 0>(), upload_grad_constants_l<Real, 1>(),
-                         upload_grad_constants_l<Real, 2>(), upload_grad_constants_l<Real, 3>(),
-                         upload_grad_constants_l<Real, 4>(), upload_grad_constants_l<Real, 5>()};
-  for (cudaError_t e : errs)
-    if (e != cudaSuccess) return e;
-  return cudaSuccess;
-}
-
 namespace {
 template <int GM>
 int launch_graph(const PassArgs<float>& a, int sm_count, cudaStream_t s) {
@@ -237,9 +217,5 @@ template GradLaunch grad_pass_config<float>(int, int, const DevModel<float>&, in
 template GradLaunch grad_pass_config<double>(int, int, const DevModel<double>&, int, int, int);
 template int launch_grad_pass<float>(int, int, const GradArgs<float>&, const GradLaunch&, cudaStream_t);
 template int launch_grad_pass<double>(int, int, const GradArgs<double>&, const GradLaunch&, cudaStream_t);
-template cudaError_t upload_pass_constants<float>();
-template cudaError_t upload_pass_constants<double>();
-template cudaError_t upload_grad_constants<float>();
-template cudaError_t upload_grad_constants<double>();
 
 }  // namespace sus2g

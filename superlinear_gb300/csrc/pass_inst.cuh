@@ -1,8 +1,6 @@
 // Launch templates of the per-atom passes for one spherical-harmonic order L.  The explicit
 // instantiations live in the small pass_fp{32,64}_l*.cu units (one group of L each) so that the
-// units compile in parallel; pass_dispatch.cu selects the unit by L at run time.  Each unit owns
-// its copy of the spherical-harmonic normalisation table and uploads it through
-// upload_pass_constants_l.
+// units compile in parallel; pass_dispatch.cu selects the unit by L at run time.
 #pragma once
 #include <algorithm>
 #include <stdexcept>
@@ -104,11 +102,7 @@ int launch_atom_pass_l(int mode, const PassArgs<Real>& a, int sm_count, cudaStre
   return pass_detail::launch_mode<Real, L, 0>(mode, 0, a, sm_count, s, pdl);
 }
 
-template <typename Real, int L>
-cudaError_t upload_pass_constants_l() { return sph_norm_upload(); }
-
 }  // namespace sus2g
 
 #define SUS2G_INSTANTIATE_PASS(REAL, L)                                                               \
-  template int launch_atom_pass_l<REAL, L>(int, const PassArgs<REAL>&, int, cudaStream_t, int, bool); \
-  template cudaError_t upload_pass_constants_l<REAL, L>();
+  template int launch_atom_pass_l<REAL, L>(int, const PassArgs<REAL>&, int, cudaStream_t, int, bool);
