@@ -90,6 +90,8 @@ struct PassArgs {
   int grid_mode;           // 0: all resident blocks; 1: the fewest blocks that keep the same atoms per warp
   int block_warps;         // launch shape: warps per block (1 .. kPassWarps; 0 = kPassWarps); the kernel
                            // reads its block size from blockDim
+  Real* keep;              // [keep_rows][kKeepBatches][2 F + H][32]: R, R', Y per edge (pass_keeps)
+  int keep_rows;
 };
 
 template <typename Real>
@@ -423,9 +425,10 @@ __device__ __forceinline__ void cheb_dot(const Real* c, int B, const Pair<Real> 
                                          Real& a, Real& ad) {
   Real cc[2 * NP];
   load_coeff_row<Real, BF, 2 * NP>(c, B, cc);
-  Pair<Real> sa{Real(0), Real(0)}, sd{Real(0), Real(0)};
+  // (T_0 = 1, D_0 = 0 and D_1 = 1 need no product)
+  Pair<Real> sa{cc[0], cc[1] * T[0].y}, sd{Real(0), cc[1]};
 #pragma unroll
-  for (int p = 0; p < NP; ++p) {
+  for (int p = 1; p < NP; ++p) {
     if (2 * p < B) {
       sa = fma2(Pair<Real>{cc[2 * p], cc[2 * p + 1]}, T[p], sa);
       if (DERIV) sd = fma2(Pair<Real>{cc[2 * p], cc[2 * p + 1]}, D[p], sd);
@@ -617,6 +620,20 @@ __device__ __forceinline__ void readout_seeds(const PassArgs<Real>& a, int atom,
 // The pass kernel.
 // ---------------------------------------------------------------------------------------------
 constexpr int kPassWarps = 4;
+// FP64: the forward keeps R, R' and Y of a centre's first kKeepBatches batches of 32 edges for its
+// adjoint -- the fused Static and outer passes in rows of the resident warps (they stay in L2), the
+// gate passes, two kernels, in rows of the centres.  The FP64 pipe is busy 85% of those passes, and
+// most of that is the radial functions: Static L3/K4/O2, 4,096 atoms 1,099 -> 752 us.  (FP32 passes
+// gain nothing: 57 -> 64 us; their recomputation is cheaper than the traffic.)
+constexpr int kKeepBatches = 4;
+template <typename Real>
+__host__ __device__ constexpr bool pass_keeps(int mode) {
+  return sizeof(Real) == 8 && (mode == kModeStatic || mode == kModeOuter || mode == kModeOuterBulk ||
+                               mode == kModeGateForward || mode == kModeGateReverse);
+}
+__host__ __device__ inline size_t pass_keep_values(int L, int F) {
+  return static_cast<size_t>(kKeepBatches) * (2 * F + (L + 1) * (L + 1)) * kWarp;
+}
 // Minimum resident blocks per SM (the register budget: 4 blocks = 128 registers, 3 = 168).  Both
 // budgets are compiled for the B = 8 passes and the engine's autotuner times them on the caller's
 // layout; without tuning: 4 for the FP32 kernels up to L = 3 and the L = 4 gate passes, 3
@@ -761,6 +778,11 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
   for (int atom = atom_first; atom < atom_stop; atom = dynamic ? grab() : atom + atom_step) {
     const int ti = C == 1 ? 0 : species_of(a.types, atom, C);
     const int e0 = a.row[atom], e1 = a.row_end[atom];
+    // the kept functions, a lane per column (batches past keep_batches evaluate them again)
+    constexpr bool kKeep = pass_keeps<Real>(MODE);
+    const int keep_row = gate_pass ? atom : blockIdx.x * warps + warp;
+    const int keep_batches = kKeep && keep_row < a.keep_rows ? kKeepBatches : 0;
+    Real* kept = kKeep ? a.keep + static_cast<size_t>(keep_row) * pass_keep_values(L, F) + lane : nullptr;
     // per-atom virial: FP64 for the FP64 form; compensated FP32 (hi, lo) for the FP32 bulk form
     double vir[6] = {0, 0, 0, 0, 0, 0};
     float vhi[6] = {0, 0, 0, 0, 0, 0}, vlo[6] = {0, 0, 0, 0, 0, 0};
@@ -794,6 +816,9 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
         // the u columns (each value read once before its u_mu overwrites it)
         if (effect_outer && !hb_on) rows_to_cols<Real>(stage, a.hsig, F, cur.j, nb, lane);
         Real* col = stage + lane;
+        const int kb = (base - e0) / kWarp;
+        const bool keep = kKeep && kb < keep_batches;
+        Real* kq = kKeep ? kept + static_cast<size_t>(kb) * (2 * F + H) * kWarp : nullptr;
         if (e < e1) {
           const V4 dv = cur.d;
           const Real r = dv.w, ir = Real(1) / r;
@@ -802,7 +827,10 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
             sph_values<L, Real>(dv.x * ir, dv.y * ir, dv.z * ir, Y);
             // (with two cutoffs the l > 0 functions beyond the angular one meet u = 0)
 #pragma unroll
-            for (int h = 0; h < H; ++h) col[(F + h) * S] = Y[h];
+            for (int h = 0; h < H; ++h) {
+              col[(F + h) * S] = Y[h];
+              if (kKeep && keep) kq[(2 * F + h) * kWarp] = Y[h];
+            }
           }
           const int pair = ti * C + cur.tj;
           const Real* pw = s_pw + pair * F;
@@ -812,8 +840,16 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
 #pragma unroll 1
           for (int k = 0; k < K; ++k) {
             Real R[Lp], Rd[Lp];
-            radial_channel<L, Real, false, BF>(dm, s_coeff, s_scal, pair, r, env, k, R, Rd);
+            if (!keep) radial_channel<L, Real, false, BF>(dm, s_coeff, s_scal, pair, r, env, k, R, Rd);
             Real* ck = col + k * Lp * S;
+            if (kKeep && keep) {
+              radial_channel<L, Real, true, BF>(dm, s_coeff, s_scal, pair, r, env, k, R, Rd);
+#pragma unroll
+              for (int l = 0; l < Lp; ++l) {
+                kq[(k * Lp + l) * kWarp] = R[l];
+                kq[(F + k * Lp + l) * kWarp] = Rd[l];
+              }
+            }
 #pragma unroll
             for (int l = 0; l < Lp; ++l) {
               Real w = pw[k * Lp + l];
@@ -953,7 +989,14 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
         ux = dv.x * ir; uy = dv.y * ir; uz = dv.z * ir;
         Real Y[2 * NPH];
         Y[2 * NPH - 1] = Real(0);
-        sph_values<L, Real>(ux, uy, uz, Y);
+        const bool have = kKeep && bt < keep_batches;
+        const Real* kq = kKeep ? kept + static_cast<size_t>(bt) * (2 * F + H) * kWarp : nullptr;
+        if (kKeep && have) {
+#pragma unroll
+          for (int h = 0; h < H; ++h) Y[h] = kq[(2 * F + h) * kWarp];
+        } else {
+          sph_values<L, Real>(ux, uy, uz, Y);
+        }
 #pragma unroll
         for (int p = 0; p < NPH; ++p) P[p] = {Real(0), Real(0)};
         const int pair = ti * C + tj;
@@ -965,7 +1008,15 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
 #pragma unroll 1
         for (int k = 0; k < K; ++k) {
           Real R[Lp], Rd[Lp];
-          radial_channel<L, Real, true, BF>(dm, s_coeff, s_scal, pair, r, env, k, R, Rd);
+          if (kKeep && have) {
+#pragma unroll
+            for (int l = 0; l < Lp; ++l) {
+              R[l] = kq[(k * Lp + l) * kWarp];
+              Rd[l] = kq[(F + k * Lp + l) * kWarp];
+            }
+          } else {
+            radial_channel<L, Real, true, BF>(dm, s_coeff, s_scal, pair, r, env, k, R, Rd);
+          }
           Real* ck = col + k * Lp * S;
           Real wR[Lp];
           Pair<Real> Sl[Lp];

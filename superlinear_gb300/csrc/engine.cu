@@ -2689,6 +2689,16 @@ int Engine::launch_shape(int mode, PassArgs<Real> a, int blocks, bool pdl) {
   // the dynamic order's counter pair of this mode (zero between launches: the launch's last
   // warp resets it, so no memset sits between this launch and its predecessor)
   if (a.atom_order == 2) a.work = work_.as<int>() + 2 * mode;
+  // FP64: the kept functions' rows, for up to 16 resident warps per SM (fused passes) or for the
+  // centres of layouts up to kKeepCentres (gate passes: 49 KB per centre at L3/K4; larger ones
+  // evaluate them again in the reverse)
+  if (pass_keeps<Real>(mode)) {
+    const bool gate = mode == kModeGateForward || mode == kModeGateReverse;
+    DevBuf& buf = gate ? keep_gate_ : keep_;
+    a.keep_rows = !gate ? std::min(16 * sm_count_, (ncentres_ + 3) / 4 * 4) : ncentres_ <= kKeepCentres ? ncentres_ : 0;
+    buf.ensure(sizeof(Real) * pass_keep_values(model_.L, model_.F) * std::max(1, a.keep_rows));
+    a.keep = buf.as<Real>();
+  }
   return launch_atom_pass<Real>(model_.L, mode, a, sm_count_, stream_, blocks, pdl);
 }
 

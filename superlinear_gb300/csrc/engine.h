@@ -330,6 +330,8 @@ class Engine {
   int gate_split_ = -1;         // Effect gate forward and reverse passes split (together: gkeep_)
   bool gate_ran_split_ = false; // the form of the last gate forward pass, which its reverse takes too
   int gate_split_blocks_[2] = {0, 0};    // their per-edge kernels' register budgets
+  static constexpr int kKeepCentres = 8192;
+  DevBuf keep_, keep_gate_;     // FP64 passes: R, R' and Y per edge for the adjoint (pass_keeps)
   DevBuf mom_;                  // the split pass's moments, then their adjoints [N][K H]
   DevBuf gkeep_;                // split gate passes: gate values kept for the reverse, adjoints of h per centre [N][F]
   // second stream for independent work inside a step (reverse edges beside the first pass, the
