@@ -42,7 +42,7 @@ void DevBuf::release() {
 // ------------------------------------------------------------------------------------------------
 namespace {
 
-// Frame of every atom; with posh / posl (FP32 engines with image-scan frames) also its position
+// Frame of every atom; with posh / posl (batches with image-scan frames) also its position
 // as double-float parts x = xh + xl, xh = fl32(x), for the image scan's FP32 arithmetic.
 __global__ void k_frame_of(const FramePlan* plans, int nframes, int* frame_of, const double* pos, float4* posh,
                            float4* posl) {
@@ -125,65 +125,7 @@ __global__ void k_bin_place(const FramePlan* plans, int nframes, bool find_frame
                           static_cast<float>(wz - hz), 0};
 }
 
-template <typename Real>
-__device__ __forceinline__ void write_edge(long long e, int j, int a, int b, int c, double x, double y, double z, double r2,
-                                           int* nbr, typename Vec4<Real>::type* d4, unsigned long long* key) {
-  nbr[e] = j;
-  typename Vec4<Real>::type v;
-  v.x = Real(x); v.y = Real(y); v.z = Real(z);
-  // FP32 records: the distance from the rounded r^2 (an FP32 square root; the FP64 one costs tens
-  // of FP64-pipe instructions)
-  if constexpr (sizeof(Real) == 4) v.w = sqrtf(static_cast<float>(r2));
-  else v.w = sqrt(r2);
-  d4[e] = v;
-  key[e] = edge_key(j, a, b, c);
-}
-
 constexpr int kFillWarps = 8;
-constexpr int kFillSortStage = 256;  // keys per warp kept in shared memory for the in-kernel sort
-constexpr int kFillSortPer = 4;
-
-// Sorts a centre's n staged edges (slots pad .. pad + n - 1) by key into the final arrays at the
-// same slots: each key's rank among the centre's keys (unique within a centre), up to
-// kFillSortPer keys per lane per pass with their payloads loaded while the ranks are counted;
-// keys from shared memory when the centre has at most kFillSortStage of them.
-template <typename Real>
-__device__ __forceinline__ void sort_centre_edges(int lane, int n, long long pad, const unsigned long long* skeys,
-                                                  const unsigned long long* key, const int* nbr,
-                                                  const typename Vec4<Real>::type* d4, unsigned long long* key_out,
-                                                  int* nbr_out, typename Vec4<Real>::type* d4_out) {
-  const unsigned long long* src = n <= kFillSortStage ? skeys : key + pad;
-  for (int q0 = 0; q0 < n; q0 += kFillSortPer * kWarp) {
-    unsigned long long kk[kFillSortPer];
-    int nb[kFillSortPer], rank[kFillSortPer];
-    typename Vec4<Real>::type dd[kFillSortPer];
-#pragma unroll
-    for (int u = 0; u < kFillSortPer; ++u) {
-      const int q = q0 + u * kWarp + lane;
-      kk[u] = ~0ull;
-      rank[u] = 0;
-      if (q < n) {
-        kk[u] = src[q];
-        nb[u] = nbr[pad + q];
-        dd[u] = d4[pad + q];
-      }
-    }
-    for (int t = 0; t < n; ++t) {
-      const unsigned long long kt = src[t];
-#pragma unroll
-      for (int u = 0; u < kFillSortPer; ++u) rank[u] += kt < kk[u];
-    }
-#pragma unroll
-    for (int u = 0; u < kFillSortPer; ++u) {
-      if (q0 + u * kWarp + lane < n) {
-        key_out[pad + rank[u]] = kk[u];
-        nbr_out[pad + rank[u]] = nb[u];
-        d4_out[pad + rank[u]] = dd[u];
-      }
-    }
-  }
-}
-
 // A centre's edges between the walk and the sort: the first kStage of them in shared memory, the
 // rest in its padded slots of the staging buffers.
 template <typename Real> struct EdgeStage {
@@ -192,8 +134,8 @@ template <typename Real> struct EdgeStage {
   int j[kStage], image[kStage];
 };
 
-// rank[u] = how many of the centre's n neighbours come before neighbour mine[u].  A cell-list frame
-// is at least 3 r_c wide, so a neighbour appears once per centre and its index alone is the order.
+// rank[u] = how many of the centre's n words come before mine[u].  A cell-list frame is at least
+// 3 r_c wide, so a neighbour appears once per centre and its index alone is the order.
 template <int U, typename Real>
 __device__ __forceinline__ void rank_neighbours(int n, const EdgeStage<Real>& st, const int* rest, const int (&mine)[U],
                                                 int (&rank)[U]) {
@@ -226,6 +168,17 @@ __device__ __forceinline__ void order_edges(int lane, int n, const EdgeStage<Rea
 #pragma unroll
   for (int u = 0; u < U; ++u)
     if (u * kWarp + lane < n) perm[rank[u]] = u * kWarp + lane;
+}
+
+template <typename Real>
+__device__ __forceinline__ void order_any(int lane, int n, const EdgeStage<Real>& st, const int* rest, int* perm) {
+  switch ((n + kWarp - 1) / kWarp) {
+    case 0: break;
+    case 1: order_edges<1, Real>(lane, n, st, rest, perm); break;
+    case 2: order_edges<2, Real>(lane, n, st, rest, perm); break;
+    case 3: order_edges<3, Real>(lane, n, st, rest, perm); break;
+    default: order_edges<4, Real>(lane, n, st, rest, perm);
+  }
 }
 
 // Cell-list frames: one warp per centre over its 125 stencil bins (warp_bin_edges), one pass.  The
@@ -295,13 +248,7 @@ k_edge_fill_bins(const FramePlan* plans, const int* frame_of, const double* pos,
   };
   if (n <= 4 * kWarp) {
     int* perm = reinterpret_cast<int*>(walks[w].queue);  // (the ring is empty)
-    switch ((n + kWarp - 1) / kWarp) {
-      case 0: break;
-      case 1: order_edges<1, Real>(lane, n, st, rest, perm); break;
-      case 2: order_edges<2, Real>(lane, n, st, rest, perm); break;
-      case 3: order_edges<3, Real>(lane, n, st, rest, perm); break;
-      default: order_edges<4, Real>(lane, n, st, rest, perm);
-    }
+    order_any<Real>(lane, n, st, rest, perm);
     __syncwarp();
     for (int q = lane; q < n; q += kWarp) write(q, perm[q]);
   } else {
@@ -317,18 +264,35 @@ k_edge_fill_bins(const FramePlan* plans, const int* frame_of, const double* pos,
 // Periodic frames too small for cell lists (a perpendicular width below 3 r_c, or at most 512
 // atoms): warp per centre i, lanes over the frame's atoms j.  For each j the image range per axis
 // is ceil(-f - reach) .. floor(-f + reach), f = (x_j - x_i) . inv(cell), and every image n in it
-// is tested exactly in FP64 (r^2 = |x_j + n.cell - x_i|^2 < r_c^2).  Accepted edges take the
-// centre's next padded slot (a shared-memory counter) and are then sorted by (j, n) like the
-// cell-list edges, so every periodic batch ends in the same padded layout without host
-// synchronisation; a count above cap raises *overflow as in the cell-list kernel.
+// with r^2 = |x_j + n.cell - x_i|^2 < r_c^2 in FP64 is an edge.  As in the cell-list fill, a lane walks
+// its images with an FP32 prefilter, what passes waits in a ring, and a full warp of it is tested:
+//   * dx = x_j - x_i in double-float (hi, lo) parts; f = dx_hi . inv(cell) in FP32 errs by at most
+//     ~7 2^-24 S, S = sum |dx_r inv_rq|; widening reach by 1e-4 + 1e-6 S keeps every image of the
+//     FP64 range.
+//   * Prefilter: dx_hi + n.cell_hi errs by less than 16 2^-24 M, M = |dx| + sum_r |n_r| |cell_r| (one
+//     norms), so nothing within r_c is lost above (r_c + 16 2^-24 M)^2 (1 + 1e-4).
+//   * FP64 engines then test in FP64.  FP32 engines accumulate the vector as double-float pairs
+//     (exact two-sums, m cell_hi split exactly by an FMA): absolute error a few dozen 2^-48 of M;
+//     rounded once to FP32, with M <= 1e6 r_c, r^2 near r_c^2 errs by well under 1e-6 r_c^2, so r^2
+//     below lo2 = (1 - 1e-4) r_c^2 is inside and above hi2 = (1 + 1e-4) r_c^2 outside in FP64 too,
+//     and the band takes the FP64 test.  The accepted set is the FP64 set.
+//   * Non-finite positions, ranges outside the packable [-64, 63] and larger M take the FP64 loop per
+//     lane, which reports the first two.
+// The accepted edges are staged, put in order by (j, n) -- in 31 bits up to 1,024 atoms -- and written
+// once to the centre's padded slots, as by the cell-list kernel.
+// Bound by instructions: with every image's vector formed in place by its lane and 64-bit keys,
+// 17,544 atoms of 256 frames took 98 us and 3,840 of 64 frames 39 us (FP64, 884 of 12 frames: 67 us);
+// so 75, 26 and 34 us.
 template <typename Real>
 __global__ void __launch_bounds__(kFillWarps * kWarp)
 k_edge_image_fill(const FramePlan* plans, const int* frame_of, const double* pos, const float4* posh,
                   const float4* posl, const int* types, int C, int natoms, double rc2, int* counts,
                   int* nbr, typename Vec4<Real>::type* d4, unsigned long long* key, int* overflow, int* error, int* row,
                   int* row_end, unsigned long long* key_out, int* nbr_out, typename Vec4<Real>::type* d4_out) {
-  __shared__ unsigned long long skeys[kFillWarps][kFillSortStage];
-  __shared__ int cursor[kFillWarps];
+  using Stage = EdgeStage<Real>;
+  __shared__ __align__(16) Stage stages[kFillWarps];
+  __shared__ int2 queues[kFillWarps][kEdgeQueue];  // (j, packed image)
+  __shared__ int cursors[kFillWarps];
   pdl_wait();  // the frame map (and, in mixed batches, the cell-list fill) of the previous kernels
   pdl_launch_dependents();
   const int i = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kWarp);
@@ -336,9 +300,13 @@ k_edge_image_fill(const FramePlan* plans, const int* frame_of, const double* pos
   const FramePlan& fp = plans[frame_of[i]];
   if (fp.use_bins) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x / kWarp;
+  const unsigned below = (1u << lane) - 1u;
   const long long pad = fp.pad0 + static_cast<long long>(i - fp.a0) * fp.cap;
   const int cap = fp.cap;
-  if (lane == 0) cursor[w] = 0;
+  Stage& st = stages[w];
+  int2* queue = queues[w];
+  int& cursor = cursors[w];
+  if (lane == 0) cursor = 0;
   __syncwarp();
   const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
   // a non-finite centre is reported and gets no edges; a non-finite neighbour is skipped (it
@@ -349,127 +317,203 @@ k_edge_image_fill(const FramePlan* plans, const int* frame_of, const double* pos
   if (lane == 0 && (types[i] < 0 || types[i] >= C)) record_error(error, kErrBadSpecies);
   const double* c = fp.cell;
   const double* inv = fp.inv;
-  float4 cih = make_float4(0.f, 0.f, 0.f, 0.f), cil = cih;
-  if (posh) { cih = posh[i]; cil = posl[i]; }
-  for (int j = fp.a0 + lane; centre_ok && j < fp.a1; j += kWarp) {
-    auto accept = [&](int a, int b, int cc, double vx, double vy, double vz, double r2) {
-      const int k = atomicAdd(&cursor[w], 1);
-      if (k < cap) {
-        write_edge<Real>(pad + k, j, a, b, cc, vx, vy, vz, r2, nbr, d4, key);
-        if (k < kFillSortStage) skeys[w][k] = edge_key(j, a, b, cc);
+  const float4 cih = posh[i], cil = posl[i];
+  float ch[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) ch[q] = fp.cellf[q];
+  const float rcf = sqrtf(fp.rc2f);
+  // frames of at most 1,024 atoms: j and the image in one staged word (see the sort below)
+  const bool one_word = fp.a1 - fp.a0 <= 1024;
+  auto stage_edge = [&](int k, int j, int image, Real x, Real y, Real z, Real r2) {
+    typename Vec4<Real>::type v;
+    v.x = x; v.y = y; v.z = z;
+    if constexpr (sizeof(Real) == 4) v.w = sqrtf(r2);
+    else v.w = sqrt(r2);
+    const int word = one_word ? ((j - fp.a0) << 21) | image : j;
+    if (k < Stage::kStage) {
+      st.d4[k] = v;
+      st.j[k] = word;
+      st.image[k] = image;
+    } else if (k < cap) {
+      d4[pad + k] = v;
+      nbr[pad + k] = word;
+      key[pad + k] = static_cast<unsigned long long>(image);
+    }
+  };
+  auto exact = [&](int j, int a, int b, int cc, double& vx, double& vy, double& vz) {
+    const double dx = pos[3 * j] - xi, dy = pos[3 * j + 1] - yi, dz = pos[3 * j + 2] - zi;
+    vx = dx + a * c[0] + b * c[3] + cc * c[6];
+    vy = dy + a * c[1] + b * c[4] + cc * c[7];
+    vz = dz + a * c[2] + b * c[5] + cc * c[8];
+    return vx * vx + vy * vy + vz * vz;
+  };
+  int head = 0, tail = 0;  // warp-uniform ring positions
+  auto drain = [&](int n) {
+    bool ok = false;
+    int j = 0, image = 0;
+    Real vx = 0, vy = 0, vz = 0, r2 = 0;
+    if (lane < n) {
+      const int2 q = queue[(head + lane) & (kEdgeQueue - 1)];
+      j = q.x;
+      image = q.y;
+      const int a = (image >> 14) - 64, b = ((image >> 7) & 127) - 64, cc = (image & 127) - 64;
+      if constexpr (sizeof(Real) == 8) {
+        r2 = exact(j, a, b, cc, vx, vy, vz);
+        ok = r2 < rc2;
+      } else {
+        const float4 hj = posh[j], lj = posl[j];
+        const float* cl = fp.celll;
+        float xh = hj.x, xl = lj.x, yh = hj.y, yl = lj.y, zh = hj.z, zl = lj.z;
+        df_acc(xh, xl, -cih.x, -cil.x);
+        df_acc(yh, yl, -cih.y, -cil.y);
+        df_acc(zh, zl, -cih.z, -cil.z);
+        const float m[3] = {static_cast<float>(a), static_cast<float>(b), static_cast<float>(cc)};
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          df_acc_mul(xh, xl, m[r], ch[3 * r], cl[3 * r]);
+          df_acc_mul(yh, yl, m[r], ch[3 * r + 1], cl[3 * r + 1]);
+          df_acc_mul(zh, zl, m[r], ch[3 * r + 2], cl[3 * r + 2]);
+        }
+        vx = xh + xl; vy = yh + yl; vz = zh + zl;
+        r2 = vx * vx + vy * vy + vz * vz;
+        ok = r2 < fp.lo2;
+        if (!ok && r2 < fp.hi2) {
+          double ex, ey, ez;
+          const double d2 = exact(j, a, b, cc, ex, ey, ez);
+          ok = d2 < rc2;
+          vx = static_cast<float>(ex); vy = static_cast<float>(ey); vz = static_cast<float>(ez);
+          r2 = static_cast<float>(d2);
+        }
       }
-    };
-    int lo[3], hi[3];
-    if constexpr (sizeof(Real) == 4) {
-      // FP32 engines: double-float arithmetic on the (hi, lo) positions, FP64 only near the cutoff.
-      //  * dx = x_j - x_i and every image vector v = dx + n . cell are accumulated as double-float
-      //    pairs (exact two-sums, m cell_hi split exactly by an FMA): their absolute error is a few
-      //    dozen 2^-48 of M, the largest magnitude involved, M = |dx| + sum_r |n_r| |cell_r|.  The
-      //    vector is then rounded once to FP32 and r^2 formed in FP32: with M <= 1e6 r_c, r^2 near
-      //    r_c^2 errs by well under 1e-6 r_c^2, so r^2 below lo2 = (1 - 1e-4) r_c^2 is inside and
-      //    above hi2 = (1 + 1e-4) r_c^2 outside in FP64 too, and the band takes the exact FP64 test.
-      //    The accepted set is the FP64 set; accepted vectors are the exact ones rounded once.
-      //  * Ranges: f = dx_hi . inv(cell) in FP32 errs by at most ~7 2^-24 S, S = sum |dx_r inv_rq|;
-      //    widening reach by 1e-4 + 1e-6 S keeps every image of the FP64 range (extra images are
-      //    rejected by the distance test).
-      //  Non-finite positions, ranges outside the packable [-64, 63] and larger M take the FP64 loop,
-      //  which reports the first two.
+      ok = ok && !(j == i && a == 0 && b == 0 && cc == 0);
+    }
+    head += n;
+    const unsigned mask = __ballot_sync(0xffffffffu, ok);
+    const int k0 = cursor;
+    __syncwarp();
+    if (lane == 0) cursor = k0 + __popc(mask);
+    if (ok) stage_edge(k0 + __popc(mask & below), j, image, vx, vy, vz, r2);
+    __syncwarp();
+  };
+  for (int j0 = fp.a0; centre_ok && j0 < fp.a1; j0 += kWarp) {
+    const int j = j0 + lane;
+    int lo[3] = {0, 0, 0}, hi[3] = {-1, -1, -1};
+    float xh = 0.f, yh = 0.f, zh = 0.f, screen = 0.f;
+    if (j < fp.a1) {
       const float4 hj = posh[j], lj = posl[j];
-      float xh = hj.x, xl = lj.x, yh = hj.y, yl = lj.y, zh = hj.z, zl = lj.z;
+      float xl = lj.x, yl = lj.y, zl = lj.z;
+      xh = hj.x; yh = hj.y; zh = hj.z;
       df_acc(xh, xl, -cih.x, -cil.x);
       df_acc(yh, yl, -cih.y, -cil.y);
       df_acc(zh, zl, -cih.z, -cil.z);
-      const float* ch = fp.cellf;
-      const float* cl = fp.celll;
       bool fast = true;
+      float m = fabsf(xh) + fabsf(yh) + fabsf(zh);
+#pragma unroll
       for (int q = 0; q < 3; ++q) {
-        const float i0 = fp.invf[q], i1 = fp.invf[3 + q], i2 = fp.invf[6 + q];
-        const float f = xh * i0 + yh * i1 + zh * i2;
-        const float S = fabsf(xh * i0) + fabsf(yh * i1) + fabsf(zh * i2);
+        const float t0 = xh * fp.invf[q], t1 = yh * fp.invf[3 + q], t2 = zh * fp.invf[6 + q];
+        const float f = t0 + t1 + t2, S = fabsf(t0) + fabsf(t1) + fabsf(t2);
         const float reach = fp.reachf[q] + 1e-4f + 1e-6f * S;
         const float l = ceilf(-f - reach), h = floorf(-f + reach);
-        if (!(l >= -64.0f && h <= 63.0f)) { fast = false; break; }
-        lo[q] = static_cast<int>(l);
-        hi[q] = static_cast<int>(h);
+        if (l >= -64.0f && h <= 63.0f) {
+          lo[q] = static_cast<int>(l);
+          hi[q] = static_cast<int>(h);
+          m += static_cast<float>(max(abs(lo[q]), abs(hi[q]))) * (fabsf(ch[3 * q]) + fabsf(ch[3 * q + 1]) + fabsf(ch[3 * q + 2]));
+        } else {
+          fast = false;
+        }
       }
-      if (fast) {
-        float m = fabsf(xh) + fabsf(yh) + fabsf(zh);
-        for (int r = 0; r < 3; ++r)
-          m += static_cast<float>(max(abs(lo[r]), abs(hi[r]))) *
-               (fabsf(ch[3 * r]) + fabsf(ch[3 * r + 1]) + fabsf(ch[3 * r + 2]));
-        fast = m * m <= 1e12f * fp.rc2f;
-      }
-      if (fast) {
-        const float lo2 = fp.lo2, hi2 = fp.hi2;
-        for (int a = lo[0]; a <= hi[0]; ++a) {
-          float axh = xh, axl = xl, ayh = yh, ayl = yl, azh = zh, azl = zl;
-          df_acc_mul(axh, axl, a, ch[0], cl[0]);
-          df_acc_mul(ayh, ayl, a, ch[1], cl[1]);
-          df_acc_mul(azh, azl, a, ch[2], cl[2]);
-          for (int b = lo[1]; b <= hi[1]; ++b) {
-            float pxh = axh, pxl = axl, pyh = ayh, pyl = ayl, pzh = azh, pzl = azl;
-            df_acc_mul(pxh, pxl, b, ch[3], cl[3]);
-            df_acc_mul(pyh, pyl, b, ch[4], cl[4]);
-            df_acc_mul(pzh, pzl, b, ch[5], cl[5]);
-            for (int cc = lo[2]; cc <= hi[2]; ++cc) {
-              float vxh = pxh, vxl = pxl, vyh = pyh, vyl = pyl, vzh = pzh, vzl = pzl;
-              df_acc_mul(vxh, vxl, cc, ch[6], cl[6]);
-              df_acc_mul(vyh, vyl, cc, ch[7], cl[7]);
-              df_acc_mul(vzh, vzl, cc, ch[8], cl[8]);
-              const float vx = vxh + vxl, vy = vyh + vyl, vz = vzh + vzl;
-              const float r2 = vx * vx + vy * vy + vz * vz;
-              if (!(r2 < hi2) || (i == j && a == 0 && b == 0 && cc == 0)) continue;
-              if (r2 < lo2) {
-                accept(a, b, cc, vx, vy, vz, r2);
-              } else {
-                const double dx = pos[3 * j] - xi, dy = pos[3 * j + 1] - yi, dz = pos[3 * j + 2] - zi;
-                const double ex = dx + a * c[0] + b * c[3] + cc * c[6];
-                const double ey = dy + a * c[1] + b * c[4] + cc * c[7];
-                const double ez = dz + a * c[2] + b * c[5] + cc * c[8];
-                const double d2 = ex * ex + ey * ey + ez * ez;
-                if (d2 < rc2) accept(a, b, cc, ex, ey, ez, d2);
-              }
-            }
+      fast = fast && m * m <= 1e12f * fp.rc2f;
+      const float lim = rcf + 9.6e-7f * m;
+      screen = lim * lim * 1.0001f;
+      if (!fast) {
+        // FP64 test of every image, by this lane
+        const double dx = pos[3 * j] - xi, dy = pos[3 * j + 1] - yi, dz = pos[3 * j + 2] - zi;
+        const bool finite = isfinite(dx) && isfinite(dy) && isfinite(dz);
+        for (int q = 0; finite && q < 3; ++q) {
+          const double f = dx * inv[q] + dy * inv[3 + q] + dz * inv[6 + q];
+          double l = ceil(-f - fp.reach[q]), h = floor(-f + fp.reach[q]);
+          if (l < -64.0 || h > 63.0) {
+            record_error(error, kErrImageRange);
+            l = fmax(l, -64.0);
+            h = fmin(h, 63.0);
           }
+          lo[q] = static_cast<int>(l);
+          hi[q] = static_cast<int>(fmax(h, l - 1.0));
         }
-        continue;
+        for (int a = lo[0]; finite && a <= hi[0]; ++a)
+          for (int b = lo[1]; b <= hi[1]; ++b)
+            for (int cc = lo[2]; cc <= hi[2]; ++cc) {
+              if (i == j && a == 0 && b == 0 && cc == 0) continue;
+              double vx, vy, vz;
+              const double r2 = exact(j, a, b, cc, vx, vy, vz);
+              if (r2 < rc2)
+                stage_edge(atomicAdd(&cursor, 1), j, ((a + 64) << 14) | ((b + 64) << 7) | (cc + 64), Real(vx), Real(vy), Real(vz), Real(r2));
+            }
+        hi[0] = lo[0] - 1;  // nothing left for the walk
       }
     }
-    // FP64: the exact test of every image (FP64 engines; FP32 engines' fallback)
-    const double dx = pos[3 * j] - xi, dy = pos[3 * j + 1] - yi, dz = pos[3 * j + 2] - zi;
-    if (!(isfinite(dx) && isfinite(dy) && isfinite(dz))) continue;
-    for (int q = 0; q < 3; ++q) {
-      const double f = dx * inv[q] + dy * inv[3 + q] + dz * inv[6 + q];
-      double l = ceil(-f - fp.reach[q]), h = floor(-f + fp.reach[q]);
-      if (l < -64.0 || h > 63.0) {
-        record_error(error, kErrImageRange);
-        l = fmax(l, -64.0);
-        h = fmin(h, 63.0);
+    __syncwarp();
+    const int mine = max(0, hi[0] - lo[0] + 1) * max(0, hi[1] - lo[1] + 1) * max(0, hi[2] - lo[2] + 1);
+    const int most = __reduce_max_sync(0xffffffffu, mine);
+    int a = lo[0], b = lo[1], cc = lo[2];
+    for (int t = 0; t < most; ++t) {
+      const float fa = static_cast<float>(a), fb = static_cast<float>(b), fc = static_cast<float>(cc);
+      const float vx = fmaf(fa, ch[0], fmaf(fb, ch[3], fmaf(fc, ch[6], xh)));
+      const float vy = fmaf(fa, ch[1], fmaf(fb, ch[4], fmaf(fc, ch[7], yh)));
+      const float vz = fmaf(fa, ch[2], fmaf(fb, ch[5], fmaf(fc, ch[8], zh)));
+      const bool pass = t < mine && vx * vx + vy * vy + vz * vz < screen;
+      const unsigned m = __ballot_sync(0xffffffffu, pass);
+      if (pass)
+        queue[(tail + __popc(m & below)) & (kEdgeQueue - 1)] = make_int2(j, ((a + 64) << 14) | ((b + 64) << 7) | (cc + 64));
+      tail += __popc(m);
+      if (++cc > hi[2]) {
+        cc = lo[2];
+        if (++b > hi[1]) { b = lo[1]; ++a; }
       }
-      lo[q] = static_cast<int>(l);
-      hi[q] = static_cast<int>(fmax(h, l - 1.0));
+      __syncwarp();
+      if (tail - head >= 32) drain(32);
     }
-    for (int a = lo[0]; a <= hi[0]; ++a)
-      for (int b = lo[1]; b <= hi[1]; ++b)
-        for (int cc = lo[2]; cc <= hi[2]; ++cc) {
-          if (i == j && a == 0 && b == 0 && cc == 0) continue;
-          const double vx = dx + a * c[0] + b * c[3] + cc * c[6];
-          const double vy = dy + a * c[1] + b * c[4] + cc * c[7];
-          const double vz = dz + a * c[2] + b * c[5] + cc * c[8];
-          const double r2 = vx * vx + vy * vy + vz * vz;
-          if (r2 < rc2) accept(a, b, cc, vx, vy, vz, r2);
-        }
   }
+  if (tail > head) drain(tail - head);
   __syncwarp();
-  const int total = cursor[w], n = min(total, cap);
+  const int total = cursor, n = min(total, cap);
   if (lane == 0) {
     counts[i] = n;
     if (total > cap) atomicMax(overflow, total);
-  }
-  sort_centre_edges<Real>(lane, n, pad, skeys[w], key, nbr, d4, key_out, nbr_out, d4_out);
-  if (lane == 0) {
     row[i] = static_cast<int>(pad);
     row_end[i] = static_cast<int>(pad) + n;
+  }
+  const int* rest = nbr + pad;
+  auto word_of = [&](int q) { return q < Stage::kStage ? st.j[q] : rest[q]; };
+  auto image_of = [&](int q) { return q < Stage::kStage ? st.image[q] : static_cast<int>(key[pad + q]); };
+  auto write = [&](int to, int from) {
+    const int word = word_of(from), j = one_word ? fp.a0 + (word >> 21) : word;
+    key_out[pad + to] = (static_cast<unsigned long long>(j) << 21) | static_cast<unsigned long long>(image_of(from));
+    nbr_out[pad + to] = j;
+    d4_out[pad + to] = from < Stage::kStage ? st.d4[from] : d4[pad + from];
+  };
+  if (one_word && n <= 4 * kWarp) {
+    int* perm = reinterpret_cast<int*>(queue);  // (the ring is empty)
+    order_any<Real>(lane, n, st, rest, perm);
+    __syncwarp();
+    for (int q = lane; q < n; q += kWarp) write(q, perm[q]);
+  } else if (one_word) {
+    for (int q = lane; q < n; q += kWarp) {
+      const int mine[1] = {word_of(q)};
+      int rank[1];
+      rank_neighbours<1, Real>(n, st, rest, mine, rank);
+      write(rank[0], q);
+    }
+  } else {
+    for (int q = lane; q < n; q += kWarp) {
+      const int j = word_of(q), image = image_of(q);
+      int rank = 0;
+      for (int t = 0; t < n; ++t) {
+        const int o = word_of(t);
+        rank += o < j || (o == j && image_of(t) < image);
+      }
+      write(rank, q);
+    }
   }
 }
 
@@ -1951,7 +1995,7 @@ void Engine::build_edges(int nframes, const int* frame_natoms, const double* cel
   // batches with cell lists only: the binning kernel finds each atom's frame itself
   const bool find_frame = bins && bins_frames_ == nframes;
   if (nframes && !find_frame) {
-    const bool split = precision_ == kFP32 && bins_frames_ < nframes;
+    const bool split = bins_frames_ < nframes;
     if (split) posf_.ensure(2 * sizeof(float4) * std::max(1, a));
     k_frame_of<<<nframes, 256, 0, s>>>(plan_.as<FramePlan>(), nframes, frame_of_.as<int>(), d_pos,
                                        split ? posf_.as<float4>() : nullptr, split ? posf_.as<float4>() + a : nullptr);
@@ -2025,7 +2069,7 @@ void Engine::build_edges(int nframes, const int* frame_natoms, const double* cel
             pad_key_.as<unsigned long long>(), overflow, error_.as<int>(), RW, RE, KO, NO, d4_.as<EdgeF>()));
       else
         SUS2G_CUDA(launch_kernel((pdl_ & kPdlFill) != 0, k_edge_image_fill<double>, dim3(warp_blocks), dim3(kFillWarps * kWarp), 0, s,
-            P, FO, d_pos, nullptr, nullptr, d_types, model_.C, a, rc2, counts_.as<int>(), pad_nbr_.as<int>(),
+            P, FO, d_pos, posf_.as<float4>(), posf_.as<float4>() + a, d_types, model_.C, a, rc2, counts_.as<int>(), pad_nbr_.as<int>(),
             pad_d4_.as<EdgeD>(),
             pad_key_.as<unsigned long long>(), overflow, error_.as<int>(), RW, RE, KO, NO, d4_.as<EdgeD>()));
       ++launches_;

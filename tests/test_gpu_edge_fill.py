@@ -53,3 +53,47 @@ def test_edges_match_direct_search(mean, precision):
     np.testing.assert_array_equal(ci, wi)
     np.testing.assert_array_equal(cj, wj)
     assert np.abs(d - wd).max() < (1e-12 if precision == sg.FP64 else 5e-7)
+
+
+def direct_images(pos, cell):
+    """As direct(), with as many images as the cell needs, ordered by (i, j, n) of the given positions."""
+    inv = np.linalg.inv(cell)
+    off = np.floor(pos @ inv)
+    home = pos - off @ cell
+    span = [int(np.ceil(RC * np.linalg.norm(inv[:, q]))) + 1 for q in range(3)]
+    out = []
+    for n in np.ndindex(*(2 * s + 1 for s in span)):
+        n = np.array(n) - span
+        d = home[None] + n @ cell - home[:, None]
+        hit = (d ** 2).sum(-1) < RC * RC
+        if not n.any():
+            np.fill_diagonal(hit, False)
+        i, j = np.nonzero(hit)
+        out.append((i, j, d[i, j], n - off[j] + off[i]))
+    i, j, d, n = (np.concatenate(x) for x in zip(*out))
+    o = np.lexsort((n[:, 2], n[:, 1], n[:, 0], j, i))
+    return i[o], j[o], d[o]
+
+
+# (cell widths, atoms, cells away from home): images of one pair, the self images of a lone atom, counts past
+# the staged and the register limits, a thin cell of more than 1,024 atoms (two-word order), ranges
+# close to the packable limit
+SMALL = [((2.6, 2.6, 2.6), 1, 0), ((3.5, 3.5, 3.5), 8, 0), ((3.0, 3.0, 3.0), 10, 3), ((7.1, 7.1, 7.1), 64, 2),
+         ((9.0, 11.0, 14.0), 333, 1), ((12.0, 20.0, 60.0), 1100, 1), ((4.0, 4.0, 30.0), 40, 29)]
+
+
+@pytest.mark.parametrize("precision", [sg.FP32, sg.FP64])
+@pytest.mark.parametrize("case", range(len(SMALL)))
+def test_image_edges_match_direct_search(case, precision):
+    widths, n, away = SMALL[case]
+    rng = np.random.default_rng(case)
+    cell = np.diag(widths) + np.array([[0, 0, 0], [0.1, 0, 0], [-0.2, 0.15, 0]]) * widths[0]
+    grid = np.stack(np.unravel_index(rng.permutation(12 ** 3)[:n], (12, 12, 12)), -1) / 12.0  # no close pairs
+    pos = (grid + rng.uniform(0, 0.02, (n, 3)) + rng.integers(-away, away + 1, (n, 3))) @ cell
+    eng = sg.Engine(sg.Model(MODEL), precision=precision)
+    eng.calc_efs([Frame(cell, pos, np.zeros(n, np.int32))])
+    ci, cj, d = eng.edges()
+    wi, wj, wd = direct_images(pos, cell)
+    np.testing.assert_array_equal(ci, wi)
+    np.testing.assert_array_equal(cj, wj)
+    assert np.abs(d - wd).max() < (1e-12 if precision == sg.FP64 else 5e-7)
