@@ -336,54 +336,6 @@ __device__ __forceinline__ void moment_batch(const Real* u, const Real* y, const
   }
 }
 
-// BF > 0: the basis size is the compile-time constant BF (= dm.B); BF = 0: runtime B <= kMaxB.
-template <int L, typename Real, bool DERIV, int BF = 0, typename Body>
-__device__ __forceinline__ void radial_loop(const DevModel<Real>& dm, const Real* s_coeff, const Real* s_scal,
-                                            int pair, Real r, Body&& body) {
-  constexpr int Lp = L + 1;
-  constexpr int NBM = BF ? BF : kMaxB;
-  const int B = BF ? BF : dm.B, C2 = dm.C * dm.C;
-  Real f0, fd0, f1, fd1;
-  envelope<Real>(r, dm.rmax, dm.poly, dm.cutoff_p, f0, fd0);
-  if (dm.split) envelope<Real>(r, dm.rang, dm.poly, dm.cutoff_p, f1, fd1);
-  else { f1 = f0; fd1 = fd0; }
-  f0 *= dm.scaling; fd0 *= dm.scaling; f1 *= dm.scaling; fd1 *= dm.scaling;
-  const bool angular_on = !(r >= dm.rang);
-  for (int k = 0; k < dm.K; ++k) {
-    Real Tv[NBM], Td[NBM];
-    int sb_prev = -1;
-#pragma unroll
-    for (int l = 0; l < Lp; ++l) {
-      if (l > 0 && !angular_on) break;
-      const int sb = scaling_block(dm.scaling_mode, k, l, Lp);
-      if (sb != sb_prev) {
-        const Real slope = s_scal[2 * sb * C2 + pair], shift = s_scal[(2 * sb + 1) * C2 + pair];
-        if (DERIV) cheb_raw<Real, NBM>(r, slope, shift, B, Tv, Td);
-        else cheb_raw_values<Real, NBM>(r, slope, shift, B, Tv);
-        sb_prev = sb;
-      }
-      const int mu = k * Lp + l;
-      const Real* c = s_coeff + mu * B;
-      Real cc[NBM];
-      load_coeff_row<Real, BF, NBM>(c, B, cc);
-      // two interleaved partial sums per dot product (shorter dependency chains)
-      Real a0 = Real(0), a1 = Real(0), d0 = Real(0), d1 = Real(0);
-#pragma unroll
-      for (int b = 0; b < NBM; ++b) {
-        if (b < B) {
-          if (b & 1) { a1 += cc[b] * Tv[b]; if (DERIV) d1 += cc[b] * Td[b]; }
-          else { a0 += cc[b] * Tv[b]; if (DERIV) d0 += cc[b] * Td[b]; }
-        }
-      }
-      const Real a = a0 + a1, ad = d0 + d1;
-      const Real f = l == 0 ? f0 : f1, fd = l == 0 ? fd0 : fd1;
-      const Real R = f * a;
-      const Real Rd = DERIV ? (fd * a + f * ad) : Real(0);
-      body(k, l, mu, R, Rd);
-    }
-  }
-}
-
 // Envelopes of an edge's l = 0 and l > 0 functions, times the model's scaling.
 template <typename Real>
 struct Envelopes { Real f0, fd0, f1, fd1; };

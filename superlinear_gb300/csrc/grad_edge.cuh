@@ -506,11 +506,12 @@ __global__ void __launch_bounds__(kWarp * grad_max_warps(L, sizeof(Real) == 4), 
           Pair<Real> T[NP], D[NP], DD[NP];
           cheb_pairs<Real, NP, true>(wv.xi, B, T, D);
           {
-            // DD_b = 4 D_b-1 + 2 xi DD_b-1 - DD_b-2
-            Real p2 = Real(0), p1 = Real(0);
+            // DD_b = 4 D_b-1 + 2 xi DD_b-1 - DD_b-2, from DD_2 = 4
+            Real p2 = Real(0), p1 = Real(4);
             DD[0] = {Real(0), Real(0)};
+            DD[1].x = p1;
 #pragma unroll
-            for (int b = 2; b < B; ++b) {
+            for (int b = 3; b < B; ++b) {
               const Real db = b & 1 ? D[b / 2].x : D[b / 2 - 1].y;  // D_b-1
               const Real v = Real(4) * db + (Real(2) * wv.xi * p1 - p2);
               p2 = p1; p1 = v;
@@ -531,9 +532,10 @@ __global__ void __launch_bounds__(kWarp * grad_max_warps(L, sizeof(Real) == 4), 
             const int m = k * Lp + l;
             Real cc[B];
             load_coeff_row<Real, B, B>(s_coeff + m * B, B, cc);
-            Pair<Real> sa{Real(0), Real(0)}, sd = sa, se = sa;
+            // (T_0 = 1, D_0 = DD_0 = DD_1 = 0 and D_1 = 1 need no product)
+            Pair<Real> sa{cc[0], cc[1] * T[0].y}, sd{Real(0), cc[1]}, se{Real(0), Real(0)};
 #pragma unroll
-            for (int p = 0; p < NP; ++p) {
+            for (int p = 1; p < NP; ++p) {
               const Pair<Real> c{cc[2 * p], cc[2 * p + 1]};
               sa = fma2(c, T[p], sa);
               sd = fma2(c, D[p], sd);

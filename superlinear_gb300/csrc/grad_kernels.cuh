@@ -304,16 +304,24 @@ __global__ void __launch_bounds__(128, PART == kGradWhole ? 3 : 4) grad_pass_ker
           for (int h = 0; h < H; ++h) { rw[2 * F + h] = Y[h]; rw[2 * F + H + h] = Yd[h]; }
           const Real* hj = effect_outer ? a.hsig + static_cast<size_t>(j) * F : nullptr;
           const Real* hdj = effect_outer ? a.hsigd + static_cast<size_t>(j) * F : nullptr;
-          radial_loop<L, Real, true, BF>(dm, s_coeff, s_scal, ti * C + tj, r, [&](int, int, int m_, Real R, Real Rd) {
-            const Real x0 = s_w0[ti * F + m_];
-            Real x3 = s_w1[tj * F + m_], x3d = Real(0);
-            if (effect_outer) {
-              x3 += s_wa[tj * F + m_] * hj[m_];
-              x3d = s_wa[tj * F + m_] * hdj[m_];
+          const Envelopes<Real> env = edge_envelopes<Real>(dm, r);
+#pragma unroll 1
+          for (int k = 0; k < K; ++k) {
+            Real R[Lp], Rd[Lp];
+            radial_channel<L, Real, true, BF>(dm, s_coeff, s_scal, ti * C + tj, r, env, k, R, Rd);
+#pragma unroll
+            for (int l = 0; l < Lp; ++l) {
+              const int m_ = k * Lp + l;
+              const Real x0 = s_w0[ti * F + m_];
+              Real x3 = s_w1[tj * F + m_], x3d = Real(0);
+              if (effect_outer) {
+                x3 += s_wa[tj * F + m_] * hj[m_];
+                x3d = s_wa[tj * F + m_] * hdj[m_];
+              }
+              rw[m_] = x0 * x3 * R[l];
+              rw[F + m_] = x0 * (x3d * R[l] + x3 * Rd[l] * rdot);
             }
-            rw[m_] = x0 * x3 * R;
-            rw[F + m_] = x0 * (x3d * R + x3 * Rd * rdot);
-          });
+          }
         }
         __syncwarp();
         // plain sums over the batch, compensated adds of the batch partials
