@@ -88,7 +88,7 @@ struct PassArgs {
                            // to finish zeroes both for the next launch
   int h_bulk;              // Effect outer pass: neighbours' h_j rows staged by bulk async copies (pass_h_bulk)
   int grid_mode;           // 0: all resident blocks; 1: the fewest blocks that keep the same atoms per warp
-  int block_warps;         // launch shape: warps per block (1 .. kPassWarps; 0 = kPassWarps); the kernel
+  int block_warps;         // launch shape: warps per block (1 .. kPassWarps; 0 = spread_warps); the kernel
                            // reads its block size from blockDim
   Real* keep;              // [keep_rows][kKeepBatches][2 F + H][32]: R, R', Y per edge (pass_keeps)
   int keep_rows;

@@ -1718,7 +1718,7 @@ bool Engine::take_params(const Model& m) {
   open_stage_ = -1;
   for (int q = 0; q < 4; ++q) {
     pass_blocks_[q] = pass_grid_[q] = pass_order_[q] = pass_stage_[q] = 0;
-    pass_wpb_[q] = 4;
+    pass_wpb_[q] = 0;
   }
   static_split_ = gate_split_ = -1;
   split_blocks_ = gate_split_blocks_[0] = gate_split_blocks_[1] = 0;

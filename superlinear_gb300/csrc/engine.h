@@ -101,7 +101,7 @@ class Engine {
     const bool split = (static_split_ > 0 && mode == (model_.gated ? 2 : 0)) || gate_split;
     if (split) shape4[0] = gate_split ? gate_split_blocks_[mode == 1 ? 0 : 1] : split_blocks_;
     shape4[2] = pass_order_[mode] + (split ? 4 : 0) + (pass_stage_[mode] ? 8 : 0);
-    shape4[3] = pass_wpb_[mode];
+    shape4[3] = pass_wpb_[mode] ? pass_wpb_[mode] : 4;
   }
   // sets the tile shape of pass `mode` as the autotuner would (blocks 0 = default, 3 or 4; grid 0
   // or 1; order 0, 1 or 2; stage 1 = h_j rows by bulk async copies, Effect outer pass): for
@@ -313,7 +313,7 @@ class Engine {
   int pass_grid_[4] = {0, 0, 0, 0};    // grid shape per pass mode (PassArgs::grid_mode)
   int pass_order_[4] = {0, 0, 0, 0};   // centre order per pass mode (PassArgs::atom_order)
   int pass_stage_[4] = {0, 0, 0, 0};   // h_j staging per pass mode (PassArgs::h_bulk; outer pass)
-  int pass_wpb_[4] = {4, 4, 4, 4};     // warps per block per pass mode (PassArgs::block_warps)
+  int pass_wpb_[4] = {0, 0, 0, 0};     // warps per block per pass mode (PassArgs::block_warps; 0: by the number of centres)
   template <typename Real> int launch_pass(int mode, PassArgs<Real> a, bool pdl);
   template <typename Real> int launch_shape(int mode, PassArgs<Real> a, int blocks, bool pdl);
   static constexpr int kWorkInts = 32;  // work_: (next centre, warps done) per pass mode (< 16)

@@ -91,6 +91,10 @@ GradLaunch grad_pass_config_l(int mode, const DevModel<Real>& dm, int natoms, in
   if (best_warps == 0 || per_sm < 1)
     throw std::runtime_error("gradient kernel does not fit on an SM (shared memory " + std::to_string(bytes(1, cfg.acc_cols)) + " B)");
   cfg.warps = best_warps;
+  if (natoms <= per_sm * best_warps * sm_count) {
+    cfg.warps = spread_warps(natoms, best_warps, sm_count);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, cfg.warps * kWarp, bytes(cfg.warps, cfg.acc_cols));
+  }
   cfg.block = cfg.warps * kWarp;
   cfg.smem = bytes(cfg.warps, cfg.acc_cols);
   const int need = std::max(1, (natoms + cfg.warps - 1) / cfg.warps);
@@ -136,6 +140,12 @@ GradLaunch warp_launch(Kern kern, int max_warps, int natoms, int sm_count, Bytes
     }
   }
   if (best == 0) return GradLaunch{};
+  if (natoms <= best * sm_count) {
+    int blocks = 0;
+    cfg.warps = spread_warps(natoms, cfg.warps, sm_count);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, cfg.warps * kWarp, bytes(cfg.warps));
+    cfg.grid = blocks * sm_count;
+  }
   cfg.block = cfg.warps * kWarp;
   cfg.smem = bytes(cfg.warps);
   cfg.grid = std::max(1, std::min((natoms + cfg.warps - 1) / cfg.warps, cfg.grid));

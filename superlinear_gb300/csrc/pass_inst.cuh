@@ -18,9 +18,12 @@ int launch_one(const PassArgs<Real>& a, int sm_count, cudaStream_t stream, bool 
   const auto& dm = a.dm;
   const bool h_bulk = MODE == kModeOuterBulk && h_rows_bulk_ok<Real>(dm.F);
   // warps per block: at most the compiled launch bound
-  const int wpb = a.block_warps > 0 && a.block_warps < kPassWarps ? a.block_warps : kPassWarps;
-  const size_t smem = sizeof(Real) * (efs_table_size(dm.C, dm.F, dm.B, dm.nblk) +
-                                      wpb * pass_warp_stride<Real>(L, dm.M, dm.K, dm.prog_parts, h_bulk));
+  int wpb = a.block_warps > 0 && a.block_warps < kPassWarps ? a.block_warps : kPassWarps;
+  auto bytes = [&](int w) {
+    return sizeof(Real) * (efs_table_size(dm.C, dm.F, dm.B, dm.nblk) +
+                           w * pass_warp_stride<Real>(L, dm.M, dm.K, dm.prog_parts, h_bulk));
+  };
+  size_t smem = bytes(wpb);
   static size_t configured = 0;
   if (smem > configured) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -30,6 +33,12 @@ int launch_one(const PassArgs<Real>& a, int sm_count, cudaStream_t stream, bool 
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, wpb * kWarp, smem);
   if (per_sm < 1) throw std::runtime_error("pass kernel does not fit on an SM (shared memory " + std::to_string(smem) + " B)");
+  // no block size chosen and every centre resident at once: spread them
+  if (a.block_warps == 0 && a.natoms <= per_sm * wpb * sm_count) {
+    wpb = spread_warps(a.natoms, kPassWarps, sm_count);
+    smem = bytes(wpb);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, wpb * kWarp, smem);
+  }
   const int need = (a.natoms + wpb - 1) / wpb;
   const int resident = per_sm * sm_count;
   int grid = std::max(1, std::min(need, resident));

@@ -47,6 +47,17 @@ GradLaunch grad_moment_config_l(int mode, const DevModel<float>& dm, int natoms,
 template <int L>
 int launch_grad_moment_l(int mode, const GradArgs<float>& a, const GradLaunch& cfg, cudaStream_t stream);
 
+// Warps per block (`most` or 2) of a launch whose n warps, one centre each, are resident at once: what
+// leaves the fullest SM with fewer warps, an odd block counted as the next even one (it leaves one of
+// the SM's four schedulers a warp short).  884 centres in blocks of 4 put 8 warps on some of 152 SMs
+// and 4 on the others, in blocks of 2 at most 6: FP64 per-edge gradient 509 -> 481 and 465 -> 440 us, gate
+// forward 229 -> 158 us (blocks of 3: 561, 524 and 193), per-atom gradient parts 317 -> 269 and 300 -> 252 us;
+// FP32 passes, bound by latency there, gain 0 to 4%.
+inline int spread_warps(int n, int most, int sm_count) {
+  auto load = [&](int w) { return ((n + w - 1) / w + sm_count - 1) / sm_count * ((w + 1) / 2 * 2); };
+  return most > 2 && load(2) < load(most) ? 2 : most;
+}
+
 // Launches atom_pass_kernel<L, Real, mode, Kahan = (Real is float)> sized as a multiple of the SM
 // count, with the register budget of `blocks` resident blocks per SM (3 or 4; 0 = the default),
 // as a programmatic dependent launch when pdl is set (the kernel stages its model tables while
