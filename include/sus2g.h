@@ -127,16 +127,16 @@ int sus2g_engine_set_moment_mma(sus2g_engine engine, int enabled);
  * readout / adjoint, and the per-edge adjoint -- through device moment arrays, and the Effect
  * gate passes as two each (edge->moment forward, then the per-atom gate graph and gate-signal
  * projection; the per-atom gate-signal adjoint gather and gate graph reverse, then the per-edge
- * adjoint), instead of one fused kernel per pass (enabled = 1; default 0; the autotuner chooses
- * per pass).  The same
- * arithmetic in the same order as the fused pass, in separately compiled kernels: results agree
- * to FP32 rounding (bit for bit on the Static models tested).  No counterpart in the reference (a
- * launch-shape choice). */
+ * adjoint), instead of one fused kernel per pass (enabled = 1: always; 0: never).  Without this
+ * call the number of centres of the evaluation decides, or the autotuner per pass once it has run; a
+ * pinned pass shape runs fused.  Results of the two forms agree to FP32 rounding; each repeats bit
+ * for bit.  No counterpart in the reference (a launch-shape choice). */
 int sus2g_engine_set_static_split(sus2g_engine engine, int enabled);
 /* The outer and gate reverse parameter-gradient passes (sus2g_engine_combination_grad and the
  * trainer) as two kernels each -- the per-atom part (forward with tangents, readout seeds, reverse
  * sweep) writing the moment adjoints, then the per-edge parameter contributions -- instead of one
- * (enabled = 1, the default; basis size 8).  The per-warp gradient slices then receive their terms
+ * (enabled = 1, the default; basis size 8; FP32 engines run the per-atom part as a moment and a graph
+ * kernel, the gate forward pass too).  The gradient slices then receive their terms
  * in another order: results agree to the rounding of the precision and repeat bit for bit.  No
  * counterpart in the reference (a kernel-shape choice). */
 int sus2g_engine_set_grad_split(sus2g_engine engine, int enabled);
