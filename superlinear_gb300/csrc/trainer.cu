@@ -609,11 +609,15 @@ class Trainer {
     bind_edges();
   }
 
+  void drop_graph() {
+    if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
+    if (graph_) { cudaGraphDestroy(graph_); graph_ = nullptr; }
+  }
+
   // The edge set of the fixed frames is built once, and again only when the engine was used for
   // other geometry in between (which also invalidates a captured graph).
   void bind_edges() {
-    if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
-    if (graph_) { cudaGraphDestroy(graph_); graph_ = nullptr; }
+    drop_graph();
     for (int attempt = 0;; ++attempt) {
       try {
         eng_.build_edges(nframes_, natoms_list_.data(), cells_.data(), pos_.as<double>(), types_.as<int>());
@@ -627,8 +631,7 @@ class Trainer {
   }
 
   ~Trainer() {
-    if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
-    if (graph_) cudaGraphDestroy(graph_);
+    drop_graph();
     if (host_scalars_) cudaFreeHost(host_scalars_);
   }
 
@@ -676,6 +679,8 @@ class Trainer {
   // Loss and gradient at the parameters already in the engine; results stay on the device.
   void eval_device() {
     if (eng_.edge_generation() != generation_) bind_edges();
+    // a captured evaluation holds the radial scaling by value (DevModel, a kernel argument)
+    if (graph_exec_ && graph_scaling_ != eng_.model().scaling) drop_graph();
     cudaStream_t s = eng_.stream();
     if (!use_graph_) {
       enqueue_eval();
@@ -688,6 +693,7 @@ class Trainer {
       enqueue_eval();
       TRAIN_CUDA(cudaStreamEndCapture(s, &graph_));
       TRAIN_CUDA(cudaGraphInstantiate(&graph_exec_, graph_, 0));
+      graph_scaling_ = eng_.model().scaling;
       ++graph_builds_;
       return;
     }
@@ -1266,6 +1272,7 @@ class Trainer {
   bool use_graph_ = true;
   cudaGraph_t graph_ = nullptr;
   cudaGraphExec_t graph_exec_ = nullptr;
+  double graph_scaling_ = 0.0;  // the radial scaling it was captured with
   int graph_builds_ = 0;
   unsigned long long generation_ = 0;
 };
