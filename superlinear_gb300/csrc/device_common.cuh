@@ -32,6 +32,11 @@ template <typename T> struct Vec4;
 template <> struct Vec4<float> { using type = EdgeF; };
 template <> struct Vec4<double> { using type = EdgeD; };
 
+// A component of a caller's edge in FP32.  One past that range (an accepted edge may be 1e150 long) is
+// brought into it: with the infinite distance beside it the edge's direction is then zero and its
+// terms are exact zeros, where an infinite component would make NaN of them.
+__device__ __forceinline__ float edge_component(double x) { return fminf(fmaxf(static_cast<float>(x), -1e38f), 1e38f); }
+
 // Per-atom graph program of one pass: the rank contraction and the product graph, forward and
 // reverse, as steps of lane-balanced work.  A step adds to one node array (v forward, adj reverse)
 //     T[target] += sum over a term list of c * X[a] * v[b]     (X = v forward, adj reverse)

@@ -844,11 +844,15 @@ __global__ void k_scatter_user_edges(const int* ei, const int* ej, const double*
   const int p = row[i] + atomicSub(cursor + i, 1) - 1;
   nbr[p] = j;
   typename Vec4<Real>::type v;
-  v.x = Real(x); v.y = Real(y); v.z = Real(z);
   // FP32 records: the distance from the rounded r^2 (an FP32 square root; the FP64 one costs tens
   // of FP64-pipe instructions)
-  if constexpr (sizeof(Real) == 4) v.w = sqrtf(static_cast<float>(r2));
-  else v.w = sqrt(r2);
+  if constexpr (sizeof(Real) == 4) {
+    v.x = edge_component(x); v.y = edge_component(y); v.z = edge_component(z);
+    v.w = sqrtf(static_cast<float>(r2));
+  } else {
+    v.x = x; v.y = y; v.z = z;
+    v.w = sqrt(r2);
+  }
   d4[p] = v;
   // Order key: neighbour, then the caller's edge index (unique, deterministic).
   key[p] = (static_cast<unsigned long long>(j) << 32) | static_cast<unsigned long long>(e & 0xffffffffLL);

@@ -109,7 +109,7 @@ __global__ void k_na_pack(int natoms, int nall, int species, const int* types, c
   const double x = vec[3 * t], y = vec[3 * t + 1], z = vec[3 * t + 2];
   const double r2 = x * x + y * y + z * z;
   if (!(r2 > 0) || !isfinite(r2)) record_error(error, kErrBadDistance);
-  d4[t] = EdgeF{static_cast<float>(x), static_cast<float>(y), static_cast<float>(z), static_cast<float>(sqrt(r2))};
+  d4[t] = EdgeF{edge_component(x), edge_component(y), edge_component(z), static_cast<float>(sqrt(r2))};
 }
 
 // Exclusive scan of the n = nall + 1 incoming-edge counts into in_row (one block of kScanThreads
