@@ -538,11 +538,9 @@ int sus2g_efs_edges_host(sus2g_engine e, int nowned, int nall, const int* types,
     for (int i = 0; i < nall; ++i) need(types[i] >= 0 && types[i] < eng.model().C, "atom species index out of range");
     cudaStream_t s = eng.stream();
     cuda(cudaSetDevice(eng.device()), "cudaSetDevice");
-    // outputs [energy][virial 6][forces 3 nall][site nowned] come back in one transfer
-    const size_t outs = 7 + 3 * static_cast<size_t>(nall) + static_cast<size_t>(nowned);
-    Slot typ(eng, 0, sizeof(int) * nall), di(eng, 1, sizeof(int) * nedges), dj(eng, 2, sizeof(int) * nedges),
-        dd(eng, 3, sizeof(double) * 3 * nedges), out(eng, 4, sizeof(double) * outs);
-    if (nall) cuda(cudaMemcpyAsync(typ.p, types, sizeof(int) * nall, cudaMemcpyHostToDevice, s), "types copy");
+    // the edges in slots that no evaluation holds after its call: a list that is refused leaves the
+    // engine's geometry whole, the types that it keeps a pointer to (slots 0 and 1) included
+    Slot di(eng, 5, sizeof(int) * nedges), dj(eng, 6, sizeof(int) * nedges), dd(eng, 7, sizeof(double) * 3 * nedges);
     if (nedges) {
       cuda(cudaMemcpyAsync(di.p, ei, sizeof(int) * nedges, cudaMemcpyHostToDevice, s), "edge copy");
       cuda(cudaMemcpyAsync(dj.p, ej, sizeof(int) * nedges, cudaMemcpyHostToDevice, s), "edge copy");
@@ -552,6 +550,10 @@ int sus2g_efs_edges_host(sus2g_engine e, int nowned, int nall, const int* types,
     // looks only at edges that the device does not pass, for the verdict and its message
     if (!eng.edges_plain(nowned, nall, nedges, di.as<int>(), dj.as<int>(), dd.as<double>()))
       check_edges(eng, nowned, nall, types, nedges, ei, ej, d);
+    // outputs [energy][virial 6][forces 3 nall][site nowned] come back in one transfer
+    const size_t outs = 7 + 3 * static_cast<size_t>(nall) + static_cast<size_t>(nowned);
+    Slot typ(eng, 0, sizeof(int) * nall), out(eng, 4, sizeof(double) * outs);
+    if (nall) cuda(cudaMemcpyAsync(typ.p, types, sizeof(int) * nall, cudaMemcpyHostToDevice, s), "types copy");
     double* o = out.as<double>();
     eng.set_edges(nowned, nall, typ.as<int>(), nedges, di.as<int>(), dj.as<int>(), dd.as<double>());
     eng.efs(o, forces ? o + 7 : nullptr, o + 1, site_energy ? o + 7 + 3 * static_cast<size_t>(nall) : nullptr);
