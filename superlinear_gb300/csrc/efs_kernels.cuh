@@ -294,6 +294,38 @@ __device__ __forceinline__ void cols_to_rows(Real* rows, const Real* stage, int 
   __syncwarp();
 }
 
+// The F columns of a row-major per-edge array [n][F] summed over the rows: 32 / W groups of
+// W = F / 4 lanes take the rows in turn, a lane reading one 16-byte unit of its row, four rows in
+// flight; the groups' sums are added in group order.  put(c, t) on lane c < W receives columns
+// 4 c .. 4 c + 3.  For rows of whole units (row_groups_ok).
+__host__ __device__ constexpr bool row_groups_ok(int F) { return F % 4 == 0 && F / 4 <= kWarp; }
+template <typename Put>
+__device__ __forceinline__ void row_group_sums(const float* rows, int F, int n, int lane, Put&& put) {
+  const int nc = F / 4, groups = kWarp / nc, grp = lane / nc, c = lane - grp * nc;
+  const float4* src = reinterpret_cast<const float4*>(rows) + c;
+  float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (grp < groups) {
+    for (int e = grp; e < n; e += 4 * groups) {
+      float4 w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (e + u * groups < n) w[u] = src[static_cast<size_t>(e + u * groups) * nc];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (e + u * groups < n) { t.x += w[u].x; t.y += w[u].y; t.z += w[u].z; t.w += w[u].w; }
+    }
+  }
+  const float4 own = t;
+  for (int q = 1; q < groups; ++q) {
+    const int from = min(lane + q * nc, kWarp - 1);
+    t.x += __shfl_sync(0xffffffffu, own.x, from);
+    t.y += __shfl_sync(0xffffffffu, own.y, from);
+    t.z += __shfl_sync(0xffffffffu, own.z, from);
+    t.w += __shfl_sync(0xffffffffu, own.w, from);
+  }
+  if (lane < nc) put(c, t);
+}
+
 // Four consecutive values of a 16-byte aligned shared-memory column as two pairs.
 template <typename Real>
 __device__ __forceinline__ void load_quad(const Real* p, Pair<Real>& a, Pair<Real>& b) {
@@ -878,7 +910,10 @@ __global__ void __launch_bounds__(kPassWarps * kWarp, MINB) atom_pass_kernel(Pas
       readout_seeds<Real>(a, atom, ti, v, adj, lane);
     } else {
       // ---------------- gate reverse: gather hbar, project, load gate values ----------------
-      if (!a.hbar_atom && F <= 2 * kWarp) {
+      if (sizeof(Real) == 4 && !a.hbar_atom && row_groups_ok(F)) {  // in the split pass's order (hbar_sum_kernel)
+        row_group_sums(reinterpret_cast<const float*>(a.hcontrib + (size_t)e0 * F), F, e1 - e0, lane,
+                       [&](int c, float4 t) { reinterpret_cast<float4*>(hbar)[c] = t; });
+      } else if (!a.hbar_atom && F <= 2 * kWarp) {
         column_sums_2<Real>(a.hcontrib + (size_t)e0 * F, F, e1 - e0, hbar, lane);
       } else {
         for (int mu = lane; mu < F; mu += kWarp) {

@@ -12,7 +12,9 @@
 // and a block's 16 (or 32) warps share the target lists of a step, longest first, with a barrier per step.
 // Only the nodes of this pass take slots, and an adjoint takes its node's slot when the reverse
 // never reads the value, which keeps two blocks per SM at L4/K8.  Every list is summed chunk by
-// chunk in run_prog's order, so that split and fused passes give the same bits.
+// chunk in run_prog's order and the gate-signal adjoints as in the fused pass, so that split and fused
+// passes give the same bits: the number of centres chooses between them, and a frame's results
+// must not depend on the frames it is evaluated with.
 // Effect L4/K8/R2/O3, 110,592 atoms: the outer pass's graph about 1.0 ms one centre a warp, 0.9 ms
 // two, 0.2 ms here; 8,000 atoms 78 -> 41 us (one wave, cold program).
 #pragma once
@@ -200,9 +202,8 @@ __global__ void __launch_bounds__(2 * kGraphWarps * kWarp, 1) graph_block_kernel
 }
 
 // The gate-signal adjoint of every centre: the F contributions of its edges (stored at the reverse
-// edges by the outer pass) summed per column, warp per centre.  32 / W groups of W lanes take the
-// edges in turn, a lane reading one 16-byte unit of its row, four rows in flight; the groups'
-// sums are added in group order.  Bound by the read of the [E][F] contributions.
+// edges by the outer pass) summed per column, warp per centre, in the fused gate reverse pass's order
+// (row_group_sums).  Bound by the read of the [E][F] contributions.
 static __global__ void __launch_bounds__(256) hbar_sum_kernel(PassArgs<float> a) {
   const int F = a.dm.F, lane = warp_lane();
   const int atom = static_cast<int>((static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kWarp);
@@ -210,34 +211,13 @@ static __global__ void __launch_bounds__(256) hbar_sum_kernel(PassArgs<float> a)
   pdl_wait();
   if (atom >= a.natoms) return;
   const int e0 = a.row[atom], n = a.row_end[atom] - e0;
+  const float* rows = a.hcontrib + static_cast<size_t>(e0) * F;
   float* out = a.hbar + static_cast<size_t>(atom) * F;
-  if (F % 4 != 0 || F / 4 > kWarp) {
-    for (int mu = lane; mu < F; mu += kWarp) out[mu] = column_sum<float>(a.hcontrib + static_cast<size_t>(e0) * F + mu, F, n);
-    return;
+  if (row_groups_ok(F)) {
+    row_group_sums(rows, F, n, lane, [&](int c, float4 t) { reinterpret_cast<float4*>(out)[c] = t; });
+  } else {
+    for (int mu = lane; mu < F; mu += kWarp) out[mu] = column_sum<float>(rows + mu, F, n);
   }
-  const int nc = F / 4, groups = kWarp / nc, grp = lane / nc, c = lane - grp * nc;
-  const float4* src = reinterpret_cast<const float4*>(a.hcontrib + static_cast<size_t>(e0) * F) + c;
-  float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (grp < groups) {
-    for (int e = grp; e < n; e += 4 * groups) {
-      float4 w[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (e + u * groups < n) w[u] = src[static_cast<size_t>(e + u * groups) * nc];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (e + u * groups < n) { t.x += w[u].x; t.y += w[u].y; t.z += w[u].z; t.w += w[u].w; }
-    }
-  }
-  const float4 own = t;
-  for (int q = 1; q < groups; ++q) {
-    const int from = min(lane + q * nc, kWarp - 1);
-    t.x += __shfl_sync(0xffffffffu, own.x, from);
-    t.y += __shfl_sync(0xffffffffu, own.y, from);
-    t.z += __shfl_sync(0xffffffffu, own.z, from);
-    t.w += __shfl_sync(0xffffffffu, own.w, from);
-  }
-  if (lane < nc) reinterpret_cast<float4*>(out)[c] = t;
 }
 
 }  // namespace sus2g
