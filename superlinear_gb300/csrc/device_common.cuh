@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "largest_per_device.h"
+
 namespace sus2g {
 
 constexpr int kWarp = 32;
@@ -239,6 +241,20 @@ inline cudaError_t launch_kernel(bool pdl, void (*kernel)(P...), dim3 grid, dim3
   cfg.attrs = pdl ? attr : nullptr;
   cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
+}
+
+// Raises a kernel's dynamic shared-memory limit on the current device to `bytes` (`largest`: one object
+// per kernel).  The limit belongs to the kernel, for every engine and host thread of the process: set to
+// each launch's own size it could fall between another thread's setting and its larger launch,
+// which is then refused.
+template <typename... P>
+inline cudaError_t allow_shared_memory(void (*kernel)(P...), size_t bytes, LargestPerDevice& largest) {
+  int device = 0;
+  const cudaError_t err = cudaGetDevice(&device);
+  if (err != cudaSuccess) return err;
+  return static_cast<cudaError_t>(largest.raise(device, bytes, [&](size_t n) {
+    return static_cast<int>(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(n)));
+  }));
 }
 
 // kernel<<<grid, block, smem, stream>>>(args...) at the given scheduling priority (a stream

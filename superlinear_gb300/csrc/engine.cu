@@ -2573,9 +2573,8 @@ void Engine::run_grad(const double* ew, const double* fw, const double* sw, doub
         const int blocks = std::max(1, std::min(nslots, (ncentres_ + kGwChunk - 1) / kGwChunk));
         const size_t smem = sizeof(Real) * kGwChunk * 2 * (m.F + m.Q);
         if (smem > 200 * 1024) throw Error(3, "gate weight gradient: radial functions + gate scalars exceed the shared-memory staging");
-        if (smem > 48 * 1024)
-          SUS2G_CUDA(cudaFuncSetAttribute(k_gate_weight_grad<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(smem)));
+        static LargestPerDevice allowed;
+        SUS2G_CUDA(allow_shared_memory(k_gate_weight_grad<Real>, smem, allowed));
         k_gate_weight_grad<Real><<<blocks, kGwThreads, smem, s>>>(ncentres_, m.F, m.Q, m.M, dm.gate_nodes,
                                                                   lh_atom_.as<double>(), gmom_.as<Real>(),
                                                                   gmomd_.as<Real>(), slots_.as<double>(), P, gw_off);

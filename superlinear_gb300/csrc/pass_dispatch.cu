@@ -57,18 +57,15 @@ int launch_graph(const PassArgs<float>& a, int sm_count, cudaStream_t s) {
   const BlockProg& g = GM == 0 ? a.dm.outer.block : a.dm.gate.block;
   auto kern = graph_block_kernel<GM>;
   const size_t smem = graph_block_bytes(g.nslots, a.dm.F, a.dm.S);
-  static size_t configured = 0;
-  if (smem > configured) {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (err != cudaSuccess) throw std::runtime_error(std::string("graph kernel shared memory: ") + cudaGetErrorString(err));
-    configured = smem;
-  }
+  static LargestPerDevice allowed;
+  cudaError_t err = allow_shared_memory(kern, smem, allowed);
+  if (err != cudaSuccess) throw std::runtime_error(std::string("graph kernel shared memory: ") + cudaGetErrorString(err));
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, g.warps * kWarp, smem);
   if (per_sm < 1) throw std::runtime_error("graph kernel does not fit on an SM");
   const int need = (a.natoms + kGraphAtoms - 1) / kGraphAtoms;
   kern<<<std::max(1, std::min(need, per_sm * sm_count)), g.warps * kWarp, smem, s>>>(a);
-  cudaError_t err = cudaGetLastError();
+  err = cudaGetLastError();
   if (err != cudaSuccess) throw std::runtime_error(std::string("graph kernel launch: ") + cudaGetErrorString(err));
   return 1;
 }
@@ -167,7 +164,8 @@ GradLaunch grad_graph_config(int mode, const DevModel<float>& dm, int natoms, in
   cfg.warps = g.warps;
   cfg.block = g.warps * kWarp;
   cfg.smem = dual_block_bytes(g.nslots, dm.F, dm.S);
-  check_gradient(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem)), "gradient graph shared memory");
+  static LargestPerDevice allowed[3];
+  check_gradient(allow_shared_memory(kern, cfg.smem, allowed[mode]), "gradient graph shared memory");
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, cfg.block, cfg.smem);
   if (per_sm < 1) throw std::runtime_error("gradient graph kernel does not fit on an SM");
@@ -187,13 +185,15 @@ int launch_lhm_sum(const GradArgs<float>& a, int Lp, cudaStream_t s) {
   return 1;
 }
 GradLaunch grad_gate_weight_config(const DevModel<float>& dm, int natoms, int sm_count) {
-  auto kern = gate_weight_tile(dm.F, dm.Q) == 4 ? grad_gate_weight_kernel<4> : grad_gate_weight_kernel<2>;
+  const int tile = gate_weight_tile(dm.F, dm.Q);
+  auto kern = tile == 4 ? grad_gate_weight_kernel<4> : grad_gate_weight_kernel<2>;
   GradLaunch cfg;
   cfg.warps = kGwThreads32 / kWarp;
   cfg.block = kGwThreads32;
   cfg.smem = gate_weight_bytes(dm.F, dm.Q);
   if (cfg.smem > 227 * 1024) throw std::runtime_error("gate weight gradient: radial functions + gate scalars exceed the shared-memory staging");
-  check_gradient(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.smem)), "gate weight shared memory");
+  static LargestPerDevice allowed[2];
+  check_gradient(allow_shared_memory(kern, cfg.smem, allowed[tile == 4]), "gate weight shared memory");
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, cfg.block, cfg.smem);
   cfg.grid = std::max(1, std::min((natoms + kDualAtoms - 1) / kDualAtoms, std::max(1, per_sm) * sm_count));

@@ -24,12 +24,9 @@ int launch_one(const PassArgs<Real>& a, int sm_count, cudaStream_t stream, bool 
                            w * pass_warp_stride<Real>(L, dm.M, dm.K, dm.prog_parts, h_bulk));
   };
   size_t smem = bytes(wpb);
-  static size_t configured = 0;
-  if (smem > configured) {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (err != cudaSuccess) throw std::runtime_error(std::string("pass shared memory: ") + cudaGetErrorString(err));
-    configured = smem;
-  }
+  static LargestPerDevice allowed;
+  cudaError_t err = allow_shared_memory(kern, smem, allowed);
+  if (err != cudaSuccess) throw std::runtime_error(std::string("pass shared memory: ") + cudaGetErrorString(err));
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, wpb * kWarp, smem);
   if (per_sm < 1) throw std::runtime_error("pass kernel does not fit on an SM (shared memory " + std::to_string(smem) + " B)");
@@ -49,7 +46,7 @@ int launch_one(const PassArgs<Real>& a, int sm_count, cudaStream_t stream, bool 
     grid = std::max(1, (need + rounds - 1) / rounds);
   }
   if (a.natoms == 0) return 0;
-  cudaError_t err = launch_kernel(pdl, kern, dim3(grid), dim3(wpb * kWarp), smem, stream, a);
+  err = launch_kernel(pdl, kern, dim3(grid), dim3(wpb * kWarp), smem, stream, a);
   if (err != cudaSuccess) throw std::runtime_error(std::string("pass launch: ") + cudaGetErrorString(err));
   return 1;
 }
