@@ -64,6 +64,9 @@ int sus2g_model_save(sus2g_model model, const char* path);
  * parameters; call sus2g_engine_update_params after sus2g_model_set_params. */
 int sus2g_engine_create(sus2g_model model, int device, int precision, sus2g_engine* out);
 void sus2g_engine_free(sus2g_engine engine);
+/* Takes the model's current parameters and scaling; the engine is then as a new one for the model:
+ * settings at their defaults, its own stream, no evaluated layout.  Waits for the work queued on the
+ * device; a stream that the engine was given need not exist any more. */
 int sus2g_engine_update_params(sus2g_engine engine, sus2g_model model);
 /* Use a caller CUDA stream (cudaStream_t passed as void*; NULL restores the engine's own). */
 int sus2g_engine_set_stream(sus2g_engine engine, void* cuda_stream);

@@ -1705,8 +1705,9 @@ void Engine::upload_block_programs(bool dual) {
 bool Engine::take_params(const Model& m) {
   if (!model_.same_structure(m)) return false;
   SUS2G_CUDA(cudaSetDevice(device_));
-  SUS2G_CUDA(cudaStreamSynchronize(stream_));
-  SUS2G_CUDA(cudaStreamSynchronize(aux_stream_));
+  // what was queued on any stream that the engine was given may still read the tables (the caller's
+  // stream itself may be gone by now, so it is not named here)
+  SUS2G_CUDA(cudaDeviceSynchronize());
   rev_pending_ = false;
   reset_step_graph();
   stream_ = own_stream_;
