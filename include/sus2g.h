@@ -153,14 +153,15 @@ int sus2g_engine_set_grad_split(sus2g_engine engine, int enabled);
  * 3 gate reverse; 0 for passes the model does not run), ms8[2 mode + budget - 3] (may be NULL) =
  * milliseconds per launch of the budget's fastest shape. */
 int sus2g_engine_autotune(sus2g_engine engine, int reps, int* blocks4, double* ms8);
-/* Tile shape of a per-atom pass (mode 0 Static, 1 gate forward, 2 outer, 3 gate reverse) as the
- * autotuner left it: shape4 = {register budget in resident blocks per SM (0 = default; for a
+/* Tile shape of a per-atom pass (mode 0 Static, 1 gate forward, 2 outer, 3 gate reverse) on the
+ * layout of the engine's last evaluation -- pinned, as the autotuner left it, or as the number of
+ * centres chose it: shape4 = {register budget in resident blocks per SM (0 = default; for a
  * split pass, that of its per-edge kernels, which the autotuner tunes separately), grid
  * (0 all resident blocks, 1 the fewest blocks with the same centres per warp), centre order
  * (0 grid-strided, 1 contiguous runs per warp, 2 taken from a device counter as warps finish;
- * plus 4 when the Static pass runs as three kernels, sus2g_engine_set_static_split; plus 8 when
+ * plus 4 when the pass runs split at the per-atom boundary, sus2g_engine_set_static_split; plus 8 when
  * the Effect outer pass brings the neighbours' gate-signal rows into shared memory by 1-D bulk
- * asynchronous copies, one 32-edge batch ahead), warps per block (2 or 4 from the autotuner)}.  No counterpart in the
+ * asynchronous copies, one 32-edge batch ahead), warps per block (2 or 4 unless pinned)}.  No counterpart in the
  * reference (its kernel has no launch shape). */
 int sus2g_engine_pass_shape(sus2g_engine engine, int mode, int* shape4);
 /* Sets the tile shape of a per-atom pass as the autotuner would: blocks = register budget (0

@@ -1725,6 +1725,7 @@ bool Engine::take_params(const Model& m) {
     pass_blocks_[q] = pass_grid_[q] = pass_order_[q] = pass_stage_[q] = 0;
     pass_wpb_[q] = 0;
   }
+  std::fill(std::begin(ran_warps_), std::end(ran_warps_), 0);
   static_split_ = gate_split_ = -1;
   split_blocks_ = gate_split_blocks_[0] = gate_split_blocks_[1] = 0;
   gate_ran_split_ = false;
@@ -2626,7 +2627,7 @@ int Engine::static_pass_external(int natoms, const int* types, const int* row, c
   a.site_energy = site;
   a.virial = vir;
   a.error = error;
-  return launch_atom_pass<float>(model_.L, kModeStatic, a, sm_count_, stream_);
+  return launch_atom_pass<float>(model_.L, kModeStatic, a, sm_count_, stream_) ? 1 : 0;
 }
 
 void Engine::efs(double* d_energy, double* d_forces, double* d_virial, double* d_site) {
@@ -2747,7 +2748,24 @@ int Engine::launch_shape(int mode, PassArgs<Real> a, int blocks, bool pdl) {
     buf.ensure(sizeof(Real) * pass_keep_values(model_.L, model_.F) * std::max(1, a.keep_rows));
     a.keep = buf.as<Real>();
   }
-  return launch_atom_pass<Real>(model_.L, mode, a, sm_count_, stream_, blocks, pdl);
+  const int warps = launch_atom_pass<Real>(model_.L, mode, a, sm_count_, stream_, blocks, pdl);
+  if (warps) ran_warps_[mode] = warps;
+  return warps ? 1 : 0;
+}
+
+void Engine::pass_shape(int mode, int* shape4) const {
+  const bool gate = mode == kModeGateForward || mode == kModeGateReverse;
+  const bool runs = mode == kModeStatic ? !model_.gated : model_.gated;
+  const bool fp32 = precision_ == kFP32;
+  const bool split = runs && (gate ? (fp32 ? use_gate_split<float>() : use_gate_split<double>())
+                                   : (fp32 ? use_static_split<float>() : use_static_split<double>()));
+  int kernel = mode;  // whose launch has the pass's block size
+  if (split) kernel = mode == kModeStatic ? kModeStaticFwd : mode == kModeOuter ? kModeOuterFwd
+                                          : mode == kModeGateForward ? kModeGateFwdEdges : kModeGateRevEdges;
+  shape4[0] = !split ? pass_blocks_[mode] : gate ? gate_split_blocks_[mode == kModeGateForward ? 0 : 1] : split_blocks_;
+  shape4[1] = pass_grid_[mode];
+  shape4[2] = pass_order_[mode] + (split ? 4 : 0) + (pass_stage_[mode] ? 8 : 0);
+  shape4[3] = pass_wpb_[mode] ? pass_wpb_[mode] : ran_warps_[kernel] ? ran_warps_[kernel] : kPassWarps;
 }
 
 // Pass-kernel autotuner: on the current layout (the last evaluation's edges), times each pass the

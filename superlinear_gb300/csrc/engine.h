@@ -92,17 +92,11 @@ class Engine {
   // register budget (3 or 4 resident blocks per SM; 0 for passes the model does not run),
   // ms_out[2 mode + (budget - 3)] = the timed milliseconds per launch.
   void autotune(int reps, int* blocks_out, double* ms_out);
-  // tile shape of pass `mode` (0 Static, 1 gate forward, 2 outer, 3 gate reverse): register budget
-  // (resident blocks per SM; 0 = default), grid shape, centre order + 4 x split (Static pass run
-  // as three kernels) + 8 x h_j staging by bulk async copies, warps per block
-  void pass_shape(int mode, int* shape4) const {
-    shape4[0] = pass_blocks_[mode]; shape4[1] = pass_grid_[mode];
-    const bool gate_split = model_.gated && (mode == 1 || mode == 3) && gate_split_ > 0;
-    const bool split = (static_split_ > 0 && mode == (model_.gated ? 2 : 0)) || gate_split;
-    if (split) shape4[0] = gate_split ? gate_split_blocks_[mode == 1 ? 0 : 1] : split_blocks_;
-    shape4[2] = pass_order_[mode] + (split ? 4 : 0) + (pass_stage_[mode] ? 8 : 0);
-    shape4[3] = pass_wpb_[mode] ? pass_wpb_[mode] : 4;
-  }
+  // tile shape of pass `mode` (0 Static, 1 gate forward, 2 outer, 3 gate reverse) on the last
+  // evaluation's layout: register budget (resident blocks per SM; 0 = default), grid shape, centre
+  // order + 4 x split at the per-atom boundary + 8 x h_j staging by bulk async copies, warps per block
+  // -- pinned, tuned, or as the rules by the number of centres (auto_split, spread_warps) chose them
+  void pass_shape(int mode, int* shape4) const;
   // sets the tile shape of pass `mode` as the autotuner would (blocks 0 = default, 3 or 4; grid 0
   // or 1; order 0, 1 or 2; stage 1 = h_j rows by bulk async copies, Effect outer pass): for
   // pinning a shape measured elsewhere
@@ -313,6 +307,7 @@ class Engine {
   int pass_grid_[4] = {0, 0, 0, 0};    // grid shape per pass mode (PassArgs::grid_mode)
   int pass_order_[4] = {0, 0, 0, 0};   // centre order per pass mode (PassArgs::atom_order)
   int pass_stage_[4] = {0, 0, 0, 0};   // h_j staging per pass mode (PassArgs::h_bulk; outer pass)
+  int ran_warps_[11] = {};             // warps per block of each kernel's last launch (PassMode)
   int pass_wpb_[4] = {0, 0, 0, 0};     // warps per block per pass mode (PassArgs::block_warps; 0: by the number of centres)
   template <typename Real> int launch_pass(int mode, PassArgs<Real> a, bool pdl);
   template <typename Real> int launch_shape(int mode, PassArgs<Real> a, int blocks, bool pdl);

@@ -48,7 +48,7 @@ int launch_one(const PassArgs<Real>& a, int sm_count, cudaStream_t stream, bool 
   if (a.natoms == 0) return 0;
   err = launch_kernel(pdl, kern, dim3(grid), dim3(wpb * kWarp), smem, stream, a);
   if (err != cudaSuccess) throw std::runtime_error(std::string("pass launch: ") + cudaGetErrorString(err));
-  return 1;
+  return wpb;
 }
 
 template <typename Real, int L, int MODE>

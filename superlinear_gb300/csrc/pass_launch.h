@@ -61,8 +61,8 @@ inline int spread_warps(int n, int most, int sm_count) {
 // Launches atom_pass_kernel<L, Real, mode, Kahan = (Real is float)> sized as a multiple of the SM
 // count, with the register budget of `blocks` resident blocks per SM (3 or 4; 0 = the default),
 // as a programmatic dependent launch when pdl is set (the kernel stages its model tables while
-// the previous kernel of the stream drains).  Returns the number of kernels launched (1) or
-// throws on a configuration error.
+// the previous kernel of the stream drains).  Returns the warps per block of the launch (0: no
+// centres, nothing launched) or throws on a configuration error.
 template <typename Real>
 int launch_atom_pass(int L, int mode, const PassArgs<Real>& args, int sm_count, cudaStream_t stream,
                      int blocks = 0, bool pdl = false);

@@ -154,10 +154,10 @@ class Engine:
         return {name: (b[q], {3: ms[2 * q], 4: ms[2 * q + 1]}) for q, name in enumerate(self.PASSES) if b[q]}
 
     def pass_shapes(self):
-        """Tile shape of each pass the model runs: {pass: {"blocks_per_sm", "grid", "order",
-        "warps_per_block", "split", "bulk_h"}} (grid "resident" / "balanced", order "strided" /
-        "contiguous" / "dynamic"; split: the Static pass as three kernels; bulk_h: the outer pass's
-        gate-signal rows by bulk async copies)."""
+        """Tile shape of each pass the model runs, on the last evaluation's layout: {pass:
+        {"blocks_per_sm", "grid", "order", "warps_per_block", "split", "bulk_h"}} (grid "resident" /
+        "balanced", order "strided" / "contiguous" / "dynamic"; split: the pass in several kernels, cut
+        at the per-atom boundary; bulk_h: the outer pass's gate-signal rows by bulk async copies)."""
         out = {}
         shape = (ctypes.c_int * 4)()
         passes = ("gate_forward", "outer", "gate_reverse") if self.model.dims["gated"] else ("static",)
