@@ -130,9 +130,9 @@ int sus2g_engine_set_moment_mma(sus2g_engine engine, int enabled);
  * readout / adjoint, and the per-edge adjoint -- through device moment arrays, and the Effect
  * gate passes as two each (edge->moment forward, then the per-atom gate graph and gate-signal
  * projection; the per-atom gate-signal adjoint gather and gate graph reverse, then the per-edge
- * adjoint), instead of one fused kernel per pass (enabled = 1: always; 0: never).  Without this
- * call the number of centres of the evaluation decides, or the autotuner per pass once it has run; a
- * pinned pass shape runs fused.  Results of the two forms agree to FP32 rounding; each repeats bit
+ * adjoint), instead of one fused kernel per pass (enabled = 1: always; 0: never; -1, the default: the
+ * number of centres of the evaluation decides, or the autotuner per pass once it has run, and a
+ * pinned pass shape runs fused).  Results of the two forms agree to FP32 rounding; each repeats bit
  * for bit.  No counterpart in the reference (a launch-shape choice). */
 int sus2g_engine_set_static_split(sus2g_engine engine, int enabled);
 /* The outer and gate reverse parameter-gradient passes (sus2g_engine_combination_grad and the

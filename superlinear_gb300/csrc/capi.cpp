@@ -188,7 +188,7 @@ int sus2g_engine_set_grad_split(sus2g_engine e, int enabled) {
 }
 
 int sus2g_engine_set_static_split(sus2g_engine e, int enabled) {
-  return guarded([&] { need(e, "engine"); e->engine->set_static_split(enabled != 0); });
+  return guarded([&] { need(e, "engine"); e->engine->set_static_split(enabled < 0 ? -1 : enabled != 0); });
 }
 
 int sus2g_engine_set_moment_mma(sus2g_engine e, int enabled) {

@@ -107,12 +107,12 @@ class Engine {
   // drops a captured step graph.
   // The per-atom passes split at the per-atom boundary instead of fused (FP32 engines, basis size
   // 8): the energy pass -- Static, or the Effect outer pass -- as three kernels (edge->moment
-  // forward, per-atom graph, per-edge adjoint), the Effect gate passes likewise.  Without this call
-  // the number of centres decides (auto_split), unless a pass's shape is pinned (fused) or the
-  // autotuner has chosen; a change drops a captured step graph.
-  void set_static_split(bool on) {
-    if (static_split_ != (on ? 1 : 0) || gate_split_ != (on ? 1 : 0)) { reset_step_graph(); ++edge_generation_; }
-    static_split_ = gate_split_ = on ? 1 : 0;
+  // forward, per-atom graph, per-edge adjoint), the Effect gate passes likewise.  1: always, 0: never,
+  // -1 (the default): the number of centres decides (auto_split), unless a pass's shape is pinned
+  // (fused) or the autotuner has chosen; a change drops a captured step graph.
+  void set_static_split(int choice) {
+    if (static_split_ != choice || gate_split_ != choice) { reset_step_graph(); ++edge_generation_; }
+    static_split_ = gate_split_ = choice;
   }
   // The outer and gate reverse parameter-gradient passes as two kernels each (per-atom part,
   // per-edge part; basis size 8) instead of one; a change drops a captured step graph and makes

@@ -189,11 +189,11 @@ class Engine:
         (default on; basis size 8)."""
         check(load().sus2g_engine_set_grad_split(self._h, 1 if on else 0))
 
-    def set_static_split(self, on: bool) -> None:
+    def set_static_split(self, on: bool | None) -> None:
         """FP32 engines, basis size 8: every per-atom pass split at the per-atom boundary (forward /
-        per-atom graph / adjoint kernels) instead of fused.  Without this call the number of centres
+        per-atom graph / adjoint kernels) instead of fused.  None, the default: the number of centres
         decides (pinned pass shapes run fused), or the autotuner once it has run."""
-        check(load().sus2g_engine_set_static_split(self._h, 1 if on else 0))
+        check(load().sus2g_engine_set_static_split(self._h, -1 if on is None else 1 if on else 0))
 
     def set_moment_mma(self, on: bool) -> None:
         """FP32 engines: edge->moment batch sums on the tensor cores (3xTF32 mma.sync) instead of
