@@ -31,6 +31,20 @@ void DevBuf::ensure(size_t n) {
   SUS2G_CUDA(cudaMalloc(&ptr, want));
   bytes = want;
 }
+bool DevBuf::try_ensure(size_t n) {
+  if (n <= bytes && ptr) return true;
+  release();
+  const size_t want = std::max<size_t>(n, 256);
+  const cudaError_t err = cudaMalloc(&ptr, want);
+  if (err == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    ptr = nullptr;
+    return false;
+  }
+  SUS2G_CUDA(err);
+  bytes = want;
+  return true;
+}
 void DevBuf::release() {
   if (ptr) cudaFree(ptr);
   ptr = nullptr;
@@ -2739,13 +2753,14 @@ int Engine::launch_shape(int mode, PassArgs<Real> a, int blocks, bool pdl) {
   // warp resets it, so no memset sits between this launch and its predecessor)
   if (a.atom_order == 2) a.work = work_.as<int>() + 2 * mode;
   // FP64: the kept functions' rows, for up to 16 resident warps per SM (fused passes) or for the
-  // centres of layouts up to kKeepCentres (gate passes: 49 KB per centre at L3/K4; larger ones
-  // evaluate them again in the reverse)
+  // centres of layouts up to kKeepCentres (gate passes); larger ones, and any on a device without the
+  // room, evaluate them again in the reverse
   if (pass_keeps<Real>(mode)) {
     const bool gate = mode == kModeGateForward || mode == kModeGateReverse;
     DevBuf& buf = gate ? keep_gate_ : keep_;
     a.keep_rows = !gate ? std::min(16 * sm_count_, (ncentres_ + 3) / 4 * 4) : ncentres_ <= kKeepCentres ? ncentres_ : 0;
-    buf.ensure(sizeof(Real) * pass_keep_values(model_.L, model_.F) * std::max(1, a.keep_rows));
+    const size_t bytes = sizeof(Real) * pass_keep_values(model_.L, model_.F) * a.keep_rows;
+    if (!keep_size_[gate].holds(buf.bytes, bytes, [&](size_t n) { return buf.try_ensure(n); })) a.keep_rows = 0;
     a.keep = buf.as<Real>();
   }
   const int warps = launch_atom_pass<Real>(model_.L, mode, a, sm_count_, stream_, blocks, pdl);

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "model.h"
+#include "optional_size.h"
 
 namespace sus2g {
 
@@ -21,6 +22,7 @@ struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
   void ensure(size_t n);
+  bool try_ensure(size_t n);  // false: the device has no room (the buffer is then empty)
   void release();
   template <typename T> T* as() const { return static_cast<T*>(ptr); }
   ~DevBuf() { release(); }
@@ -325,8 +327,10 @@ class Engine {
   int gate_split_ = -1;         // Effect gate forward and reverse passes split (together: gkeep_)
   bool gate_ran_split_ = false; // the form of the last gate forward pass, which its reverse takes too
   int gate_split_blocks_[2] = {0, 0};    // their per-edge kernels' register budgets
+  // 49 KB a row at L3/K4, 135 KB at L5/K8, the largest: at most 1.1 GB in keep_gate_, 0.33 GB in keep_
   static constexpr int kKeepCentres = 8192;
   DevBuf keep_, keep_gate_;     // FP64 passes: R, R' and Y per edge for the adjoint (pass_keeps)
+  OptionalSize keep_size_[2];   // of keep_, keep_gate_
   DevBuf mom_;                  // the split pass's moments, then their adjoints [N][K H]
   DevBuf gkeep_;                // split gate passes: gate values kept for the reverse, adjoints of h per centre [N][F]
   // second stream for independent work inside a step (reverse edges beside the first pass, the
