@@ -830,9 +830,8 @@ __global__ void k_check_user_edges(const int* ei, const int* ej, const double* d
   const double x = d[3 * e], y = d[3 * e + 1], z = d[3 * e + 2], r2 = x * x + y * y + z * z;
   if (i < 0 || i >= nowned || j < 0 || j >= nall || !(r2 > 1e-290) || !(r2 < 1e299)) *flag = 1;
 }
-// Counts per centre and per neighbour.  An
-// edge with a centre or neighbour index out of range is flagged and left out here and by the
-// scatter below alike, so that no row keeps an unfilled slot.
+// Counts per centre and per neighbour.  An edge with a centre or neighbour index out of range is
+// flagged and left out here and by the scatter below alike, so that no row keeps an unfilled slot.
 __global__ void k_count_user_edges(const int* ei, const int* ej, long long n, int* out_count, int* in_count, int nowned,
                                    int nall, int* error) {
   const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;

@@ -104,9 +104,6 @@ class Engine {
   // pinning a shape measured elsewhere
   void set_pass_shape(int mode, int blocks, int grid, int order, int stage, int warps);
   void reset_step_graph();
-  // Edge->moment batch sums of the FP32 passes on the tensor cores (3xTF32 mma.sync) instead of
-  // CUDA-core FMAs; off by default (measured slower on GB300, see the design notes); a change
-  // drops a captured step graph.
   // The per-atom passes split at the per-atom boundary instead of fused (FP32 engines, basis size
   // 8): the energy pass -- Static, or the Effect outer pass -- as three kernels (edge->moment
   // forward, per-atom graph, per-edge adjoint), the Effect gate passes likewise.  1: always, 0: never,
@@ -123,6 +120,8 @@ class Engine {
     if (on != grad_split_) { reset_step_graph(); ++edge_generation_; }
     grad_split_ = on;
   }
+  // Edge->moment batch sums of the FP32 passes on the tensor cores (3xTF32 mma.sync) instead of
+  // CUDA-core FMAs; off by default (measured slower on GB300); a change drops a captured step graph.
   void set_moment_mma(bool on) {
     if (on != moment_mma_) reset_step_graph();
     moment_mma_ = on;

@@ -20,13 +20,18 @@
 // The Effect gate chain runs the same steps for the gate pass, seeded with
 // dJ/dh_j and dJ/dhdot_j gathered per atom (stored at the reverse edge, like the force path).
 //
-// Reductions are deterministic.  Per-edge contributions to the per-(k, l) parameters (Chebyshev
+// Reductions are deterministic.  Which kernels run the pass is decided in Engine::run_grad: split at
+// the per-atom boundary (basis size 8), the per-edge part is grad_edge_kernel and in FP32 engines the
+// per-atom part the moment and block graph kernels (grad_edge.cuh, grad_graph.cuh).  grad_pass_kernel
+// below covers the rest: FP64 per-atom parts, other basis sizes, warps per (k, l), models that do not
+// fit those kernels.  In it the per-edge contributions to the per-(k, l) parameters (Chebyshev
 // coefficients, species factors, warp slope / shift, gate additive factors) go to lane-private
 // shared-memory columns (stride 33: conflict-free for a fixed column across lanes and for a fixed
 // lane across columns); after each 32-edge batch and radial index k the warp sums every column over
 // its 32 lanes in a fixed order (one column per lane) and adds the result to its private FP64
-// gradient slice.  Slices are summed in a fixed order by k_slot_reduce.  When the columns do not
-// fit in shared memory (many species), the contributions are summed with shuffle trees instead.
+// gradient slice; where the columns do not fit in shared memory (many species), the contributions
+// are summed with shuffle trees instead.  The slices of all kernels are summed in a fixed order
+// (k_slot_partial, k_slot_finish).
 #pragma once
 #include "efs_kernels.cuh"
 
